@@ -495,7 +495,8 @@ int nes_selftest_bounded_wait(nes_ctx *ctx, uint32_t poll_limit, int arrive);
  * device memory (table_bytes / load_bytes a power of two), XOR-folded into
  * sink_dev[thread]; the caller times it on `stream`.
  * nes_probe_gather_replay replays the march's own load stream for the views
- * on a tensor-core context -- the same rays, warp refills, sample positions,
+ * on a tensor-core context -- the same rays, sample positions (one step of
+ * 32 rays per warp at a time; the march takes 4, 8 or 32 steps of each),
  * record and table addresses, with no interpolation, MLP or compositing --
  * with `threads` (256 or 512) ray slots per SM, and returns its device time
  * (CUDA events) in *replay_ms; sink_dev holds at least (SM count) x threads

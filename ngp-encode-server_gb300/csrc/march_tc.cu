@@ -14,11 +14,12 @@
 // layers, colour input) lives in TMEM and feeds tcgen05.mma directly.
 //
 // One CTA per SM: 4 groups x (4 ENCODER warps + 4 MLP warps) = 1024 threads.
-//  - ENCODER thread = one ray slot.  Per tile it claims rays (a warp-wide
-//    chunk of 32 at a time), encodes its slot's next occupied sample from the
+//  - ENCODER thread = one row of the tile.  A ray takes 4, 8 or 32 of a
+//    warp's rows (lane_shift) with as many of its steps; per tile the warp
+//    claims rays when all of its own are done, hands each row's ray id, flags
+//    and t over in shared memory, encodes the row's occupied sample from the
 //    FP16 table, writes the 32 FP16 features as its TMEM lane of the tile (16
-//    columns), hands the row's ray id, flags and t over in shared memory and
-//    marks the tile full.  It never waits for results: only for
+//    columns) and marks the tile full.  It never waits for results: only for
 //    its tile buffer to be free again (two buffers), which the MLP side
 //    releases once its first layer is done and every row's hand-off has been
 //    read.  Encoder warps run independently.
@@ -26,10 +27,11 @@
 //    (32->64, 64->16, 32->64, 64->64, 64->16 [3 used]) as tcgen05.mma
 //    kind::f16 with A from TMEM and B from shared memory, FP32 accumulators in
 //    TMEM; between layers every thread loads its lane, applies ReLU / exp and
-//    stores the next FP16 A operand back to TMEM.  The same thread then
-//    composites its row's sample into the row's ray (FP32 transmittance,
-//    colour, depth): a row's samples arrive in order, so each ray is
-//    composited by one thread with one state.
+//    stores the next FP16 A operand back to TMEM.  The threads of a ray then
+//    composite its samples of the tile one after another (FP32 transmittance,
+//    colour, depth; values by shuffle, every thread the same state): a ray's
+//    samples arrive in order and are always combined in that order, whatever
+//    the number of its rows.
 //  - Early termination (T < 1e-4) is noticed by the MLP thread, which writes
 //    the ray and tells the row's encoder to move on; samples the encoder
 //    produced meanwhile are dropped.
@@ -87,6 +89,7 @@ constexpr int kSmemAlign = 128;  // operand images need 16 B, mbarriers 8 B
 constexpr int kSmemRequest = kSmemUsed + kSmemAlign;
 // 1 KiB of each CTA's shared memory is reserved by the system.
 static_assert(kSmemRequest + 1024 <= 32 * 1024, "shared memory above the 32 KiB configuration");
+constexpr uint32_t kNoRay = 0xFFFFFFFFu;
 constexpr uint32_t kIdMask = (1u << 28) - 1u;  // ray ids < 2^27 (max_pixels bound)
 
 // Byte offset of 16-byte chunk c (K elements 8c..8c+7) of row n in a
@@ -281,20 +284,178 @@ __device__ __forceinline__ void write_ray(const ViewBatch& vb, const DevScratch&
 }
 
 // Per-row hand-off flags of a tile (with the ray id, encoder -> MLP).
-constexpr uint32_t kTagSample = 1u, kTagFirst = 2u, kTagLast = 4u;
+// kTagRay: the row belongs to a live ray, with or without a sample of its own.
+// A ray has ended when its row turns to another or to none.
+constexpr uint32_t kTagSample = 1u, kTagFirst = 2u, kTagRay = 8u;
 
-// Encoder-side state of one ray slot.
+// log2 of the steps of one ray that a tile takes at once, in neighbouring rows
+// of a warp (32 >> shift rays per warp).  Two things set it.  A batch of few
+// rays must be split along them to fill the chip's 77,824 rows: at one row per
+// ray a 64x48 view keeps 2 % of them busy for as many tiles as its longest
+// ray has steps.  And a warp's 32 samples should lie close together, so that
+// its gathers share cells: a 4x2-pixel patch four steps deep is nearer a cube
+// than a 4x8 patch of single steps.  Measured, ms with L2 flushed, one row per
+// ray (as it was) against 4, 8 and 32 steps:
+//                 rays     seeded scene                 opaque, sparse scene
+//   64x48         1.6k     4.7  -> 1.25, 0.70, 0.24     1.06 -> 0.31, 0.21, 0.15
+//   256x256       34k      4.7  -> 1.39, 0.90, 0.74     1.25 -> 0.39, 0.27, 0.31
+//   320x240       39k              1.39, 1.32, 1.08             0.41, 0.34, 0.44
+//   480x360       88k              2.53, 2.31, 2.22             0.60, 0.54, 0.83
+//   640x360       118k     4.9  -> 3.4,  3.7,  3.9
+//   1280x720      470k    13.4  -> 11.5, 12.5, 15.1
+//   1920x1080     1.06M   25.2  -> 23.8, 26.8, 33.3
+//   2x1920x1832           32.2  -> 29.8, 33.0, 40.8
+//   3x853x481                                           3.19 -> 2.08, 2.16, 4.1
+// Sixteen steps were slower than both neighbours from 256x256 up.  Within the
+// warp a ray's steps are neighbours: with the rays next to each other and the
+// steps apart the 1080p march took 25.1 ms, with both interleaved 24.1.
+__device__ __forceinline__ uint32_t lane_shift(uint32_t nrays, uint32_t rows) {
+  if (nrays <= rows / 2) return 5;
+  if (nrays <= rows + rows / 4) return 3;
+  return 2;
+}
+
+// Position of set bit number j (from 0) of m; m has more than j set bits.
+__device__ __forceinline__ int nth_set_bit(uint32_t m, int j) {
+  int pos = 0;
+#pragma unroll
+  for (int w = 16; w > 0; w >>= 1) {
+    const int c = __popc(m & ((1u << w) - 1u));
+    if (j >= c) {
+      j -= c;
+      m >>= w;
+      pos += w;
+    }
+  }
+  return pos;
+}
+
+// Encoder-side state of one ray slot (the same in all lanes of the ray).
 struct Slot {
   bool live = false;
-  bool first = false;
   float3 o, d;
   float ts = 0.0f;
-  int n = 0, ei = 0;
+  int n = 0;
+  int wb = 0;        // first step after the window
+  uint32_t wm = 0;   // occupied steps of the window [wb - 32, wb) not yet taken
   uint32_t id = 0;
 };
 
-__device__ __forceinline__ void skip_empty(const DevScene& sc, Slot& q) {
-  while (q.ei < q.n && !occupied(sc.occ, sample_pos(q.o, q.d, fmaf((float)q.ei + 0.5f, kDt, q.ts)))) ++q.ei;
+// sample_pos and the occupancy test of it, in fewer instructions: the clamp
+// to the unit cube is the FMA's saturation, and a coordinate of at least 0
+// needs no lower bound on its cell.
+__device__ __forceinline__ float3 sample_pos_sat(const float3& o, const float3& d, float t) {
+  return make_float3(__saturatef(fmaf(t, d.x, o.x)), __saturatef(fmaf(t, d.y, o.y)), __saturatef(fmaf(t, d.z, o.z)));
+}
+__device__ __forceinline__ uint32_t occupied_at(const uint32_t* __restrict__ occ, const float3& x) {
+  const int cx = min(__float2int_rd(x.x * kOccRes), kOccRes - 1), cy = min(__float2int_rd(x.y * kOccRes), kOccRes - 1),
+            cz = min(__float2int_rd(x.z * kOccRes), kOccRes - 1);
+  const uint32_t i = (uint32_t)cx + kOccRes * ((uint32_t)cy + kOccRes * (uint32_t)cz);
+  return (__ldg(occ + (i >> 5)) >> (i & 31)) & 1u;
+}
+
+// Moves every ray whose window is used up to its next 32-step window with an
+// occupied step; a ray without one is no longer live.  The ray's lanes test
+// the window's steps between them.  Whole warps call it.
+template <int kShift>
+__device__ __forceinline__ void next_window(const DevScene& sc, Slot& q, int j) {
+  for (;;) {
+    const bool need = q.live && q.wm == 0u && q.wb < q.n;
+    if (__ballot_sync(0xffffffffu, need) == 0u) break;
+    uint32_t bits = 0;
+    if (need) {
+      const int lim = min(32, q.n - q.wb);
+      for (int i = j; i < lim; i += 1 << kShift)
+        bits |= occupied_at(sc.occ, sample_pos_sat(q.o, q.d, fmaf((float)(q.wb + i) + 0.5f, kDt, q.ts))) << i;
+    }
+#pragma unroll
+    for (int k = 0; k < kShift; ++k) bits |= __shfl_xor_sync(0xffffffffu, bits, 1 << k);
+    if (need) {
+      q.wm = bits;
+      q.wb += 32;
+    }
+  }
+  if (q.wm == 0u) q.live = false;
+}
+
+// The encoder warps' loop; true when a wait ran out.
+template <int kRec, int kShift>
+__device__ __forceinline__ bool encoder_loop(const ViewBatch& vb, const DevScene& sc, const DevScratch& s,
+                                             uint32_t nrays, uint64_t* bar, volatile uint32_t* gdone,
+                                             const uint32_t* term, uint2* hand, uint32_t* wfin, uint32_t enc_row) {
+  constexpr int kLanes = 1 << kShift;
+  const int lane = threadIdx.x & 31, wq = (threadIdx.x >> 5) & 3, row = threadIdx.x % kRoleThreads;
+  const int j = lane & (kLanes - 1), ray_lane = lane - j;
+  Slot q;
+  bool exhausted = false;
+  for (uint32_t k = 0;; ++k) {
+    const int b = (int)(k & 1u);
+    if (k >= 2) {
+      // Lane 0 waits and reads the group's stop flag; the warp learns both
+      // from it, so every lane takes the same exit.
+      int st = 0;
+      if (lane == 0) st = !tc::mbar_wait_sleep(bar + 2 + b, ((k >> 1) - 1u) & 1u) ? 1 : (*gdone ? 2 : 0);
+      st = __shfl_sync(0xffffffffu, st, 0);
+      if (st == 1) return true;
+      if (st == 2) return false;
+    }
+    // A ray the MLP terminated early (T < 1e-4) is encoded no further.
+    {
+      const uint32_t over = __ballot_sync(0xffffffffu, q.live && term[row] == q.id + 1u);
+      if ((over >> ray_lane) & 1u) q.live = false;
+    }
+    // Refill a whole warp at once: the warp claims 32 / kLanes consecutive
+    // rays (a compact patch of pixels) only when all its lanes are done, so
+    // its 32 samples stay neighbours in space and each warp-wide gather stays
+    // coherent.
+    bool first = false;
+    for (;;) {
+      next_window<kShift>(sc, q, j);
+      if (first && !q.live && j == 0) write_ray(vb, s, q.id, 0.0f, 0.0f, 0.0f, 0.0f);  // no occupied sample
+      if (exhausted || __ballot_sync(0xffffffffu, q.live) != 0u) break;
+      first = false;
+      uint32_t base = 0;
+      if (lane == 0) base = atomicAdd(s.counters + kCtrCursor, 32u >> kShift);
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (base >= nrays) {
+        exhausted = true;
+        break;
+      }
+      const uint32_t id = base + ((uint32_t)lane >> kShift);
+      if (id < nrays) {
+        const float4 rd = s.ray_dt[id];
+        const RayMeta m = s.ray_meta[id];
+        const DevView& V = vb.v[m.view];
+        q.o = make_float3(V.M[3], V.M[7], V.M[11]);
+        q.d = make_float3(rd.x, rd.y, rd.z);
+        q.ts = rd.w;
+        q.n = m.n;
+        q.id = id;
+        q.wb = 0;
+        q.wm = 0u;
+        q.live = first = true;
+      }
+    }
+    // The ray's next occupied steps of its window, one per lane.
+    const bool has = q.live && __popc(q.wm) > j;
+    int bit = 31;
+    if (has) {  // mostly the window's steps are consecutive from its first one
+      const int low = __ffs(q.wm) - 1;
+      bit = low + j;
+      if ((~(q.wm >> low) & ((2u << j) - 1u)) != 0u) bit = nth_set_bit(q.wm, j);
+    }
+    const float t = has ? fmaf((float)(q.wb - 32 + bit) + 0.5f, kDt, q.ts) : 0.0f;
+    const float3 x = sample_pos_sat(q.o, q.d, t);
+    q.wm &= ~0u << __shfl_sync(0xffffffffu, bit, ray_lane + kLanes - 1) << 1;
+    const uint32_t tag = q.live ? kTagRay | (has ? kTagSample : 0u) | (first ? kTagFirst : 0u) : 0u;
+    hand[b * 128 + row] = make_uint2(q.id | (tag << 28), __float_as_uint(t));
+    const bool fin = exhausted && __ballot_sync(0xffffffffu, q.live) == 0u;
+    if (lane == 0) wfin[b * 4 + wq] = fin ? 1u : 0u;
+    encode_all<kRec>(sc.table16, sc.rec16, sc.T, sc.dense_mask, x, has, enc_row + 16 * b);
+    tc::tmem_wait_st();
+    tc::fence_before();
+    tc::mbar_arrive(bar + b);
+  }
 }
 
 template <class Src, int kRec>
@@ -357,11 +518,13 @@ march_tc_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScr
   static_assert(kGroups * kRoleThreads * (kEncRegs + kMlpRegs) == kTcThreads * kLaunchRegs, "register split");
 
   unsigned long long my_samples = 0;
+  const uint32_t nrays = min(s.counters[kCtrRays], s.max_rays);
+  const uint32_t shift = lane_shift(nrays, gridDim.x * kGroups * kRoleThreads);
   if (!fail && is_mlp) {
     // ======================= MLP warps =======================
     // One thread per tile row: it evaluates the row's sample through the
-    // five layers and composites it into the row's current ray, so a ray's
-    // samples are composited in order by one thread with one state.
+    // five layers; the threads of a ray's rows then composite its samples in
+    // order, each with the same state.
     tc::regs_dec<kMlpRegs>();
     const uint32_t sW = tc::smem_addr(smem + kOffW);
     const uint32_t h_col = tmem + kMlpBase + g * kMlpColsPerGroup;  // hidden activations (lane 0)
@@ -369,9 +532,10 @@ march_tc_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScr
     const uint32_t d_row = d_col + lane_off, h_row = h_col + lane_off;
     constexpr uint32_t id64 = tc::idesc_f16_f32(128, 64), id16 = tc::idesc_f16_f32(128, 16);
     uint32_t pm = 0;
-    uint32_t cur = 0xFFFFFFFFu;  // ray being composited in this row (none)
+    uint32_t cur = kNoRay;  // ray being composited in this row
     float T = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f, cz = 0.0f;
     float dx = 0.0f, dy = 0.0f, dz = 1.0f;  // direction of the row's current ray
+    const int lanes = 1 << shift, ray_lane = lane & ~(lanes - 1);  // the row's ray: its lanes of the warp
 
     // Issues one layer (one thread) and waits for it (every thread); the
     // free barrier of the tile's buffer, if given, is released by the same
@@ -405,6 +569,13 @@ march_tc_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScr
       if (row == 0) ok = tc::mbar_wait_sleep(bar + b, (k >> 1) & 1u);
       if (sync_bad()) { fail = true; break; }
       tc::fence_after();
+      const uint2 hd = hand[b * 128 + row];
+      const uint32_t rid = hd.x & kIdMask, flags = hd.x >> 28;
+      const float t = __uint_as_float(hd.y);
+      if ((flags & kTagFirst) || !(flags & kTagRay)) {  // the row's ray, if it has not terminated, is complete
+        if (cur != kNoRay && lane == ray_lane) write_ray(vb, s, cur, cr, cg, cb, cz);
+        cur = kNoRay;
+      }
       if (wfin[b * 4 + 0] & wfin[b * 4 + 1] & wfin[b * 4 + 2] & wfin[b * 4 + 3]) {
         // Every encoder warp of the group is out of rays: release the
         // encoders that wait for this buffer and stop.
@@ -414,14 +585,14 @@ march_tc_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScr
         }
         break;
       }
-      const uint2 hd = hand[b * 128 + row];
-      const uint32_t rid = hd.x & kIdMask, flags = hd.x >> 28;
-      const float t = __uint_as_float(hd.y);
-      if (flags & kTagFirst) {  // a new ray in this row: its direction, for the colour MLP
+      if (flags & kTagFirst) {  // a new ray in this row; its direction is for the colour MLP
         const float4 rd = s.ray_dt[rid];
         dx = rd.x;
         dy = rd.y;
         dz = rd.z;
+        cur = rid;
+        T = 1.0f;
+        cr = cg = cb = cz = 0.0f;
       }
       const uint32_t a_col = enc_cols + 16 * b;  // encoded features of this tile
       // density 32 -> 64 -> 16 (the first layer is the features' last reader)
@@ -462,29 +633,35 @@ march_tc_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScr
       layer(h_col, kWoffCW3, 64, id16, nullptr);
       float v5[16];
       tc::tmem_ld16(d_row, v5);
-      // Compositing (FP32, every operation rounded explicitly).
-      if (flags & kTagSample) {
-        if (flags & kTagFirst) {
-          cur = rid;
-          T = 1.0f;
-          cr = cg = cb = cz = 0.0f;
-        }
-        if (cur == rid) {  // samples of a ray that already terminated are dropped
+      // Compositing (FP32, every operation rounded explicitly).  A ray's rows
+      // of the tile, its next steps in order, are composited one after another
+      // by each of its lanes alike.
+      const float alpha = -expm1f(__fmul_rn(-sigma, kDt));
+      const float s0 = sigmoidf(v5[0]), s1 = sigmoidf(v5[1]), s2 = sigmoidf(v5[2]);
+      const uint32_t have = __ballot_sync(0xffffffffu, (flags & kTagSample) != 0u);
+      const bool open = cur != kNoRay;  // samples of a ray that already terminated are dropped
+      bool stop_early = false;
+      for (int i = 0; i < lanes; ++i) {
+        const float ai = __shfl_sync(0xffffffffu, alpha, ray_lane + i);
+        const float ri = __shfl_sync(0xffffffffu, s0, ray_lane + i);
+        const float gi = __shfl_sync(0xffffffffu, s1, ray_lane + i);
+        const float bi = __shfl_sync(0xffffffffu, s2, ray_lane + i);
+        const float ti = __shfl_sync(0xffffffffu, t, ray_lane + i);
+        if (open && !stop_early && ((have >> (ray_lane + i)) & 1u)) {
           ++my_samples;
-          const float alpha = -expm1f(__fmul_rn(-sigma, kDt));
-          const float wgt = __fmul_rn(T, alpha);
-          cr = __fmaf_rn(wgt, sigmoidf(v5[0]), cr);
-          cg = __fmaf_rn(wgt, sigmoidf(v5[1]), cg);
-          cb = __fmaf_rn(wgt, sigmoidf(v5[2]), cb);
-          cz = __fmaf_rn(wgt, t, cz);
+          const float wgt = __fmul_rn(T, ai);
+          cr = __fmaf_rn(wgt, ri, cr);
+          cg = __fmaf_rn(wgt, gi, cg);
+          cb = __fmaf_rn(wgt, bi, cb);
+          cz = __fmaf_rn(wgt, ti, cz);
           T = __fsub_rn(T, wgt);
-          const bool stop_early = T < kTStop;
-          if (stop_early || (flags & kTagLast)) {
-            write_ray(vb, s, cur, cr, cg, cb, cz);
-            if (stop_early && !(flags & kTagLast)) term[row] = cur + 1u;  // tells the encoder to move on
-            cur = 0xFFFFFFFFu;
-          }
+          stop_early = T < kTStop;
         }
+      }
+      if (stop_early) {
+        if (lane == ray_lane) write_ray(vb, s, cur, cr, cg, cb, cz);
+        term[row] = cur + 1u;  // tells the encoder to move on
+        cur = kNoRay;
       }
       // The next tile's first layer overwrites the accumulator this thread
       // has just read: the wait at the top of the loop is a barrier.
@@ -494,77 +671,9 @@ march_tc_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScr
     // Each warp runs on its own: it waits only for its tile buffer to be
     // free (the MLP's first layer has read it), never for results.
     tc::regs_inc<kEncRegs>();
-    const uint32_t nrays = min(s.counters[kCtrRays], s.max_rays);
-    const int wq = warp & 3;
-    Slot q;
-    bool exhausted = false;
-    for (uint32_t k = 0;; ++k) {
-      const int b = (int)(k & 1u);
-      if (k >= 2) {
-        // Lane 0 waits and reads the group's stop flag; the warp learns both
-        // from it, so every lane takes the same exit.
-        int st = 0;
-        if (lane == 0) st = !tc::mbar_wait_sleep(bar + 2 + b, ((k >> 1) - 1u) & 1u) ? 1 : (*gdone ? 2 : 0);
-        st = __shfl_sync(0xffffffffu, st, 0);
-        if (st == 1) { fail = true; break; }
-        if (st == 2) break;
-      }
-      // A ray the MLP terminated early (T < 1e-4) is encoded no further.
-      if (q.live && term[row] == q.id + 1u) q.live = false;
-      // Refill a whole warp at once: the warp claims 32 consecutive rays (one
-      // 4x8 pixel tile) only when all its lanes are done, so its 32 samples
-      // stay neighbours in space and each warp-wide gather stays coherent.
-      for (;;) {
-        if (__ballot_sync(0xffffffffu, q.live) != 0u || exhausted) break;
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(s.counters + kCtrCursor, 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= nrays) {
-          exhausted = true;
-          break;
-        }
-        const uint32_t id = base + lane;
-        if (id < nrays) {
-          const float4 rd = s.ray_dt[id];
-          const RayMeta m = s.ray_meta[id];
-          const DevView& V = vb.v[m.view];
-          q.o = make_float3(V.M[3], V.M[7], V.M[11]);
-          q.d = make_float3(rd.x, rd.y, rd.z);
-          q.ts = rd.w;
-          q.n = m.n;
-          q.ei = 0;
-          q.id = id;
-          skip_empty(sc, q);
-          if (q.ei < q.n) {
-            q.live = true;
-            q.first = true;
-          } else {
-            write_ray(vb, s, id, 0.0f, 0.0f, 0.0f, 0.0f);  // no occupied sample
-          }
-        }
-      }
-      const bool has = q.live;
-      uint32_t tag = 0;
-      const float t = has ? fmaf((float)q.ei + 0.5f, kDt, q.ts) : 0.0f;
-      const float3 x = sample_pos(q.o, q.d, t);
-      encode_all<kRec>(sc.table16, sc.rec16, sc.T, sc.dense_mask, x, has, enc_cols + 16 * b + lane_off);
-      if (has) {
-        tag = kTagSample | (q.first ? kTagFirst : 0u);
-        q.first = false;
-        ++q.ei;
-        skip_empty(sc, q);
-        if (q.ei >= q.n) {
-          tag |= kTagLast;
-          q.live = false;
-        }
-      }
-      hand[b * 128 + row] = make_uint2(q.id | (tag << 28), __float_as_uint(t));
-      const bool fin = exhausted && __ballot_sync(0xffffffffu, has) == 0u;
-      if (lane == 0) wfin[b * 4 + wq] = fin ? 1u : 0u;
-      tc::tmem_wait_st();
-      tc::fence_before();
-      tc::mbar_arrive(bar + b);
-    }
+    if (shift == 5) fail = encoder_loop<kRec, 5>(vb, sc, s, nrays, bar, gdone, term, hand, wfin, enc_cols + lane_off);
+    else if (shift == 3) fail = encoder_loop<kRec, 3>(vb, sc, s, nrays, bar, gdone, term, hand, wfin, enc_cols + lane_off);
+    else fail = encoder_loop<kRec, 2>(vb, sc, s, nrays, bar, gdone, term, hand, wfin, enc_cols + lane_off);
   }
 
   if (fail) atomicExch(s.counters + kCtrError, 1u);
@@ -576,8 +685,8 @@ march_tc_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScr
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) my_samples += __shfl_down_sync(0xffffffffu, my_samples, off);
-  if (lane == 0 && my_samples)
-    atomicAdd(reinterpret_cast<unsigned long long*>(s.counters + kCtrSamples), my_samples);
+  if (lane == 0 && my_samples)  // each of a ray's lanes counted its samples
+    atomicAdd(reinterpret_cast<unsigned long long*>(s.counters + kCtrSamples), my_samples >> shift);
 }
 
 // FP32 weight blob -> FP16 operand image (see the kWoff* map).

@@ -28,6 +28,15 @@ struct DevView {
 // reuse of the hash-table gathers than a 32x1 row strip).
 constexpr int kTileW = 4, kTileH = 8;
 
+// Pixel (x, y) of index `in` of a tile: x and y bits alternate, so that
+// every aligned group of 2, 4, 8 or 16 consecutive rays is as near square as
+// it can be (2x1, 2x2, 4x2, 4x4): the groups a warp takes when it marches
+// several steps of each ray at once.
+__host__ __device__ inline void tile_pixel(uint32_t in, int* x, int* y) {
+  *x = (int)((in & 1u) | ((in >> 1) & 2u));
+  *y = (int)(((in >> 1) & 1u) | ((in >> 2) & 6u));
+}
+
 __host__ __device__ inline uint32_t view_threads(int W, int H) {
   return (uint32_t)((W + kTileW - 1) / kTileW) * (uint32_t)((H + kTileH - 1) / kTileH) * (kTileW * kTileH);
 }

@@ -41,8 +41,10 @@ raygen_kernel(const __grid_constant__ Src src, float4* __restrict__ ray_dt, RayM
       const uint32_t local = gid - V.pix_offset;
       const uint32_t tile = local / (kTileW * kTileH), in = local % (kTileW * kTileH);
       const uint32_t tiles_x = (uint32_t)(V.W + kTileW - 1) / kTileW;
-      const int px = (int)((tile % tiles_x) * kTileW + in % kTileW);
-      const int py = (int)((tile / tiles_x) * kTileH + in / kTileW);
+      int px, py;
+      tile_pixel(in, &px, &py);
+      px += (int)((tile % tiles_x) * kTileW);
+      py += (int)((tile / tiles_x) * kTileH);
       if (px < V.W && py < V.H) {  // tile padding beyond the frame edge does nothing
         pix = py * V.W + px;
         n = ray_setup(V.M, V.W, V.H, V.focal, px, py, o, d, ts);
