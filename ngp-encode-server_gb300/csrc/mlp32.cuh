@@ -1,6 +1,6 @@
 // mlp32.cuh -- FP32 density and colour MLPs evaluated per thread with the
-// weights broadcast from shared memory (the plain CUDA-core path, the
-// occupancy build and the training kernels).
+// weights broadcast from shared memory (the occupancy build and the training
+// kernels; the march's form is tile32.cuh).
 #pragma once
 #include "render_common.cuh"
 

@@ -10,13 +10,33 @@
 
 #include "kernels.h"
 #include "mlp32.cuh"
+#include "ray_slot.cuh"
+#include "tile32.cuh"
 
 namespace nes {
 
 namespace {
 
 constexpr int kRaygenThreads = 256;
-constexpr int kMarchThreads = 128;
+// Twelve warps of the march per SM: 150 KB of shared memory (weights and the
+// warps' tiles) leave L1 to the gathers, and 159 registers a thread hold the
+// tile product's operands ahead.  1080p: 8 warps 156 ms, 10 151, 12 145, 14
+// (126 registers) 145, 16 168 (before packed FMAs, against 150 with 12).
+constexpr int kMarchWarps = 12;
+constexpr int kMarchThreads = 32 * kMarchWarps;
+
+// log2 of the steps of one ray that a warp takes at once: many where the rays
+// are too few for the chip's 58,368 rows, fewer where that would evaluate
+// steps behind an opaque surface or leave lanes without an occupied step.  ms,
+// one ray per thread (as it was) -> 8 and 32 steps:
+//               rays   seeded scene          opaque, sparse scene
+//   64x48       1.6k   20   -> 2.2,  0.64    10.0 -> 0.61, 0.41
+//   256x256     34k    24   -> 3.6,  2.9     13.1 -> 0.86, 0.97
+//   400x300     61k    26.7 -> 7.2,  6.7     13.7 -> 1.5,  1.9
+//   640x360     118k   37.7 -> 16.5, 16.4    18.2 -> 2.9,  4.3
+//   853x481     210k   54.6 -> 28.5, 28.9    24.2 -> 4.9,  7.4
+//   1920x1080   1.06M  232  -> 138,  145     (1, 2, 4, 16 steps: 163, 144, 139, 141)
+__device__ __forceinline__ int march32_shift(uint32_t nrays, uint32_t rows) { return nrays <= rows / 3 * 2 ? 5 : 3; }
 
 // Grid-stride over the batch's ray-generation threads (the loop bound is
 // uniform per block, and every view's thread count is a multiple of 32, so
@@ -75,64 +95,107 @@ raygen_kernel(const __grid_constant__ Src src, float4* __restrict__ ray_dt, RayM
   }
 }
 
+// The march: one CTA per SM, its warps independent, each with 32 samples at a
+// time: (32 >> kShift) rays with their next 1 << kShift occupied steps each.
+// The warp encodes its lanes' samples into its shared-memory tile, evaluates
+// the MLPs as matrix products over it (tile32.cuh) and composites each ray's
+// samples in step order, every lane of the ray alike, by shuffle.
+struct MarchSmem32 {
+  TileWeights32 w;
+  float tile[kMarchWarps][kTileFloats];
+};
+
+template <int kShift>
+__device__ __forceinline__ unsigned long long march_fp32_loop(const ViewBatch& vb, const DevScene& sc,
+                                                              const DevScratch& s, uint32_t nrays,
+                                                              const TileWeights32& W, float* X) {
+  constexpr int kLanes = 1 << kShift;
+  const int lane = threadIdx.x & 31, j = lane & (kLanes - 1), ray_lane = lane - j;
+  Slot q;
+  bool exhausted = false, open = false;  // open: the slot's ray is being composited
+  float T = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f, dep = 0.0f;
+  unsigned long long my_samples = 0;
+  for (;;) {
+    for (;;) {
+      next_window<kShift>(sc, q, j);
+      if (open && !q.live) {
+        if (j == 0) write_ray(vb, s, q.id, cr, cg, cb, dep);
+        open = false;
+      }
+      if (exhausted || __ballot_sync(0xffffffffu, q.live) != 0u) break;
+      const uint32_t base = warp_claim(s.counters + kCtrCursor, 32u >> kShift);
+      if (base >= nrays) {
+        exhausted = true;
+        break;
+      }
+      const uint32_t id = base + ((uint32_t)lane >> kShift);
+      if (id < nrays) {
+        q.start(vb, s, id);
+        open = true;
+        T = 1.0f;
+        cr = cg = cb = dep = 0.0f;
+      }
+    }
+    if (__ballot_sync(0xffffffffu, q.live) == 0u) return my_samples;  // out of rays
+    float t;
+    const bool has = take_step<kShift>(q, j, ray_lane, &t);
+    const float3 x = sample_pos(q.o, q.d, t);
+#pragma unroll
+    for (int l = 0; l < kLevels; ++l) {
+      float f0 = 0.0f, f1 = 0.0f;
+      if (has) encode_level_fp32(sc.table32, sc.T, sc.dense_mask, x, l, f0, f1);
+      X[(2 * l) * 32 + (lane ^ tile_swap(2 * l))] = f0;
+      X[(2 * l + 1) * 32 + (lane ^ tile_swap(2 * l + 1))] = f1;
+    }
+    __syncwarp();
+    float3 c;
+    const float sigma = tile_mlp32(W, X, lane, q.d, &c);
+    const float alpha_own = -expm1f(-sigma * kDt);
+    const uint32_t have = __ballot_sync(0xffffffffu, has);
+    bool stop = false;
+#pragma unroll 4
+    for (int i = 0; i < kLanes; ++i) {
+      const float alpha = __shfl_sync(0xffffffffu, alpha_own, ray_lane + i);
+      const float ci0 = __shfl_sync(0xffffffffu, c.x, ray_lane + i);
+      const float ci1 = __shfl_sync(0xffffffffu, c.y, ray_lane + i);
+      const float ci2 = __shfl_sync(0xffffffffu, c.z, ray_lane + i);
+      const float ti = __shfl_sync(0xffffffffu, t, ray_lane + i);
+      if (q.live && !stop && ((have >> (ray_lane + i)) & 1u)) {
+        ++my_samples;
+        const float w = T * alpha;
+        cr = fmaf(w, ci0, cr);
+        cg = fmaf(w, ci1, cg);
+        cb = fmaf(w, ci2, cb);
+        dep = fmaf(w, ti, dep);
+        T -= w;
+        stop = T < kTStop;
+      }
+    }
+    if (stop) q.live = false;  // written at the top of the loop
+  }
+}
+
 template <class Src>
-__global__ void __launch_bounds__(kMarchThreads)
+__global__ void __launch_bounds__(kMarchThreads, 1)
 march_fp32_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScratch s) {
   const ViewBatch& vb = src.get();
   extern __shared__ float4 smem_raw[];
-  SmemWeights32& W = *reinterpret_cast<SmemWeights32*>(smem_raw);
-  load_weights32(W, sc.weights);
+  MarchSmem32& S = *reinterpret_cast<MarchSmem32*>(smem_raw);
+  load_tile_weights32(S.w, sc.weights);
   __syncthreads();
-
   const uint32_t nrays = min(s.counters[kCtrRays], s.max_rays);
-  const unsigned lane = threadIdx.x & 31u;
-  unsigned long long my_samples = 0;
-  for (;;) {
-    const uint32_t base = warp_claim(s.counters + kCtrCursor, 32);
-    if (base >= nrays) break;
-    const uint32_t r = base + lane;
-    if (r < nrays) {
-    const float4 rd = s.ray_dt[r];
-    const RayMeta m = s.ray_meta[r];
-    const DevView& V = vb.v[m.view];
-    const float3 o = make_float3(V.M[3], V.M[7], V.M[11]);
-    const float3 d = make_float3(rd.x, rd.y, rd.z);
-    float sh[16];
-    sh16(d, sh);
-    float T = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f, dep = 0.0f;
-    for (int i = 0; i < m.n; ++i) {
-      const float t = fmaf((float)i + 0.5f, kDt, rd.w);
-      const float3 x = sample_pos(o, d, t);
-      if (!occupied(sc.occ, x)) continue;
-      float enc[kEnc];
-      encode_fp32(sc.table32, sc.T, sc.dense_mask, x, enc);
-      float dout[kDOut];
-      density_mlp32(W, enc, dout);
-      const float sigma = expf(dout[0] - 1.0f);
-      const float3 c = colour_mlp32(W, sh, dout);
-      ++my_samples;
-      const float alpha = -expm1f(-sigma * kDt);
-      const float w = T * alpha;
-      cr = fmaf(w, c.x, cr);
-      cg = fmaf(w, c.y, cg);
-      cb = fmaf(w, c.z, cb);
-      dep = fmaf(w, t, dep);
-      T -= w;
-      if (T < kTStop) break;
-    }
-    if (V.rgb) {
-      V.rgb[(size_t)m.pixel * 3 + 0] = cr;
-      V.rgb[(size_t)m.pixel * 3 + 1] = cg;
-      V.rgb[(size_t)m.pixel * 3 + 2] = cb;
-    }
-    if (V.depth) V.depth[m.pixel] = dep;
-    }
-  }
-  // One 64-bit atomic per warp for the sample count.
+  const uint32_t rows = gridDim.x * kMarchThreads;
+  float* X = S.tile[threadIdx.x >> 5];
+  unsigned long long my_samples;
+  const int shift = march32_shift(nrays, rows);
+  if (shift == 5) my_samples = march_fp32_loop<5>(vb, sc, s, nrays, S.w, X);
+  else my_samples = march_fp32_loop<3>(vb, sc, s, nrays, S.w, X);
+  // One 64-bit atomic per warp for the sample count, which each of a ray's
+  // lanes has.
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) my_samples += __shfl_down_sync(0xffffffffu, my_samples, off);
-  if (lane == 0 && my_samples)
-    atomicAdd(reinterpret_cast<unsigned long long*>(s.counters + kCtrSamples), my_samples);
+  if ((threadIdx.x & 31u) == 0 && my_samples)
+    atomicAdd(reinterpret_cast<unsigned long long*>(s.counters + kCtrSamples), my_samples >> shift);
 }
 
 constexpr int kOccThreads = 128;
@@ -187,19 +250,14 @@ namespace {
 template <class Src>
 cudaError_t launch_march_fp32_src(const Src& src, const DevScene& scene, const DevScratch& s, int num_sms,
                                   cudaStream_t stream) {
-  const int smem = (int)sizeof(SmemWeights32);
+  const int smem = (int)sizeof(MarchSmem32);
   static bool attr_set = false;  // idempotent; harmless if two threads race on it
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(march_fp32_kernel<Src>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  int per_sm = 0;
-  cudaError_t e =
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, march_fp32_kernel<Src>, kMarchThreads, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) per_sm = 1;
-  march_fp32_kernel<Src><<<num_sms * per_sm, kMarchThreads, smem, stream>>>(src, scene, s);
+  march_fp32_kernel<Src><<<num_sms, kMarchThreads, smem, stream>>>(src, scene, s);
   return cudaGetLastError();
 }
 

@@ -1,10 +1,11 @@
-"""The tensor-core march gives a ray 4, 8 or 32 rows of a tile by the number
-of rays in the batch.  A ray's samples are composited in one order whatever
-that number is, so a view's pixels must not depend on what it is batched with:
-the same view alone (32 rows per ray), behind a batch of some 40,000 rays (8)
-and behind one of 160,000 (4), bit for bit, and the sample counts add up.
-Against the oracle: a partial grid (windows with gaps), an opaque field (rays
-that end inside a tile) and ray counts around a warp."""
+"""The marches take several steps of a ray at a time, as many as the number of
+rays in the batch asks for (tensor cores: 4, 8 or 32; plain FP32: 8 or 32).  A
+ray's samples are composited in one order whatever that number is, so a view's
+pixels must not depend on what it is batched with: the same view alone (32
+steps), behind a batch of some 40,000 rays (8) and behind one of 160,000 (4 or
+8), bit for bit, and the sample counts add up.  Against the oracle: a partial
+grid (windows with gaps), an opaque field (rays that end inside a tile) and ray
+counts around a warp."""
 import numpy as np
 import pytest
 
@@ -21,13 +22,15 @@ def _render(r, torch, nes_lib, views):
 
 
 @pytest.mark.parametrize("field", ["seeded", "partial", "opaque"])
-def test_rows_per_ray_do_not_change_a_view(nes_lib, oracle_mod, cuda, field):
+@pytest.mark.parametrize("prec", ["fp32", "tc"])
+def test_steps_at_a_time_do_not_change_a_view(nes_lib, oracle_mod, cuda, field, prec):
     poses = nes_lib.shell_poses(21, 4, 1.3, 1.5)
     view = (poses[0], 37, 29, nes_lib.focal_from_fov(37, 80.0))
     inside = [1, 0, 0, .5, 0, -1, 0, .5, 0, 0, -1, .5]  # every ray hits: 40,000 and 160,000 rays
     mid = (inside, 200, 200, nes_lib.focal_from_fov(200, 100.0))
     large = (inside, 400, 400, nes_lib.focal_from_fov(400, 100.0))
-    with nes_lib.Renderer(precision=nes_lib.PREC_FP16_TC, record_levels=10, max_pixels=200000) as r:
+    p = nes_lib.PREC_FP32 if prec == "fp32" else nes_lib.PREC_FP16_TC
+    with nes_lib.Renderer(precision=p, record_levels=10, max_pixels=200000) as r:
         sc = oracle_mod.Scene(0, 19)
         if field == "partial":
             r.rebuild_occupancy(0.37)
@@ -45,12 +48,13 @@ def test_rows_per_ray_do_not_change_a_view(nes_lib, oracle_mod, cuda, field):
             assert both == count + alone
     orgb, odep, _ = sc.render(*view, occ=occ)
     assert oracle_mod.psnr(rgb, orgb) >= 45.0
-    # The opaque field's bound is one march step (its logit weights scale the FP16 rounding into sigma).
-    assert np.abs(dep - odep).max() <= (oracle_mod.dt() if field == "opaque" else 1e-3)
+    # The opaque field's bound in FP16 is one march step (its logit weights scale the rounding into sigma).
+    assert np.abs(dep - odep).max() <= (oracle_mod.dt() if field == "opaque" and prec == "tc" else 1e-3)
     if field != "opaque":  # FP16: a ray's T may cross the threshold one sample earlier or later
-        # The plain march visits the same steps (the oracle looks the grid up at FP64 positions, where a
+        # The other precision's march visits the same steps (the oracle looks the grid up at FP64 positions, where a
         # step on a cell's border may fall to the other side).
-        with nes_lib.Renderer(precision=nes_lib.PREC_FP32, max_pixels=37 * 29) as r:
+        other = nes_lib.PREC_FP16_TC if prec == "fp32" else nes_lib.PREC_FP32
+        with nes_lib.Renderer(precision=other, record_levels=10, max_pixels=37 * 29) as r:
             if field == "partial":
                 r.rebuild_occupancy(0.37)
             assert np.array_equal(r.occupancy(), occ)
@@ -58,9 +62,9 @@ def test_rows_per_ray_do_not_change_a_view(nes_lib, oracle_mod, cuda, field):
 
 
 @pytest.mark.parametrize("w,h", [(5, 1), (8, 4), (33, 1), (16, 9)])
-def test_few_rays_vs_oracle(nes_lib, rtc, cuda, scene0, oracle_mod, w, h):
+def test_few_rays_vs_oracle(nes_lib, renderer, cuda, scene0, oracle_mod, w, h):
     view = (nes_lib.shell_poses(5, 2, 1.2, 1.3)[1], w, h, nes_lib.focal_from_fov(w, 60.0))
-    ((rgb, dep),), samples = _render(rtc, cuda, nes_lib, [view])
+    ((rgb, dep),), samples = _render(renderer, cuda, nes_lib, [view])
     orgb, odep, osamples = scene0.render(*view)
     assert samples == osamples
     assert oracle_mod.psnr(rgb, orgb) >= 45.0
