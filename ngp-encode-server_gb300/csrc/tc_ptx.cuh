@@ -100,9 +100,10 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// Shared-memory matrix descriptor, no swizzle, K-major canonical layout:
-// 8x16-byte core matrices; lbo = byte stride between core matrices along K,
-// sbo = byte stride between 8-row groups; bits 46-47 = descriptor version 1.
+// Shared-memory matrix descriptor, no swizzle, canonical layout: 8x16-byte
+// core matrices (K-major: 8 M/N rows of 16 bytes along K; MN-major: 8 K rows
+// of 16 bytes along M/N); lbo = byte stride between core matrices along K, sbo
+// = along M/N; bits 46-47 = descriptor version 1.
 __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
          (1ull << 46);
@@ -117,6 +118,12 @@ __host__ __device__ constexpr uint32_t idesc_f16_f32(int M, int N) {
 // and B type fields), D = F32, both K-major.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+// The same with both operands MN-major (transpose bits 15 and 16): each
+// 16-byte row of a core matrix holds 8 consecutive M (or N) elements of one K.
+__host__ __device__ constexpr uint32_t idesc_bf16_f32_mn(int M, int N) {
+  return idesc_bf16_f32(M, N) | (1u << 15) | (1u << 16);
 }
 
 // Instruction descriptor, kind::tf32: A = B = TF32 (format 2 in the A and B

@@ -727,7 +727,7 @@ dw_tc_kernel(Staging st, uint32_t ntiles, float* __restrict__ dw, uint32_t* __re
       if (!tc::mbar_wait_sleep(&S.full[i % kTcStages], (i / kTcStages) & 1u)) atomicExch(err, kErrTimeout);
     }
   } else if (warp == 1 && lane == 0) {  // MMA issuer
-    constexpr uint32_t id1 = tc::idesc_bf16_f32(128, 144), id2 = tc::idesc_bf16_f32(128, 80);
+    constexpr uint32_t id1 = tc::idesc_bf16_f32_mn(128, 144), id2 = tc::idesc_bf16_f32_mn(128, 80);
     for (uint32_t i = 0; i < my; ++i) {
       const int sidx = (int)(i % kTcStages);
       if (!tc::mbar_wait_sleep(&S.full[sidx], (i / kTcStages) & 1u)) {
@@ -944,58 +944,28 @@ __global__ void pack_bt_images_kernel(const float* __restrict__ w, uint8_t* __re
 
 __device__ __forceinline__ uint32_t f2u(float v) { return __float_as_uint(v); }
 
-// Staging of features f..f+7 (f % 8 == 0) of this thread's record as BF16,
-// in the canonical K-major layout of a 16-bit tensor-core operand with
-// K = record: 8 features x 8 records per 128-byte core matrix (16-byte rows,
-// one feature each), record groups of 8 at 128 B, feature groups of 8 at
-// 512 B; an F-wide array's 32-record tile is F x 64 contiguous bytes.  The
-// eight lanes of an octet hold eight consecutive records; an 8x8 transpose of
-// 16-bit values inside the octet -- packed halves exchanged with the
-// neighbouring lane, then a 4x4 transpose of 32-bit words across lanes 2 and
-// 4 apart, six shuffles -- leaves lane r with feature f + r of all eight
-// records: one 16-byte row.  A warp's 32 records are one tile, so each call
-// writes one contiguous 512-byte block.  Every lane of the warp must call it.
 // Two FP32 values -> packed BF16 (round to nearest even), lo in the low half.
 __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
+
+// Staging of features f..f+7 (f % 8 == 0) of this thread's record as BF16,
+// in the canonical MN-major layout of a 16-bit tensor-core operand with
+// K = record: a record's 8 features are one 16-byte row, 8 records a 128-byte
+// core matrix, record groups of 8 at 128 B, feature groups of 8 at 512 B; an
+// F-wide array's 32-record tile is F x 64 contiguous bytes.  A thread's row
+// needs nothing from its neighbours and a warp's 32 rows are one contiguous
+// 512-byte block.  (The K-major layout, whose rows hold one feature of 8
+// records, took an 8x8 transpose by six shuffles per call: 45 of the backward
+// phase's 161 ms at 122 M records.)
 __device__ __forceinline__ void stage8(float* arr, int F, uint32_t s, int f, float a0, float a1, float a2, float a3,
                                        float a4, float a5, float a6, float a7, bool stage) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t w[4] = {bf16x2(a0, a1), bf16x2(a2, a3), bf16x2(a4, a5), bf16x2(a6, a7)};  // low half: even feature
-  // Records 2p and 2p + 1 (lanes r and r ^ 1): the even lane keeps the even
-  // features of both, the odd lane the odd ones.
-  const bool even = (lane & 1u) == 0u;
-  const uint32_t give = even ? 0x7632u : 0x5410u;  // the halves the neighbour keeps
-  const uint32_t r0 = __shfl_xor_sync(0xffffffffu, __byte_perm(w[0], w[1], give), 1);
-  const uint32_t r1 = __shfl_xor_sync(0xffffffffu, __byte_perm(w[2], w[3], give), 1);
-  uint32_t z0, z1, z2, z3;  // z_j: feature 2j + (lane & 1) of records 2p, 2p + 1
-  if (even) {
-    z0 = __byte_perm(w[0], r0, 0x5410u);
-    z1 = __byte_perm(w[1], r0, 0x7610u);
-    z2 = __byte_perm(w[2], r1, 0x5410u);
-    z3 = __byte_perm(w[3], r1, 0x7610u);
-  } else {
-    z0 = __byte_perm(r0, w[0], 0x7610u);
-    z1 = __byte_perm(r0, w[1], 0x7632u);
-    z2 = __byte_perm(r1, w[2], 0x7610u);
-    z3 = __byte_perm(r1, w[3], 0x7632u);
-  }
-  // 4x4 transpose over (record pair p = lane bits 1-2, j).
-  const bool odd = (lane >> 1) & 1u, hi = (lane >> 2) & 1u;
-  uint32_t t = __shfl_xor_sync(0xffffffffu, odd ? z0 : z1, 2);
-  if (odd) z0 = t; else z1 = t;
-  t = __shfl_xor_sync(0xffffffffu, odd ? z2 : z3, 2);
-  if (odd) z2 = t; else z3 = t;
-  t = __shfl_xor_sync(0xffffffffu, hi ? z0 : z2, 4);
-  if (hi) z0 = t; else z2 = t;
-  t = __shfl_xor_sync(0xffffffffu, hi ? z1 : z3, 4);
-  if (hi) z1 = t; else z3 = t;
   if (stage) {
     uint8_t* tile = reinterpret_cast<uint8_t*>(arr) + (size_t)(s >> 5) * (size_t)F * 64u;
-    *reinterpret_cast<uint4*>(tile + (f >> 3) * 512 + (lane >> 3) * 128 + (lane & 7u) * 16) = make_uint4(z0, z1, z2, z3);
+    *reinterpret_cast<uint4*>(tile + (f >> 3) * 512 + (s & 31u) * 16) =
+        make_uint4(bf16x2(a0, a1), bf16x2(a2, a3), bf16x2(a4, a5), bf16x2(a6, a7));
   }
 }
 
