@@ -7,30 +7,31 @@
 // Per step:
 //  1. rays: (view, pixel) pairs (drawn from the step seed or given) -> the
 //     FP32 ray set-up of rendering, with the target colour and depth;
-//  2. forward: the rays' occupied steps listed (thread per ray), the field
-//     evaluated at every listed sample (by default the MLP products on the
-//     tensor cores as 3xTF32, FP32-level; exact_weight_grads = 1: FP32 on the
-//     CUDA cores), then each ray composited with early termination (thread
-//     per ray), keeping each
-//     evaluated sample's t, alpha, transmittance and colour in the ray's
-//     scratch row; loss; then walk the samples backwards carrying
+//  2. forward, as many rays at a time as the sample list holds: the rays'
+//     occupied steps listed (thread per ray), each listed sample's hash-grid
+//     encoding gathered (encode_kernel; kept for the backward), the MLPs
+//     evaluated (by default on the tensor cores as 3xTF32, FP32-level;
+//     exact_weight_grads = 1: FP32 on the CUDA cores), then each ray
+//     composited with early termination (thread per ray), keeping each
+//     evaluated sample's t, alpha, transmittance and colour at its place in
+//     the list; loss; then walk the samples backwards carrying
 //     A = dL/dT_k for each one's compositing adjoint
 //        g_w = g_C . c_k + g_D t_k,   dL/dc_k = g_C w_k,
 //        dL/dsigma_k = dt T_{k+1} (g_w - A_{k+1}),
 //        A_k = g_w alpha_k + A_{k+1} (1 - alpha_k),   A_K = 0,
 //     with g_C = 2 (C - C*)/B and g_D = 2 lambda (D - D*)/B, written as a
-//     compact 32-byte record (position, ray, dsigma, dc).  The backward
-//     sweep keeps every term proportional to T_{k+1}; the equivalent
+//     compact 32-byte record (position, place in the list, dsigma, dc).  The
+//     backward sweep keeps every term proportional to T_{k+1}; the equivalent
 //     forward form with suffix sums (C - prefix) cancels in FP32 late in
 //     the ray;
-//  3. backward (thread per record, in chunks): recompute the encoding and
-//     both MLPs, backpropagate, scatter-add the encoding gradient into the
-//     FP32 gradient table with float2 atomics, and stage every layer's input
-//     activations and output deltas.  By default the ten layer products of
-//     the recompute and the backpropagation run on the tensor cores
-//     (backward_tc_kernel, tcgen05 kind::tf32) and the staging is BF16;
-//     exact_weight_grads = 1 keeps them in FP32 on the CUDA cores
-//     (backward_kernel) with FP32 staging;
+//  3. backward (thread per record, in chunks): recompute both MLPs from the
+//     kept encoding, backpropagate, and stage every layer's input activations
+//     and output deltas.  By default the ten layer products of the recompute
+//     and the backpropagation run on the tensor cores (backward_tc_kernel,
+//     tcgen05 kind::tf32), the staging is BF16 and scatter_kernel adds the
+//     encoding gradients into the FP32 gradient table; exact_weight_grads = 1
+//     keeps the products in FP32 on the CUDA cores with FP32 staging and
+//     scatter-adds in the same kernel (backward_kernel);
 //  4. weight gradients: per layer dW[out][in] += sum_s delta[s][out] act[s][in]
 //     over the chunk (by default dw_tc_kernel, tcgen05 kind::f16 with BF16
 //     operands; exact: dw_kernel, register-tiled split-K reduction);
@@ -39,6 +40,7 @@
 // perturbed, for central finite differences.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -70,13 +72,13 @@ struct TrainRay {
   float tr, tg, tb, td;  // target colour and depth
 };
 
-struct ScratchSample {  // pass-1 state of one evaluated sample
+struct ScratchSample {  // state of one evaluated sample, at its place in the sample list
   float t, alpha, T, cr, cg, cb, pad0, pad1;  // T: transmittance before the sample
 };
 
 struct SampleRec {  // compacted sample with its compositing adjoint
   float x, y, z;
-  uint32_t ray;
+  uint32_t place;  // in the sample list
   float dsigma, dcr, dcg, dcb;
 };
 
@@ -158,91 +160,178 @@ __global__ void make_rays_kernel(const int2* __restrict__ pairs, int n, const Tr
 
 struct RayOut {  // composited result of one training ray
   float C0, C1, C2, D;
-  int K;           // evaluated samples up to early termination, in the ray's scratch row
-  uint32_t first;  // the ray's occupied steps in the sample list: [first, first + count)
+  int K;           // evaluated samples up to early termination
+  uint32_t first;  // the ray's occupied steps in the sample list, from its block's first one (block_first)
   uint32_t count;
   int pad;
 };
 
-// Forward, in three passes, so that the per-sample MLP runs with every lane
-// of a warp busy (marched one ray per thread, the lanes whose ray is at an
-// empty step would idle while the others evaluate) or on the tensor cores in
-// 128-sample tiles:
-//  1. enumerate_kernel, thread per ray: the ray's occupied steps in order --
-//     the march's sample set before early termination -- listed contiguously
-//     as (ray, k | step << 16), k the sample's index along the ray;
-//  2. eval_kernel (FP32, thread per listed sample) or eval_tc_kernel (the
+// Forward, in passes over the batch's samples, so that the per-sample work
+// runs with every lane of a warp busy (marched one ray per thread, the lanes
+// whose ray is at an empty step would idle while the others evaluate) or on
+// the tensor cores in 128-sample tiles:
+//  1. count_kernel and scan_kernel: the rays' occupied steps -- the march's
+//     sample set before early termination -- counted, and their places in a
+//     list of all of them, ray after ray;
+// then for as many rays at a time as kListSamples samples hold:
+//  2. list_kernel, thread per ray: (ray, step) of each sample;
+//  3. encode_kernel, thread per listed sample: the hash-grid encoding, kept
+//     for the backward (a warp's samples are consecutive samples of one or two
+//     rays: coherent gathers);
+//  4. eval_kernel (FP32, thread per listed sample) or eval_tc_kernel (the
 //     MLP products on tcgen05 as 3xTF32, thread = TMEM lane per sample): the
-//     encoding and MLPs at that sample, its t, alpha and colour written to the
-//     ray's scratch row k (a warp's samples are consecutive samples of one or
-//     two rays: coherent gathers);
-//  3. composite_kernel, thread per ray: the ray's rows in order, composited
+//     MLPs at that sample, its t, alpha and colour written to the sample's
+//     place;
+//  5. composite_kernel, thread per ray: the ray's samples in order, composited
 //     and stopped at T < kTStop exactly as a one-pass march composites, with
-//     each row's transmittance and the ray's RayOut filled in.
+//     each sample's transmittance and the ray's RayOut filled in.
 // With eval_kernel the per-sample arithmetic is the one-pass FP32 march's;
 // only the samples after an early termination are evaluated and then left
 // unused.
-constexpr uint32_t kListStepShift = 16;
-static_assert(kMaxSteps <= (1 << kListStepShift), "k and step share one word");
+constexpr int kRayBlock = 256;  // rays per block of the per-ray kernels
+constexpr uint32_t kListSamples = 1u << 26;  // samples listed at a time
+static_assert((uint32_t)kRayBlock * kMaxSteps <= kListSamples, "a block of rays fits the list");
 
-__global__ void __launch_bounds__(256)
-enumerate_kernel(const TrainRay* __restrict__ rays, int n, const DevScene sc, uint2* __restrict__ list,
-                 uint32_t capacity, RayOut* __restrict__ rout, uint32_t* __restrict__ cursor,
-                 uint32_t* __restrict__ err) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned lane = threadIdx.x & 31u;
+__global__ void __launch_bounds__(kRayBlock)
+count_kernel(const TrainRay* __restrict__ rays, int n, const DevScene sc, RayOut* __restrict__ rout,
+             uint32_t* __restrict__ block_count) {
+  __shared__ uint32_t warp_sum[kRayBlock / 32];
+  const int i = blockIdx.x * kRayBlock + threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   TrainRay r{};
   if (i < n) r = rays[i];
   const float3 o = make_float3(r.ox, r.oy, r.oz), d = make_float3(r.dx, r.dy, r.dz);
-  int cnt = 0;
+  uint32_t cnt = 0;
   for (int st = 0; st < r.n; ++st)
     if (occupied(sc.occ, sample_pos(o, d, fmaf((float)st + 0.5f, kDt, r.ts)))) ++cnt;
-  int incl = cnt;
+  uint32_t incl = cnt;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, off);
-    if ((int)lane >= off) incl += v;
+    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += v;
   }
-  uint32_t base = 0;
-  if (lane == 31 && incl > 0) base = atomicAdd(cursor, (uint32_t)incl);
-  base = __shfl_sync(0xffffffffu, base, 31) + (uint32_t)(incl - cnt);
-  if (i >= n) return;
-  RayOut ro{};
-  ro.first = base;
-  if (cnt > 0 && (base > capacity || (uint32_t)cnt > capacity - base)) {
-    atomicExch(err, kErrOverflow);
-  } else if (cnt > 0) {
-    ro.count = (uint32_t)cnt;
-    uint32_t k = 0;
-    for (int st = 0; st < r.n; ++st)
-      if (occupied(sc.occ, sample_pos(o, d, fmaf((float)st + 0.5f, kDt, r.ts)))) {
-        list[base + k] = make_uint2((uint32_t)i, k | ((uint32_t)st << kListStepShift));
-        ++k;
-      }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  uint32_t before = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kRayBlock / 32; ++w) {
+    before += w < warp ? warp_sum[w] : 0u;
+    total += warp_sum[w];
   }
-  rout[i] = ro;
+  if (threadIdx.x == 0) block_count[blockIdx.x] = total;
+  if (i < n) {
+    RayOut ro{};
+    ro.first = before + incl - cnt;
+    ro.count = cnt;
+    rout[i] = ro;
+  }
 }
 
-// Persistent grid-stride over the list; its length is the enumeration's
-// cursor (read on the device: no host round trip between the passes).
+// block_first[b] = samples of the blocks before b (one block of 1,024 threads;
+// block_first[blocks] = all samples).
+constexpr int kScanThreads = 1024, kScanItems = 4;
+static_assert((1 << 20) / kRayBlock <= kScanThreads * kScanItems, "one scan block covers the largest batch");
+__global__ void __launch_bounds__(kScanThreads)
+scan_kernel(const uint32_t* __restrict__ block_count, int blocks, uint32_t* __restrict__ block_first) {
+  __shared__ uint32_t warp_sum[kScanThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i0 = threadIdx.x * kScanItems;
+  uint32_t v[kScanItems], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    v[k] = i0 + k < blocks ? block_count[i0 + k] : 0u;
+    sum += v[k];
+  }
+  uint32_t incl = sum;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += u;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  uint32_t first = incl - sum;
+  for (int w = 0; w < warp; ++w) first += warp_sum[w];
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    if (i0 + k <= blocks) block_first[i0 + k] = first;
+    first += v[k];
+  }
+}
+
+// The samples of rays [0, n) from list place 0 (the rays' blocks start at
+// sample `base` of the batch).
+__global__ void __launch_bounds__(kRayBlock)
+list_kernel(const TrainRay* __restrict__ rays, int n, const DevScene sc, const RayOut* __restrict__ rout,
+            const uint32_t* __restrict__ block_first, uint32_t base, uint2* __restrict__ list) {
+  const int i = blockIdx.x * kRayBlock + threadIdx.x;
+  if (i >= n) return;
+  const TrainRay r = rays[i];
+  const float3 o = make_float3(r.ox, r.oy, r.oz), d = make_float3(r.dx, r.dy, r.dz);
+  uint2* out = list + (block_first[blockIdx.x] - base + rout[i].first);
+  for (int st = 0; st < r.n; ++st)
+    if (occupied(sc.occ, sample_pos(o, d, fmaf((float)st + 0.5f, kDt, r.ts)))) *out++ = make_uint2((uint32_t)i, (uint32_t)st);
+}
+
+// Encodings of the listed samples, FP32: 32-sample tiles of 8 chunks, a
+// chunk four features (two levels) of the tile's samples, 16 bytes each.
+constexpr int kEncTileFloats = kEnc * 32;
+__device__ __forceinline__ float4* enc_chunk(float* enc, uint32_t sample, int chunk) {
+  return reinterpret_cast<float4*>(enc + (size_t)(sample >> 5) * kEncTileFloats + chunk * 128 + (sample & 31u) * 4);
+}
+__device__ __forceinline__ float4 enc_chunk(const float* __restrict__ enc, uint32_t sample, int chunk) {
+  return __ldg(reinterpret_cast<const float4*>(enc + (size_t)(sample >> 5) * kEncTileFloats + chunk * 128 + (sample & 31u) * 4));
+}
+
+// Gathering in a kernel of its own lets every SM hold as many samples as its
+// registers allow and overlap their table reads; inside the MLP kernels only
+// the 256 or 512 threads that TMEM has room for did, twice per sample: 58 of
+// the backward phase's 161 ms and 16 of the forward's 50 ms at 122 M samples.
+constexpr int kEncThreads = 256;
+__global__ void __launch_bounds__(kEncThreads)
+encode_kernel(const uint2* __restrict__ list, uint32_t m, const TrainRay* __restrict__ rays, const DevScene sc,
+              float* __restrict__ enc) {
+  const uint32_t j = blockIdx.x * kEncThreads + threadIdx.x;
+  if (j >= m) return;
+  const uint2 e = list[j];
+  const TrainRay& r = rays[e.x];
+  const float t = fmaf((float)e.y + 0.5f, kDt, r.ts);
+  const float3 x = sample_pos(make_float3(r.ox, r.oy, r.oz), make_float3(r.dx, r.dy, r.dz), t);
+#pragma unroll
+  for (int c = 0; c < kEnc / 4; ++c) {
+    float4 f;
+    encode_level_fp32(sc.table32, sc.T, sc.dense_mask, x, 2 * c, f.x, f.y);
+    encode_level_fp32(sc.table32, sc.T, sc.dense_mask, x, 2 * c + 1, f.z, f.w);
+    *enc_chunk(enc, j, c) = f;
+  }
+}
+
+// All 32 features of a listed sample.
+__device__ __forceinline__ void load_enc(const float* __restrict__ enc, uint32_t sample, float (&f)[kEnc]) {
+#pragma unroll
+  for (int c = 0; c < kEnc / 4; ++c) {
+    const float4 v = enc_chunk(enc, sample, c);
+    f[4 * c + 0] = v.x;
+    f[4 * c + 1] = v.y;
+    f[4 * c + 2] = v.z;
+    f[4 * c + 3] = v.w;
+  }
+}
+
+// Persistent grid-stride over the list.
 __global__ void __launch_bounds__(kFwdThreads)
-eval_kernel(const uint2* __restrict__ list, const uint32_t* __restrict__ total, uint32_t capacity,
-            const TrainRay* __restrict__ rays, int n, const DevScene sc, ScratchSample* __restrict__ scratch) {
+eval_kernel(const uint2* __restrict__ list, uint32_t m, const TrainRay* __restrict__ rays, const DevScene sc,
+            const float* __restrict__ encs, ScratchSample* __restrict__ scratch) {
   extern __shared__ float4 smem_raw[];
   SmemWeights32& W = *reinterpret_cast<SmemWeights32*>(smem_raw);
   load_weights32(W, sc.weights);
   __syncthreads();
-  const uint32_t m = min(*total, capacity);
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
     const uint2 e = list[j];
-    const uint32_t k = e.y & ((1u << kListStepShift) - 1u), st = e.y >> kListStepShift;
-    if (e.x >= (uint32_t)n || k >= (uint32_t)kMaxSteps) continue;  // only after an overflow (flagged)
     const TrainRay& r = rays[e.x];
-    const float3 o = make_float3(r.ox, r.oy, r.oz), d = make_float3(r.dx, r.dy, r.dz);
-    const float t = fmaf((float)st + 0.5f, kDt, r.ts);
-    const float3 x = sample_pos(o, d, t);
+    const float3 d = make_float3(r.dx, r.dy, r.dz);
+    const float t = fmaf((float)e.y + 0.5f, kDt, r.ts);
     float enc[kEnc];
-    encode_fp32(sc.table32, sc.T, sc.dense_mask, x, enc);
+    load_enc(encs, j, enc);
     float dout[kDOut];
     density_mlp32(W, enc, dout);
     const float sigma = expf(dout[0] - 1.0f);
@@ -250,16 +339,17 @@ eval_kernel(const uint2* __restrict__ list, const uint32_t* __restrict__ total, 
     sh16(d, sh);
     const float3 c = colour_mlp32(W, sh, dout);
     const float alpha = -expm1f(-sigma * kDt);
-    scratch[(size_t)e.x * kMaxSteps + k] = ScratchSample{t, alpha, 0.0f, c.x, c.y, c.z, 0.0f, 0.0f};
+    scratch[j] = ScratchSample{t, alpha, 0.0f, c.x, c.y, c.z, 0.0f, 0.0f};
   }
 }
 
-__global__ void __launch_bounds__(256)
-composite_kernel(int n, ScratchSample* __restrict__ scratch, RayOut* __restrict__ rout) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kRayBlock)
+composite_kernel(int n, ScratchSample* __restrict__ scratch, const uint32_t* __restrict__ block_first, uint32_t base,
+                 RayOut* __restrict__ rout) {
+  const int i = blockIdx.x * kRayBlock + threadIdx.x;
   if (i >= n) return;
   RayOut ro = rout[i];
-  ScratchSample* row = scratch + (size_t)i * kMaxSteps;
+  ScratchSample* row = scratch + (block_first[blockIdx.x] - base + ro.first);
   float T = 1.0f, C0 = 0.0f, C1 = 0.0f, C2 = 0.0f, D = 0.0f;
   int K = 0;
   bool stop = false;
@@ -296,12 +386,13 @@ composite_kernel(int n, ScratchSample* __restrict__ scratch, RayOut* __restrict_
 // Loss and compositing adjoint, thread per ray: the ray's samples are walked
 // backwards carrying A = dL/dT (see the file comment) and written as compact
 // records; one record-range atomic per warp (warp prefix sum of K).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kRayBlock)
 adjoint_kernel(const TrainRay* __restrict__ rays, const RayOut* __restrict__ rout, int n,
-               const ScratchSample* __restrict__ scratch, SampleRec* __restrict__ recs, uint32_t capacity,
+               const ScratchSample* __restrict__ scratch, const uint32_t* __restrict__ block_first, uint32_t list_base,
+               SampleRec* __restrict__ recs, uint32_t capacity,
                uint32_t* __restrict__ cursor, uint32_t* __restrict__ err, double* __restrict__ loss_sum,
                float depth_w, float inv_n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * kRayBlock + threadIdx.x;
   const unsigned lane = threadIdx.x & 31u;
   TrainRay r{};
   RayOut ro{};
@@ -329,7 +420,8 @@ adjoint_kernel(const TrainRay* __restrict__ rays, const RayOut* __restrict__ rou
       const float gC0 = 2.0f * ec0 * inv_n, gC1 = 2.0f * ec1 * inv_n, gC2 = 2.0f * ec2 * inv_n;
       const float gD = 2.0f * depth_w * ed * inv_n;
       const float3 o = make_float3(r.ox, r.oy, r.oz), d = make_float3(r.dx, r.dy, r.dz);
-      const ScratchSample* row = scratch + (size_t)i * kMaxSteps;
+      const uint32_t place = block_first[blockIdx.x] - list_base + ro.first;
+      const ScratchSample* row = scratch + place;
       float A = 0.0f;
       // Rows in batches of kBatch from the back, all loaded before the
       // first is used (the loads do not wait on the sweep's arithmetic).
@@ -349,7 +441,7 @@ adjoint_kernel(const TrainRay* __restrict__ rays, const RayOut* __restrict__ rou
           const float gw = fmaf(gC0, q.cr, fmaf(gC1, q.cg, fmaf(gC2, q.cb, gD * q.t)));
           const float dsig = kDt * T1 * (gw - A);
           const float3 x = sample_pos(o, d, q.t);
-          recs[base + k] = SampleRec{x.x, x.y, x.z, (uint32_t)i, dsig, gC0 * w, gC1 * w, gC2 * w};
+          recs[base + k] = SampleRec{x.x, x.y, x.z, place + (uint32_t)k, dsig, gC0 * w, gC1 * w, gC2 * w};
           A = fmaf(gw, q.alpha, A * (1.0f - q.alpha));
         }
       }
@@ -385,8 +477,9 @@ struct SmemBackward {
 };
 
 __global__ void __launch_bounds__(kBwdThreads, 2)
-backward_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t count, const TrainRay* __restrict__ rays,
-                const DevScene sc, Staging st, float2* __restrict__ gtable) {
+backward_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t count, const uint2* __restrict__ list,
+                const TrainRay* __restrict__ rays, const float* __restrict__ encs, const DevScene sc, Staging st,
+                float2* __restrict__ gtable) {
   extern __shared__ float4 smem_raw[];
   SmemBackward& S = *reinterpret_cast<SmemBackward*>(smem_raw);
   SmemWeights32& W = S.w;
@@ -421,7 +514,7 @@ backward_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t cou
   float* const r_dlog = stage_row(st.dlog, 8, s);
   // ---- forward recompute ----
   float enc[kEnc];
-  encode_fp32(sc.table32, sc.T, sc.dense_mask, x, enc);
+  load_enc(encs, q.place, enc);
 #pragma unroll
   for (int k = 0; k < kEnc; ++k) r_enc[soff(k)] = enc[k];
   float out[kDOut];
@@ -446,7 +539,7 @@ backward_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t cou
   const float sigma = expf(out[0] - 1.0f);
   float cin[kCIn];
   {
-    const TrainRay& r = rays[q.ray];
+    const TrainRay& r = rays[list[q.place].x];
     sh16(make_float3(r.dx, r.dy, r.dz), cin);
   }
 #pragma unroll
@@ -807,83 +900,112 @@ constexpr int kBtGroups = 4;
 constexpr int kBtThreads = 128 * kBtGroups;
 constexpr uint32_t kBtColsPerGroup = 128;  // A: 64 columns, D: 64 columns
 
-// Hash-grid scatter-add of one record's encoding gradient,
-// dtable[l][corner] += w_corner * denc[2l..2l+1].  Every lane of the warp
-// calls it (valid = false for a lane without a record).  A warp's records
-// are consecutive samples of one or two rays, so at the coarse levels runs
-// of neighbouring lanes share a cell: levels 0..kAggLevels-1 sum each run's
-// corner gradients with shuffles and add them with one atomic per run.
+// Hash-grid scatter-add of one record's encoding gradient (d0, d1) at level L,
+// dtable[L][corner] += w_corner * d.  Every lane of the warp calls it (valid =
+// false for a lane without a record).  A warp's records are consecutive
+// samples of one or two rays, so at the coarse levels runs of neighbouring
+// lanes share a cell: levels 0..kAggLevels-1 sum each run's corner gradients
+// with shuffles and add them with one atomic per run.  Corners k and k + 1 are
+// one aligned entry pair {i, i ^ 1} half the time (a dense level's even index;
+// a hashed level's even x, the x prime being 1): one 16-byte atomic then.
+__constant__ int level_res_table[kLevels] = {level_res(0),  level_res(1),  level_res(2),  level_res(3),
+                                            level_res(4),  level_res(5),  level_res(6),  level_res(7),
+                                            level_res(8),  level_res(9),  level_res(10), level_res(11),
+                                            level_res(12), level_res(13), level_res(14), level_res(15)};
 constexpr int kAggLevels = 13;  // levels whose scatter-add is warp-aggregated (N <= 776)
 static_assert(level_res(kAggLevels - 1) < 1024, "cell key packs 10 bits per coordinate");
 
-__device__ __forceinline__ void scatter_add_levels(float2* __restrict__ gtable, const DevScene& sc, float3 x,
-                                                   const float (&denc)[kEnc], bool valid, uint32_t lane) {
-#pragma unroll 1
-  for (int l = 0; l < kLevels; ++l) {
-    const int N = level_res(l);
-    const LevelCell c = level_cell(x, N);
-    uint32_t idx[8];
-    corner_indices(c, N, (sc.dense_mask >> l) & 1u, sc.T, idx);
-    float w[8];
-    corner_weights(c, w);
-    float2* gt = gtable + (size_t)l * sc.T;
-    float d0 = 0.0f, d1 = 0.0f;
-#pragma unroll
-    for (int k = 0; k < kLevels; ++k)
-      if (k == l) {
-        d0 = denc[2 * k];
-        d1 = denc[2 * k + 1];
-      }
-    if (l >= kAggLevels) {
-      if (valid && !((sc.dense_mask >> l) & 1u) && (c.ix & 1u) == 0u) {
-        // Hashed level, even x: the x prime is 1, so corners k and k + 1
-        // are the aligned entry pair {i, i ^ 1}; one 16-byte atomic each.
-#pragma unroll
-        for (int k = 0; k < 8; k += 2) {
-          const uint32_t i = idx[k];
-          const float4 v = (i & 1u) ? make_float4(w[k + 1] * d0, w[k + 1] * d1, w[k] * d0, w[k] * d1)
-                                    : make_float4(w[k] * d0, w[k] * d1, w[k + 1] * d0, w[k + 1] * d1);
-          atomicAdd(reinterpret_cast<float4*>(gt + (i & ~1u)), v);
-        }
-      } else if (valid) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) atomicAdd(gt + idx[k], make_float2(w[k] * d0, w[k] * d1));
-      }
-      continue;
-    }
-    // Runs of lanes with the same cell (invalid lanes form runs of their
-    // own and add nothing).  N <= 776 here: 10 bits per coordinate.
+__device__ __forceinline__ void add_pair(float2* __restrict__ gt, uint32_t i, uint32_t j, float2 a, float2 b) {
+  if ((i ^ j) == 1u) {
+    const float4 v = (i & 1u) ? make_float4(b.x, b.y, a.x, a.y) : make_float4(a.x, a.y, b.x, b.y);
+    atomicAdd(reinterpret_cast<float4*>(gt + (i & ~1u)), v);
+  } else {
+    atomicAdd(gt + i, a);
+    atomicAdd(gt + j, b);
+  }
+}
+
+__device__ __forceinline__ void scatter_add_level(int L, int N, float2* __restrict__ gtable, uint32_t T,
+                                                  uint32_t dense_mask, const float3& x, float d0, float d1, bool valid,
+                                                  uint32_t lane) {
+  const LevelCell c = level_cell(x, N);
+  uint32_t idx[8];
+  corner_indices(c, N, (dense_mask >> L) & 1u, T, idx);
+  float w[8];
+  corner_weights(c, w);
+  float2* gt = gtable + (size_t)L * T;
+  uint32_t heads = 0xffffffffu;  // lanes that start a run
+  if (L < kAggLevels) {
+    // Runs of lanes with the same cell (invalid lanes form runs of their own
+    // and add nothing).  N <= 776 here: 10 bits per coordinate.
     const uint32_t key = valid ? (c.ix | (c.iy << 10) | (c.iz << 20)) : (0x80000000u | lane);
     const uint32_t kprev = __shfl_up_sync(0xffffffffu, key, 1);
-    const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || kprev != key);
-    if (heads == 0xffffffffu) {  // no lane shares its cell
-      if (valid)
+    heads = __ballot_sync(0xffffffffu, lane == 0 || kprev != key);
+  }
+  if (heads == 0xffffffffu) {  // no lane shares its cell
+    if (valid)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) atomicAdd(gt + idx[k], make_float2(w[k] * d0, w[k] * d1));
-      continue;
+      for (int k = 0; k < 8; k += 2)
+        add_pair(gt, idx[k], idx[k + 1], make_float2(w[k] * d0, w[k] * d1), make_float2(w[k + 1] * d0, w[k + 1] * d1));
+    return;
+  }
+  // Step o adds the partial sum of lane + o when no run starts in (lane, lane
+  // + o]; afterwards each run's first lane holds its total.  Steps beyond the
+  // warp's longest run are left out (more[b]: some run has over 2^b lanes).
+  uint32_t more = ~heads, take = 0;
+  int steps = 0;
+#pragma unroll
+  for (int o = 1, b = 0; o < 32; o <<= 1, ++b) {
+    const uint32_t span = (uint32_t)(((1ull << o) - 1ull) << (lane + 1));  // lanes lane+1 .. lane+o
+    if (lane + o < 32u && (heads & span) == 0u) take |= 1u << b;
+    if (more != 0u) steps = b + 1;
+    more &= more >> o;
+  }
+  const bool add = valid && ((heads >> lane) & 1u);
+  float a[16];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    a[2 * k] = w[k] * d0;
+    a[2 * k + 1] = w[k] * d1;
+  }
+  for (int b = 0; b < steps; ++b) {
+    const bool t = (take >> b) & 1u;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const float p = __shfl_down_sync(0xffffffffu, a[e], 1 << b);
+      if (t) a[e] += p;
     }
-    // Step o adds the partial sum of lane + o when no run starts in
-    // (lane, lane + o]; afterwards each run's first lane holds its total.
-    uint32_t take = 0;
+  }
+  if (add)
 #pragma unroll
-    for (int o = 1, b = 0; o < 32; o <<= 1, ++b) {
-      const uint32_t span = (uint32_t)(((1ull << o) - 1ull) << (lane + 1));  // lanes lane+1 .. lane+o
-      if (lane + o < 32u && (heads & span) == 0u) take |= 1u << b;
-    }
-    const bool head = (heads >> lane) & 1u;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      float a0 = w[k] * d0, a1 = w[k] * d1;
-#pragma unroll
-      for (int o = 1, b = 0; o < 32; o <<= 1, ++b) {
-        const float p0 = __shfl_down_sync(0xffffffffu, a0, o), p1 = __shfl_down_sync(0xffffffffu, a1, o);
-        if ((take >> b) & 1u) {
-          a0 += p0;
-          a1 += p1;
-        }
-      }
-      if (valid && head) atomicAdd(gt + idx[k], make_float2(a0, a1));
-    }
+    for (int k = 0; k < 8; k += 2)
+      add_pair(gt, idx[k], idx[k + 1], make_float2(a[2 * k], a[2 * k + 1]), make_float2(a[2 * k + 2], a[2 * k + 3]));
+}
+
+// The encoding gradients of `count` records from `first` -> the gradient table.
+// In a kernel of its own the atomics of 36 warps per SM overlap, where the
+// backward's TMEM leaves 16; it is bound by them: 73 sectors a record, 0.92 ms
+// per 2^22 records = 330 G sectors/s (inside the MLP kernel it took 44 of 161
+// ms at 122 M records, here 27).
+constexpr int kScatThreads = 256;
+__global__ void __launch_bounds__(kScatThreads)
+scatter_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t count, const DevScene sc,
+               const float* __restrict__ denc, float2* __restrict__ gtable) {
+  const uint32_t s = blockIdx.x * kScatThreads + threadIdx.x;
+  const bool valid = s < count;
+  float3 x = make_float3(0.0f, 0.0f, 0.0f);
+  if (valid) {
+    const float4 q = __ldg(reinterpret_cast<const float4*>(recs + first + s));
+    x = make_float3(q.x, q.y, q.z);
+  }
+  // One copy of the level's code: unrolled, the sixteen levels overran the
+  // instruction caches.
+#pragma unroll 1
+  for (int l = 0; l < kLevels; ++l) {
+    float2 d = make_float2(0.0f, 0.0f);
+    if (valid) d = __ldg(reinterpret_cast<const float2*>(denc + (size_t)(s >> 5) * kEncTileFloats + (l >> 1) * 128 +
+                                                         (s & 31u) * 4 + (l & 1) * 2));
+    scatter_add_level(l, level_res_table[l], gtable, sc.T, sc.dense_mask, x, d.x, d.y, valid, threadIdx.x & 31u);
   }
 }
 
@@ -971,8 +1093,9 @@ __device__ __forceinline__ void stage8(float* arr, int F, uint32_t s, int f, flo
 
 __global__ void __launch_bounds__(kBtThreads, 1)
 backward_tc_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t count,
-                   const TrainRay* __restrict__ rays, const DevScene sc, const uint8_t* __restrict__ images,
-                   Staging st, float2* __restrict__ gtable, uint32_t* __restrict__ err) {
+                   const uint2* __restrict__ list, const TrainRay* __restrict__ rays, const float* __restrict__ encs,
+                   const uint8_t* __restrict__ images, Staging st, float* __restrict__ denc,
+                   uint32_t* __restrict__ err) {
   extern __shared__ __align__(128) uint8_t smem_bt[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_bt + kBtImageBytes);  // [group] mma, [kBtGroups] weights
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + kBtGroups + 1);
@@ -1034,18 +1157,16 @@ backward_tc_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t 
       if (valid) {
         q = recs[first + s];
       } else {
-        q.x = q.y = q.z = 0.0f;
-        q.ray = 0;
+        q.place = 0;
         q.dsigma = q.dcr = q.dcg = q.dcb = 0.0f;
       }
-      const float3 x = make_float3(q.x, q.y, q.z);
       uint32_t u[32];
       float v[32];
       // ---- forward recompute ----
       {
         float enc[kEnc];
         if (valid) {
-          encode_fp32(sc.table32, sc.T, sc.dense_mask, x, enc);
+          load_enc(encs, q.place, enc);
         } else {
 #pragma unroll
           for (int k = 0; k < kEnc; ++k) enc[k] = 0.0f;
@@ -1082,7 +1203,7 @@ backward_tc_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t 
         tc::tmem_ld16(d_row, reinterpret_cast<float(&)[16]>(out));
         sigma = expf(out[0] - 1.0f);
         float cin[kCIn];
-        const TrainRay& r = rays[q.ray];
+        const TrainRay& r = rays[list[q.place].x];
         sh16(make_float3(r.dx, r.dy, r.dz), cin);
 #pragma unroll
         for (int k = 0; k < 15; ++k) cin[16 + k] = out[1 + k];
@@ -1152,7 +1273,9 @@ backward_tc_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t 
       if (!mma(9)) break;
       tc::tmem_ld32(d_row, v);  // denc
       // The next tile's first product overwrites D: its sync follows these reads.
-      scatter_add_levels(gtable, sc, x, v, valid, (uint32_t)(tid & 31));
+      if (valid)
+#pragma unroll
+        for (int k = 0; k < kEnc; k += 4) *enc_chunk(denc, s, k / 4) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
     }
   }
   if (fail || !ok) atomicExch(err, kErrTimeout);
@@ -1179,10 +1302,10 @@ constexpr int kBtSmem = (int)kBtImageBytes + 8 * (kBtGroups + 1) + 16;
 // issues the three K-chains against the weight images' high and low parts in
 // shared memory, and every thread reads its row of D back for the
 // elementwise step (ReLU, exp, SH, sigmoid) and the next layer's input.  The
-// table gathers of the group's next tile run while the MMAs of layers 1-4 of
-// the current one do (four levels per layer), into TMEM columns of their own
+// encodings of the group's next tile are read while the MMAs of layers 1-4 of
+// the current one run (four levels per layer), into TMEM columns of their own
 // that layer 0 of the next tile reads: only two tiles' worth of warps per SM
-// fit the TMEM, so the gathers' latency is hidden behind the layer chain.
+// fit the TMEM, so the reads' latency is hidden behind the layer chain.
 constexpr int kEtGroups = 2;
 constexpr int kEtThreads = 128 * kEtGroups;
 // A_hi: 0..63, A_lo: 64..127, D: 128..191, next tile's encoding E_hi:
@@ -1216,27 +1339,21 @@ __global__ void pack_et_images_kernel(const float* __restrict__ w, uint8_t* __re
 
 // One listed sample's inputs.
 struct EtSample {
-  uint32_t ray, k;
   float t;
-  float3 o, d;
+  float3 d;
   bool valid;
 };
 
 __device__ __forceinline__ EtSample et_sample(const uint2* __restrict__ list, uint32_t j, uint32_t m,
-                                              const TrainRay* __restrict__ rays, int n) {
+                                              const TrainRay* __restrict__ rays) {
   EtSample q;
-  const uint2 e = j < m ? list[j] : make_uint2(0xFFFFFFFFu, 0u);
-  q.ray = e.x;
-  q.k = e.y & ((1u << kListStepShift) - 1u);
-  // (an out-of-range entry exists only after an overflow, which is flagged)
-  q.valid = j < m && q.ray < (uint32_t)n && q.k < (uint32_t)kMaxSteps;
+  q.valid = j < m;
   q.t = 0.0f;
-  q.o = make_float3(0.0f, 0.0f, 0.0f);
   q.d = make_float3(0.0f, 0.0f, 1.0f);
   if (q.valid) {
-    const TrainRay& r = rays[q.ray];
-    q.t = fmaf((float)(e.y >> kListStepShift) + 0.5f, kDt, r.ts);
-    q.o = make_float3(r.ox, r.oy, r.oz);
+    const uint2 e = list[j];
+    const TrainRay& r = rays[e.x];
+    q.t = fmaf((float)e.y + 0.5f, kDt, r.ts);
     q.d = make_float3(r.dx, r.dy, r.dz);
   }
   return q;
@@ -1245,22 +1362,20 @@ __device__ __forceinline__ EtSample et_sample(const uint2* __restrict__ list, ui
 // Levels L0..L0+3 of a sample's encoding -> E_hi / E_lo columns 2 L0 ..
 // 2 L0 + 7 of this thread's lane (no wait).  Every lane of the warp calls it.
 template <int L0>
-__device__ __forceinline__ void et_encode4(const DevScene& sc, const EtSample& q, uint32_t ehi_row,
+__device__ __forceinline__ void et_encode4(const float* __restrict__ encs, uint32_t j, bool valid, uint32_t ehi_row,
                                            uint32_t elo_row) {
-  float f[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) f[j] = 0.0f;
-  if (q.valid) {
-    const float3 x = sample_pos(q.o, q.d, q.t);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) encode_level_fp32(sc.table32, sc.T, sc.dense_mask, x, L0 + j, f[2 * j], f[2 * j + 1]);
+  float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+  if (valid) {
+    a = enc_chunk(encs, j, L0 / 2);
+    b = enc_chunk(encs, j, L0 / 2 + 1);
   }
+  const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   uint32_t h[8], l[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float hi = tf32_hi(f[j]);
-    h[j] = __float_as_uint(hi);
-    l[j] = __float_as_uint(f[j] - hi);
+  for (int k = 0; k < 8; ++k) {
+    const float hi = tf32_hi(f[k]);
+    h[k] = __float_as_uint(hi);
+    l[k] = __float_as_uint(f[k] - hi);
   }
   tc::tmem_st4(ehi_row + 2 * L0, h[0], h[1], h[2], h[3]);
   tc::tmem_st4(ehi_row + 2 * L0 + 4, h[4], h[5], h[6], h[7]);
@@ -1269,9 +1384,9 @@ __device__ __forceinline__ void et_encode4(const DevScene& sc, const EtSample& q
 }
 
 __global__ void __launch_bounds__(kEtThreads, 1)
-eval_tc_kernel(const uint2* __restrict__ list, const uint32_t* __restrict__ total, uint32_t capacity,
-               const TrainRay* __restrict__ rays, int n, const DevScene sc, const uint8_t* __restrict__ images,
-               ScratchSample* __restrict__ scratch, uint32_t* __restrict__ err) {
+eval_tc_kernel(const uint2* __restrict__ list, uint32_t m, const TrainRay* __restrict__ rays,
+               const float* __restrict__ encs, const uint8_t* __restrict__ images, ScratchSample* __restrict__ scratch,
+               uint32_t* __restrict__ err) {
   extern __shared__ __align__(128) uint8_t smem_et[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_et + kEtImageBytes);  // [group] mma, [kEtGroups] images
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + kEtGroups + 1);
@@ -1360,28 +1475,28 @@ eval_tc_kernel(const uint2* __restrict__ list, const uint32_t* __restrict__ tota
     }
   };
 
-  const uint32_t m = min(*total, capacity);
   const uint32_t ntiles = (m + 127u) / 128u;
   const uint32_t stride = gridDim.x * kEtGroups;
   uint32_t tile = blockIdx.x * kEtGroups + g;
   if (!fail && tile < ntiles) {
-    // The first tile's encoding; later tiles' are gathered during the
-    // previous tile's layers.
-    EtSample cur = et_sample(list, tile * 128u + (uint32_t)row, m, rays, n);
-    et_encode4<0>(sc, cur, ehi_row, elo_row);
-    et_encode4<4>(sc, cur, ehi_row, elo_row);
-    et_encode4<8>(sc, cur, ehi_row, elo_row);
-    et_encode4<12>(sc, cur, ehi_row, elo_row);
-    for (; tile < ntiles; tile += stride) {
-      const bool more = tile + stride < ntiles;
-      const EtSample nxt = et_sample(list, (tile + stride) * 128u + (uint32_t)row, more ? m : 0u, rays, n);
+    // The first tile's encoding; later tiles' are read during the previous
+    // tile's layers.
+    uint32_t j = tile * 128u + (uint32_t)row;
+    EtSample cur = et_sample(list, j, m, rays);
+    et_encode4<0>(encs, j, cur.valid, ehi_row, elo_row);
+    et_encode4<4>(encs, j, cur.valid, ehi_row, elo_row);
+    et_encode4<8>(encs, j, cur.valid, ehi_row, elo_row);
+    et_encode4<12>(encs, j, cur.valid, ehi_row, elo_row);
+    for (; tile < ntiles; tile += stride, j += stride * 128u) {
+      const uint32_t jn = j + stride * 128u;
+      const EtSample nxt = et_sample(list, jn, tile + stride < ntiles ? m : 0u, rays);
       float x[64];
       if (!issue(0, ehi_col, elo_col)) break;  // h1 = relu(enc dW1^T)
       wait();
       relu64(x);
       put(x, kHid);
       if (!issue(1, hi_col, lo_col)) break;  // out = h1 dW2^T
-      et_encode4<0>(sc, nxt, ehi_row, elo_row);
+      et_encode4<0>(encs, jn, nxt.valid, ehi_row, elo_row);
       wait();
       float sigma;
       {
@@ -1398,24 +1513,24 @@ eval_tc_kernel(const uint2* __restrict__ list, const uint32_t* __restrict__ tota
       }
       put(x, kCIn);
       if (!issue(2, hi_col, lo_col)) break;  // g1 = relu(cin cW1^T)
-      et_encode4<4>(sc, nxt, ehi_row, elo_row);
+      et_encode4<4>(encs, jn, nxt.valid, ehi_row, elo_row);
       wait();
       relu64(x);
       put(x, kHid);
       if (!issue(3, hi_col, lo_col)) break;  // g2 = relu(g1 cW2^T)
-      et_encode4<8>(sc, nxt, ehi_row, elo_row);
+      et_encode4<8>(encs, jn, nxt.valid, ehi_row, elo_row);
       wait();
       relu64(x);
       put(x, kHid);
       if (!issue(4, hi_col, lo_col)) break;  // logit = g2 cW3^T
-      et_encode4<12>(sc, nxt, ehi_row, elo_row);
+      et_encode4<12>(encs, jn, nxt.valid, ehi_row, elo_row);
       wait();
       float lg[16];
       tc::tmem_ld16(d_row, lg);
       // The next tile's first product overwrites D: its sync follows these reads.
       if (cur.valid) {
         const float alpha = -expm1f(-sigma * kDt);
-        scratch[(size_t)cur.ray * kMaxSteps + cur.k] =
+        scratch[j] =
             ScratchSample{cur.t, alpha, 0.0f, sigmoidf(lg[0]), sigmoidf(lg[1]), sigmoidf(lg[2]), 0.0f, 0.0f};
       }
       cur = nxt;
@@ -1596,24 +1711,33 @@ struct nes_trainer {
   uint32_t max_rays = 0;
   int2* d_pairs = nullptr;
   TrainRay* d_rays = nullptr;
-  ScratchSample* d_scratch = nullptr;  // max_rays * kMaxSteps
+  // Per listed sample (list_capacity of each): list entry, encoding, state
+  // and record of the backward.
+  uint32_t list_capacity = 0;
+  uint2* d_list = nullptr;
+  float* d_enc = nullptr;
+  ScratchSample* d_scratch = nullptr;
   SampleRec* d_recs = nullptr;
-  uint32_t rec_capacity = 0;
-  uint32_t* d_ctr = nullptr;  // [0] record cursor, [1] error word, [2] sample-list cursor
+  uint32_t* d_ctr = nullptr;  // [0] record cursor, [1] error word
   RayOut* d_rout = nullptr;
+  uint32_t* d_block_count = nullptr;  // samples per block of kRayBlock rays
+  uint32_t* d_block_first = nullptr;  // and before each block (one more entry: all)
+  uint32_t* h_block_first = nullptr;  // pinned copy
   double* d_loss = nullptr;
   float2* d_gtable = nullptr;
   float* d_gw = nullptr;
   float *d_mt = nullptr, *d_vt = nullptr, *d_mw = nullptr, *d_vw = nullptr;
   float* d_stage = nullptr;
+  float* d_denc = nullptr;  // encoding gradients of a tensor-core backward chunk, tiled as d_enc
   uint8_t* d_bimg = nullptr;  // TF32 weight images of backward_tc_kernel
   uint8_t* d_eimg = nullptr;  // high/low TF32 forward images of eval_tc_kernel
   uint32_t chunk = 0;
   int fwd_blocks = 0;  // persistent eval_kernel grid: SMs x resident blocks
   uint64_t steps = 0;
   uint64_t last_samples = 0;
-  // Phase events on the trainer's stream: 0 forward start, 1 forward end,
-  // 2 backward + weight-gradient end, 3 Adam start, 4 Adam end.
+  // Phase events on the trainer's stream: 0 start of a part's forward, 1 its
+  // end, 2 end of the part's backward and weight gradients (read before the
+  // next part records them), 3 Adam start, 4 Adam end.
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   float phase_ms[3] = {0.0f, 0.0f, 0.0f};
 };
@@ -1654,88 +1778,126 @@ cudaError_t launch_dw(const float* act, const float* delta, uint32_t S, float* d
   return cudaGetLastError();
 }
 
-// Loss and gradients (accumulated into d_gtable / d_gw) for the n rays in d_rays.
-int loss_and_grad(nes_trainer* t, int n, double* loss) {
+// Backward of the `total` records in d_recs, accumulated into d_gtable / d_gw.
+int backward_records(nes_trainer* t, const TrainRay* rays, uint32_t total) {
   nes_ctx* c = t->ctx;
-  TR_CUDA(cudaMemsetAsync(t->d_loss, 0, sizeof(double), t->st));
-  TR_CUDA(cudaMemsetAsync(t->d_ctr, 0, sizeof(uint32_t), t->st));  // the error word is cleared by the caller
-  TR_CUDA(cudaMemsetAsync(t->d_ctr + 2, 0, sizeof(uint32_t), t->st));
-  TR_CUDA(cudaEventRecord(t->ev[0], t->st));
-  // The sample list lives in the records' buffer until the adjoint (after
-  // the composite) writes the records there.
-  uint2* list = reinterpret_cast<uint2*>(t->d_recs);
-  const uint32_t list_capacity = t->rec_capacity;  // SampleRec slots hold at least as many uint2
-  enumerate_kernel<<<(n + 255) / 256, 256, 0, t->st>>>(t->d_rays, n, c->scene, list, list_capacity, t->d_rout,
-                                                       t->d_ctr + 2, t->d_ctr + 1);
-  TR_CUDA(cudaGetLastError());
-  if (t->cfg.exact_weight_grads) {
-    eval_kernel<<<t->fwd_blocks, kFwdThreads, kSmemW, t->st>>>(list, t->d_ctr + 2, list_capacity, t->d_rays, n,
-                                                            c->scene, t->d_scratch);
-  } else {  // this step's weights as high/low TF32 operand images
-    pack_et_images_kernel<<<(kFwdImageBytes / 4 + 255) / 256, 256, 0, t->st>>>(c->d_weights, t->d_eimg);
-    TR_CUDA(cudaGetLastError());
-    eval_tc_kernel<<<c->num_sms, kEtThreads, kEtSmem, t->st>>>(list, t->d_ctr + 2, list_capacity, t->d_rays, n,
-                                                             c->scene, t->d_eimg, t->d_scratch, t->d_ctr + 1);
-  }
-  TR_CUDA(cudaGetLastError());
-  composite_kernel<<<(n + 255) / 256, 256, 0, t->st>>>(n, t->d_scratch, t->d_rout);
-  TR_CUDA(cudaGetLastError());
-  adjoint_kernel<<<(n + 255) / 256, 256, 0, t->st>>>(t->d_rays, t->d_rout, n, t->d_scratch, t->d_recs,
-                                                     t->rec_capacity, t->d_ctr, t->d_ctr + 1, t->d_loss,
-                                                     t->cfg.depth_weight, 1.0f / (float)n);
-  TR_CUDA(cudaGetLastError());
-  TR_CUDA(cudaEventRecord(t->ev[1], t->st));
-  uint32_t h[2] = {0, 0};
-  TR_CUDA(cudaMemcpyAsync(h, t->d_ctr, sizeof(h), cudaMemcpyDeviceToHost, t->st));
-  TR_CUDA(cudaMemcpyAsync(loss, t->d_loss, sizeof(double), cudaMemcpyDeviceToHost, t->st));
-  TR_CUDA(cudaStreamSynchronize(t->st));
-  if (h[1] == kErrOverflow) return NES_ENOMEM;
-  if (h[1] == kErrTimeout) return NES_ETIMEDOUT;
-  if (h[1]) return NES_EINVAL;
-  const uint32_t total = h[0];
-  t->last_samples = total;
   const Staging sg = staging(t);
   float* gw = t->d_gw;
   const int sms = c->num_sms;
-  if (!t->cfg.exact_weight_grads) {  // this step's weights as TF32 operand images
-    pack_bt_images_kernel<<<(kBtImageBytes / 4 + 255) / 256, 256, 0, t->st>>>(c->d_weights, t->d_bimg);
-    TR_CUDA(cudaGetLastError());
-  }
   // BF16 staging (tensor-core mode) holds twice the records in the same bytes.
   const uint32_t chunk = t->cfg.exact_weight_grads ? t->chunk : 2u * t->chunk;
   for (uint32_t first = 0; first < total; first += chunk) {
     const uint32_t cnt = total - first < chunk ? total - first : chunk;
     if (t->cfg.exact_weight_grads) {
       backward_kernel<<<(cnt + kBwdThreads - 1) / kBwdThreads, kBwdThreads, kSmemB, t->st>>>(
-          t->d_recs, first, cnt, t->d_rays, c->scene, sg, t->d_gtable);
-    } else {
-      const uint32_t groups = (cnt + 127u) / 128u;
-      const uint32_t want = (groups + kBtGroups - 1) / kBtGroups;
-      backward_tc_kernel<<<want < (uint32_t)sms ? want : (uint32_t)sms, kBtThreads, kBtSmem, t->st>>>(
-          t->d_recs, first, cnt, t->d_rays, c->scene, t->d_bimg, sg, t->d_gtable, t->d_ctr + 1);
-    }
-    TR_CUDA(cudaGetLastError());
-    if (t->cfg.exact_weight_grads) {
+          t->d_recs, first, cnt, t->d_list, rays, t->d_enc, c->scene, sg, t->d_gtable);
+      TR_CUDA(cudaGetLastError());
       TR_CUDA((launch_dw<kEnc, kHid, kHid>(sg.enc, sg.dh1, cnt, gw + kOffDW1, sms, t->st)));
       TR_CUDA((launch_dw<kHid, kDOut, kDOut>(sg.h1, sg.dout, cnt, gw + kOffDW2, sms, t->st)));
       TR_CUDA((launch_dw<kCIn, kHid, kHid>(sg.cin, sg.dg1, cnt, gw + kOffCW1, sms, t->st)));
       TR_CUDA((launch_dw<kHid, kHid, kHid>(sg.g1, sg.dg2, cnt, gw + kOffCW2, sms, t->st)));
       TR_CUDA((launch_dw<kHid, 3, kFDlog>(sg.g2, sg.dlog, cnt, gw + kOffCW3, sms, t->st)));
     } else {
+      const uint32_t groups = (cnt + 127u) / 128u;
+      const uint32_t want = (groups + kBtGroups - 1) / kBtGroups;
+      backward_tc_kernel<<<want < (uint32_t)sms ? want : (uint32_t)sms, kBtThreads, kBtSmem, t->st>>>(
+          t->d_recs, first, cnt, t->d_list, rays, t->d_enc, t->d_bimg, sg, t->d_denc, t->d_ctr + 1);
+      TR_CUDA(cudaGetLastError());
+      scatter_kernel<<<(cnt + kScatThreads - 1) / kScatThreads, kScatThreads, 0, t->st>>>(
+          t->d_recs, first, cnt, c->scene, t->d_denc, t->d_gtable);
+      TR_CUDA(cudaGetLastError());
       const uint32_t tiles = (cnt + 31) / 32;
       const uint32_t grid = tiles < (uint32_t)sms ? tiles : (uint32_t)sms;
       dw_tc_kernel<<<grid, kDwTcThreads, sizeof(DwTcSmem), t->st>>>(sg, tiles, gw, t->d_ctr + 1);
       TR_CUDA(cudaGetLastError());
     }
   }
-  {  // a tensor-core wait that ran out reports through the error word
-    uint32_t e = 0;
-    TR_CUDA(cudaMemcpyAsync(&e, t->d_ctr + 1, sizeof(e), cudaMemcpyDeviceToHost, t->st));
-    TR_CUDA(cudaStreamSynchronize(t->st));
-    if (e == kErrTimeout) return NES_ETIMEDOUT;
-    if (e) return NES_EINVAL;
+  return NES_OK;
+}
+
+int train_error(uint32_t word) {
+  switch (word) {
+    case 0: return NES_OK;
+    case kErrOverflow: return NES_ENOMEM;
+    case kErrTimeout: return NES_ETIMEDOUT;
+    default: return NES_EINVAL;
   }
-  TR_CUDA(cudaEventRecord(t->ev[2], t->st));
+}
+
+// Loss and gradients (accumulated into d_gtable / d_gw) for the n rays in
+// d_rays, as many blocks of kRayBlock rays at a time as the sample list holds.
+int loss_and_grad(nes_trainer* t, int n, double* loss) {
+  nes_ctx* c = t->ctx;
+  const int blocks = (n + kRayBlock - 1) / kRayBlock;
+  t->last_samples = 0;
+  t->phase_ms[0] = t->phase_ms[1] = 0.0f;
+  TR_CUDA(cudaMemsetAsync(t->d_loss, 0, sizeof(double), t->st));
+  TR_CUDA(cudaEventRecord(t->ev[0], t->st));
+  count_kernel<<<blocks, kRayBlock, 0, t->st>>>(t->d_rays, n, c->scene, t->d_rout, t->d_block_count);
+  TR_CUDA(cudaGetLastError());
+  scan_kernel<<<1, kScanThreads, 0, t->st>>>(t->d_block_count, blocks, t->d_block_first);
+  TR_CUDA(cudaGetLastError());
+  TR_CUDA(cudaMemcpyAsync(t->h_block_first, t->d_block_first, (size_t)(blocks + 1) * sizeof(uint32_t),
+                          cudaMemcpyDeviceToHost, t->st));
+  if (!t->cfg.exact_weight_grads) {  // this step's weights as TF32 operand images
+    pack_et_images_kernel<<<(kFwdImageBytes / 4 + 255) / 256, 256, 0, t->st>>>(c->d_weights, t->d_eimg);
+    TR_CUDA(cudaGetLastError());
+    pack_bt_images_kernel<<<(kBtImageBytes / 4 + 255) / 256, 256, 0, t->st>>>(c->d_weights, t->d_bimg);
+    TR_CUDA(cudaGetLastError());
+  }
+  TR_CUDA(cudaStreamSynchronize(t->st));
+  const uint32_t* first = t->h_block_first;
+  for (int b0 = 0; b0 < blocks;) {
+    int b1 = b0 + 1;
+    while (b1 < blocks && first[b1 + 1] - first[b0] <= t->list_capacity) ++b1;
+    const uint32_t base = first[b0], m = first[b1] - base;
+    const int r0 = b0 * kRayBlock, nr = std::min(n, b1 * kRayBlock) - r0, nb = b1 - b0;
+    const TrainRay* rays = t->d_rays + r0;
+    RayOut* rout = t->d_rout + r0;
+    const uint32_t* block_first = t->d_block_first + b0;
+    if (b0 > 0) TR_CUDA(cudaEventRecord(t->ev[0], t->st));
+    TR_CUDA(cudaMemsetAsync(t->d_ctr, 0, sizeof(uint32_t), t->st));  // the error word is cleared by the caller
+    if (m > 0) {
+      list_kernel<<<nb, kRayBlock, 0, t->st>>>(rays, nr, c->scene, rout, block_first, base, t->d_list);
+      TR_CUDA(cudaGetLastError());
+      encode_kernel<<<(m + kEncThreads - 1) / kEncThreads, kEncThreads, 0, t->st>>>(t->d_list, m, rays, c->scene,
+                                                                                  t->d_enc);
+      TR_CUDA(cudaGetLastError());
+      if (t->cfg.exact_weight_grads)
+        eval_kernel<<<t->fwd_blocks, kFwdThreads, kSmemW, t->st>>>(t->d_list, m, rays, c->scene, t->d_enc,
+                                                                  t->d_scratch);
+      else
+        eval_tc_kernel<<<c->num_sms, kEtThreads, kEtSmem, t->st>>>(t->d_list, m, rays, t->d_enc, t->d_eimg,
+                                                                  t->d_scratch, t->d_ctr + 1);
+      TR_CUDA(cudaGetLastError());
+    }
+    composite_kernel<<<nb, kRayBlock, 0, t->st>>>(nr, t->d_scratch, block_first, base, rout);
+    TR_CUDA(cudaGetLastError());
+    adjoint_kernel<<<nb, kRayBlock, 0, t->st>>>(rays, rout, nr, t->d_scratch, block_first, base, t->d_recs,
+                                                t->list_capacity, t->d_ctr, t->d_ctr + 1, t->d_loss,
+                                                t->cfg.depth_weight, 1.0f / (float)n);
+    TR_CUDA(cudaGetLastError());
+    TR_CUDA(cudaEventRecord(t->ev[1], t->st));
+    uint32_t h[2] = {0, 0};
+    TR_CUDA(cudaMemcpyAsync(h, t->d_ctr, sizeof(h), cudaMemcpyDeviceToHost, t->st));
+    TR_CUDA(cudaMemcpyAsync(loss, t->d_loss, sizeof(double), cudaMemcpyDeviceToHost, t->st));
+    TR_CUDA(cudaStreamSynchronize(t->st));
+    int rc = train_error(h[1]);
+    if (rc != NES_OK) return rc;
+    t->last_samples += h[0];
+    if ((rc = backward_records(t, rays, h[0])) != NES_OK) return rc;
+    TR_CUDA(cudaEventRecord(t->ev[2], t->st));
+    // A tensor-core wait that ran out reports through the error word.
+    TR_CUDA(cudaMemcpyAsync(h, t->d_ctr, sizeof(h), cudaMemcpyDeviceToHost, t->st));
+    TR_CUDA(cudaStreamSynchronize(t->st));
+    if ((rc = train_error(h[1])) != NES_OK) return rc;
+    float ms = 0.0f;
+    TR_CUDA(cudaEventElapsedTime(&ms, t->ev[0], t->ev[1]));
+    t->phase_ms[0] += ms;
+    TR_CUDA(cudaEventElapsedTime(&ms, t->ev[1], t->ev[2]));
+    t->phase_ms[1] += ms;
+    b0 = b1;
+  }
   return NES_OK;
 }
 
@@ -1767,8 +1929,6 @@ int adam(nes_trainer* t) {
   TR_CUDA(cudaGetLastError());
   TR_CUDA(cudaEventRecord(t->ev[4], t->st));
   TR_CUDA(cudaStreamSynchronize(t->st));
-  TR_CUDA(cudaEventElapsedTime(&t->phase_ms[0], t->ev[0], t->ev[1]));
-  TR_CUDA(cudaEventElapsedTime(&t->phase_ms[1], t->ev[1], t->ev[2]));
   TR_CUDA(cudaEventElapsedTime(&t->phase_ms[2], t->ev[3], t->ev[4]));
   return NES_OK;
 }
@@ -1777,8 +1937,13 @@ void free_trainer(nes_trainer* t) {
   cudaFree(t->d_views);
   cudaFree(t->d_pairs);
   cudaFree(t->d_rays);
+  cudaFree(t->d_list);
+  cudaFree(t->d_enc);
   cudaFree(t->d_scratch);
   cudaFree(t->d_recs);
+  cudaFree(t->d_block_count);
+  cudaFree(t->d_block_first);
+  if (t->h_block_first) cudaFreeHost(t->h_block_first);
   cudaFree(t->d_rout);
   cudaFree(t->d_ctr);
   cudaFree(t->d_loss);
@@ -1789,6 +1954,7 @@ void free_trainer(nes_trainer* t) {
   cudaFree(t->d_mw);
   cudaFree(t->d_vw);
   cudaFree(t->d_stage);
+  cudaFree(t->d_denc);
   cudaFree(t->d_bimg);
   cudaFree(t->d_eimg);
   for (cudaEvent_t e : t->ev)
@@ -1834,11 +2000,18 @@ int nes_trainer_create(nes_ctx* ctx, const nes_train_config* cfg, nes_trainer** 
   for (cudaEvent_t& e : t->ev)
     if (cudaEventCreate(&e) != cudaSuccess) return fail(NES_EIO);
   const size_t nt = (size_t)kLevels * ctx->scene.T * 2;
-  const size_t max_samples = (size_t)t->max_rays * kMaxSteps;  // every step of every ray: never overflows
-  t->rec_capacity = (uint32_t)max_samples;
+  // Every step of every ray, or as many samples as are listed at a time.
+  const size_t blocks = (t->max_rays + kRayBlock - 1) / kRayBlock;
+  const size_t max_samples = std::min<size_t>((size_t)t->max_rays * kMaxSteps, kListSamples);
+  t->list_capacity = (uint32_t)max_samples;
   t->chunk = 1u << 21;
   if (cudaMalloc(&t->d_pairs, (size_t)t->max_rays * sizeof(int2)) != cudaSuccess ||
       cudaMalloc(&t->d_rays, (size_t)t->max_rays * sizeof(TrainRay)) != cudaSuccess ||
+      cudaMalloc(&t->d_list, max_samples * sizeof(uint2)) != cudaSuccess ||
+      cudaMalloc(&t->d_enc, (max_samples + 31) / 32 * kEncTileFloats * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&t->d_block_count, blocks * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMalloc(&t->d_block_first, (blocks + 1) * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMallocHost(&t->h_block_first, (blocks + 1) * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&t->d_scratch, max_samples * sizeof(ScratchSample)) != cudaSuccess ||
       cudaMalloc(&t->d_recs, max_samples * sizeof(SampleRec)) != cudaSuccess ||
       cudaMalloc(&t->d_rout, (size_t)t->max_rays * sizeof(RayOut)) != cudaSuccess ||
@@ -1851,6 +2024,8 @@ int nes_trainer_create(nes_ctx* ctx, const nes_train_config* cfg, nes_trainer** 
       cudaMalloc(&t->d_mw, kWeightFloats * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&t->d_vw, kWeightFloats * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&t->d_stage, (size_t)t->chunk * kStageFloats * sizeof(float)) != cudaSuccess ||
+      (!cfg->exact_weight_grads &&
+       cudaMalloc(&t->d_denc, (size_t)2 * t->chunk * kEnc * sizeof(float)) != cudaSuccess) ||
       cudaMalloc(&t->d_bimg, kBtImageBytes) != cudaSuccess ||
       cudaMalloc(&t->d_eimg, kEtImageBytes) != cudaSuccess)
     return fail(NES_ENOMEM);
