@@ -125,49 +125,67 @@ __device__ __forceinline__ uint32_t interp_lerp(const __half2 (&e)[8], float fx,
   return h2u(__hfma2(hz, __hsub2(b1, b0), b0));
 }
 
+// Cell coordinate and fraction along one axis, p = x N with x in [0, 1): p is
+// rounded down to a multiple of 1 by adding 2^23 (round towards minus
+// infinity), so the sum's bits are 0x4B000000 + the cell and no conversion is
+// needed.  Index arithmetic carries the bias along: the record and dense
+// forms subtract its multiple as a constant, the hashed form masks it away
+// (its low 24 bits, and those of its multiples, are zero; T <= 2^24).
+constexpr uint32_t kCellBias = 0x4B000000u;
+__device__ __forceinline__ uint32_t biased_cell(float p, float* f) {
+  const float t = __fadd_rd(p, 8388608.0f);
+  *f = p - (t - 8388608.0f);
+  return __float_as_uint(t);
+}
+
 // Level L of the FP16 table at x -> its two features packed as FP16.
-// Instruction-lean form of the trilinear interpolation (the march is
-// issue-bound here): integer floor/clamp for the cell, hash terms masked
+// Instruction-lean form of the trilinear interpolation (encoder instructions
+// lengthen the march: 5 % more of them cost 4 %): conversion-free cells
+// without a clamp (no coordinate is 1, see last_below_one), hash terms masked
 // once so each corner index is one 3-input XOR, and the interpolation as
 // packed FP16 lerps (interp_lerp).
 // The recorded levels (0..kRec-1) also exist as per-cell records: the 8 corner
 // entries of every cell (c = dx + 2 dy + 4 dz) in 32 contiguous bytes, so a
-// sample's level costs two 16-byte loads instead of eight scattered 4-byte
+// sample's level costs one 32-byte load instead of eight scattered 4-byte
 // gathers (the encoder is bound by L1 wavefronts).  The records are copies of
 // table entries (built by build_records_kernel), so the result is the same.
 // Records of levels kEvictFirstFrom and up are read once per sample and come
-// from HBM (cells smaller than a sample step): they are loaded with an L2
-// evict-first policy so that they do not displace the table and the coarser
-// records, which are reused (1080p march 24.2 -> 23.6 ms; from level 7 up: no
-// gain, those records are still reused).
+// from HBM (cells smaller than a sample step): they are loaded L2 evict-first
+// so that they do not displace the table and the coarser records, which are
+// reused (1080p march 24.2 -> 23.6 ms; from level 7 up: no gain, those records
+// are still reused).  1080p march: 23.8 ms with integer conversions, clamps
+// and two 16-byte loads per record, 23.4 without the clamps, 23.1 with all of
+// this (256-bit loads alone: 24.1).
 constexpr int kEvictFirstFrom = 10;
 
-__device__ __forceinline__ uint4 ldg_evict_first(const uint4* p, uint64_t policy) {
-  uint4 r;
-  asm("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
-      : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-      : "l"(p), "l"(policy));
-  return r;
+// The largest float below 1 in place of 1: the cell of x = 1 is the last one
+// and its fraction rounds to 1 in FP16, as clamping the cell index gives it.
+__device__ __forceinline__ float3 last_below_one(const float3& x) {
+  return make_float3(fminf(x.x, 0x1.fffffep-1f), fminf(x.y, 0x1.fffffep-1f), fminf(x.z, 0x1.fffffep-1f));
+}
+
+template <bool kEvictFirst>
+__device__ __forceinline__ void load_record(const uint4* p, uint4* a, uint4* b) {
+  if constexpr (kEvictFirst)
+    asm("ld.global.nc.L2::evict_first.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(a->x), "=r"(a->y), "=r"(a->z), "=r"(a->w), "=r"(b->x), "=r"(b->y), "=r"(b->z), "=r"(b->w)
+        : "l"(p));
+  else
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(a->x), "=r"(a->y), "=r"(a->z), "=r"(a->w), "=r"(b->x), "=r"(b->y), "=r"(b->z), "=r"(b->w)
+        : "l"(p));
 }
 
 template <int L>
 __device__ __forceinline__ uint32_t encode_level_rec(const uint4* __restrict__ rec, const float3& x) {
-  constexpr int N = level_res(L);
-  const float px = x.x * (float)N, py = x.y * (float)N, pz = x.z * (float)N;
-  const int ix = min(__float2int_rd(px), N - 1), iy = min(__float2int_rd(py), N - 1),
-            iz = min(__float2int_rd(pz), N - 1);
-  const float fx = px - (float)ix, fy = py - (float)iy, fz = pz - (float)iz;
-  const uint32_t cell = rec_cell_offset(L) + (uint32_t)ix + (uint32_t)N * ((uint32_t)iy + (uint32_t)N * (uint32_t)iz);
+  constexpr uint32_t N = (uint32_t)level_res(L);
+  float fx, fy, fz;
+  const uint32_t ix = biased_cell(x.x * (float)N, &fx), iy = biased_cell(x.y * (float)N, &fy),
+                 iz = biased_cell(x.z * (float)N, &fz);
+  constexpr uint32_t kFirst = rec_cell_offset(L) - kCellBias * (1u + N + N * N);
+  const uint32_t cell = kFirst + ix + N * (iy + N * iz);
   uint4 a, b;
-  if constexpr (L >= kEvictFirstFrom) {
-    uint64_t policy;
-    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
-    a = ldg_evict_first(rec + 2 * cell, policy);
-    b = ldg_evict_first(rec + 2 * cell + 1, policy);
-  } else {
-    a = __ldg(rec + 2 * cell);
-    b = __ldg(rec + 2 * cell + 1);
-  }
+  load_record<(L >= kEvictFirstFrom)>(rec + 2 * (size_t)cell, &a, &b);
   __half2 e[8];
   e[0] = *reinterpret_cast<const __half2*>(&a.x);
   e[1] = *reinterpret_cast<const __half2*>(&a.y);
@@ -183,22 +201,21 @@ __device__ __forceinline__ uint32_t encode_level_rec(const uint4* __restrict__ r
 template <int L>
 __device__ __forceinline__ uint32_t encode_level(const __half2* __restrict__ table, uint32_t T, uint32_t dense_mask,
                                                  const float3& x) {
-  constexpr int N = level_res(L);
-  const float px = x.x * (float)N, py = x.y * (float)N, pz = x.z * (float)N;
-  const int ix = min(__float2int_rd(px), N - 1), iy = min(__float2int_rd(py), N - 1),
-            iz = min(__float2int_rd(pz), N - 1);  // x >= 0, so the floor is >= 0
-  const float fx = px - (float)ix, fy = py - (float)iy, fz = pz - (float)iz;
+  constexpr uint32_t N = (uint32_t)level_res(L);
+  float fx, fy, fz;
+  const uint32_t ix = biased_cell(x.x * (float)N, &fx), iy = biased_cell(x.y * (float)N, &fy),
+                 iz = biased_cell(x.z * (float)N, &fz);
   uint32_t idx[8];
   if ((dense_mask >> L) & 1u) {
-    constexpr uint32_t s = (uint32_t)N + 1u;
-    const uint32_t b = (uint32_t)ix + s * ((uint32_t)iy + s * (uint32_t)iz);
+    constexpr uint32_t s = N + 1u;
+    const uint32_t b = (0u - kCellBias * (1u + s + s * s)) + ix + s * (iy + s * iz);
 #pragma unroll
     for (int k = 0; k < 8; ++k) idx[k] = b + (k & 1) + ((k >> 1) & 1) * s + ((k >> 2) & 1) * s * s;
   } else {
     const uint32_t m = T - 1u;
-    const uint32_t x0 = (uint32_t)ix & m, x1 = (uint32_t)(ix + 1) & m;
-    const uint32_t y0 = ((uint32_t)iy * kPrime1) & m, y1 = ((uint32_t)iy * kPrime1 + kPrime1) & m;
-    const uint32_t z0 = ((uint32_t)iz * kPrime2) & m, z1 = ((uint32_t)iz * kPrime2 + kPrime2) & m;
+    const uint32_t x0 = ix & m, x1 = (ix + 1u) & m;
+    const uint32_t y0 = (iy * kPrime1) & m, y1 = (iy * kPrime1 + kPrime1) & m;
+    const uint32_t z0 = (iz * kPrime2) & m, z1 = (iz * kPrime2 + kPrime2) & m;
 #pragma unroll
     for (int k = 0; k < 8; ++k) idx[k] = ((k & 1) ? x1 : x0) ^ ((k & 2) ? y1 : y0) ^ ((k & 4) ? z1 : z0);
   }
@@ -355,7 +372,7 @@ __device__ __forceinline__ bool encoder_loop(const ViewBatch& vb, const DevScene
     }
     float t;
     const bool has = take_step<kShift>(q, j, ray_lane, &t);
-    const float3 x = sample_pos_sat(q.o, q.d, t);
+    const float3 x = last_below_one(sample_pos_sat(q.o, q.d, t));
     const uint32_t tag = q.live ? kTagRay | (has ? kTagSample : 0u) | (first ? kTagFirst : 0u) : 0u;
     hand[b * 128 + row] = make_uint2(q.id | (tag << 28), __float_as_uint(t));
     const bool fin = exhausted && __ballot_sync(0xffffffffu, q.live) == 0u;
