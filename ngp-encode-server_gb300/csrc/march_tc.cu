@@ -303,22 +303,86 @@ constexpr uint32_t kTagSample = 1u, kTagFirst = 2u, kTagRay = 8u;
 // than a 4x8 patch of single steps.  Measured, ms with L2 flushed, one row per
 // ray (as it was) against 4, 8 and 32 steps:
 //                 rays     seeded scene                 opaque, sparse scene
-//   64x48         1.6k     4.7  -> 1.25, 0.70, 0.24     1.06 -> 0.31, 0.21, 0.15
-//   256x256       34k      4.7  -> 1.39, 0.90, 0.74     1.25 -> 0.39, 0.27, 0.31
-//   320x240       39k              1.39, 1.32, 1.08             0.41, 0.34, 0.44
-//   480x360       88k              2.53, 2.31, 2.22             0.60, 0.54, 0.83
-//   640x360       118k     4.9  -> 3.4,  3.7,  3.9
-//   1280x720      470k    13.4  -> 11.5, 12.5, 15.1
-//   1920x1080     1.06M   25.2  -> 23.8, 26.8, 33.3
-//   2x1920x1832           32.2  -> 29.8, 33.0, 40.8
-//   3x853x481                                           3.19 -> 2.08, 2.16, 4.1
+//   64x48         1.6k     4.7  -> 1.16, 0.70, 0.21     1.06 -> 0.30, 0.20, 0.15
+//   256x256       34k      4.7  -> 1.22, 0.79, 0.70     1.25 -> 0.35, 0.25, 0.29
+//   320x240       39k              1.24, 1.17, 0.99             0.37, 0.32, 0.40
+//   400x300       61k              1.82, 1.62, 1.48
+//   480x360       88k              2.14, 2.01, 2.01             0.53, 0.49, 0.70
+//   640x360       118k     4.9  -> 3.18, 3.14, 3.54             0.75, 0.70, 1.18
+//   853x480       210k             5.10, 5.15, 6.24             1.14, 1.15, 2.04
+//   1280x720      470k     13.4 -> 10.3, 10.6, 13.8
+//   1920x1080     1.06M    25.2 -> 21.4, 22.4, 30.5
+//   2x1920x1832            32.2 -> 26.8, 27.7, 37.4
+//   3x853x481                                           3.19 -> 1.94, 1.99, 3.67
 // Sixteen steps were slower than both neighbours from 256x256 up.  Within the
 // warp a ray's steps are neighbours: with the rays next to each other and the
-// steps apart the 1080p march took 25.1 ms, with both interleaved 24.1.
+// steps apart the 1080p march took 25.1 ms, with both interleaved 24.1, so 23.8.
 __device__ __forceinline__ uint32_t lane_shift(uint32_t nrays, uint32_t rows) {
   if (nrays <= rows / 2) return 5;
-  if (nrays <= rows + rows / 4) return 3;
+  if (nrays <= rows * 2) return 3;
   return 2;
+}
+
+// What a ray has gathered so far: every lane its transmittance, lane c of
+// each four the channel c (red, green, blue, expected depth).
+struct RayAcc {
+  float T = 1.0f, v = 0.0f;
+};
+
+// Composites the tile's samples of each ray (FP32, every operation rounded
+// explicitly): its rows, its next steps in order, one after another.  The
+// lanes of four transpose their samples' (r, g, b, t) so that each
+// accumulates one channel; the transmittance is every lane's.  True when it
+// fell below kTStop; later samples are then dropped.  1080p march 21.7 ms;
+// with all channels in every lane, five shuffles a sample, 21.9; with that
+// loop over the samples not unrolled, 23.1: the MLP warps' part of a tile is as
+// long as the encoders'.
+template <int kShift>
+__device__ __forceinline__ bool composite_tile(RayAcc& acc, bool open, bool sample, float alpha, const float (&c)[3],
+                                               float t, unsigned long long* samples) {
+  constexpr int kLanes = 1 << kShift;
+  const int lane = threadIdx.x & 31, ray_lane = lane & ~(kLanes - 1);
+  const uint32_t have = __ballot_sync(0xffffffffu, sample) >> ray_lane;
+  float m[4] = {c[0], c[1], c[2], t};  // own sample's channels -> own channel of the four lanes' samples
+  {
+    const bool o1 = lane & 1, o2 = lane & 2;
+    float u = __shfl_xor_sync(0xffffffffu, o1 ? m[0] : m[1], 1);
+    if (o1) m[0] = u; else m[1] = u;
+    u = __shfl_xor_sync(0xffffffffu, o1 ? m[2] : m[3], 1);
+    if (o1) m[2] = u; else m[3] = u;
+    u = __shfl_xor_sync(0xffffffffu, o2 ? m[0] : m[2], 2);
+    if (o2) m[0] = u; else m[2] = u;
+    u = __shfl_xor_sync(0xffffffffu, o2 ? m[1] : m[3], 2);
+    if (o2) m[1] = u; else m[3] = u;
+  }
+  bool stop = false;
+  uint32_t count = 0;
+#pragma unroll
+  for (int i = 0; i < kLanes; ++i) {
+    const float ai = __shfl_sync(0xffffffffu, alpha, ray_lane + i);
+    float vi = m[i & 3];
+    if constexpr (kLanes > 4) vi = __shfl_sync(0xffffffffu, vi, ray_lane + (i & ~3) + (lane & 3));
+    if (open && !stop && ((have >> i) & 1u)) {
+      ++count;
+      const float wgt = __fmul_rn(acc.T, ai);
+      acc.v = __fmaf_rn(wgt, vi, acc.v);
+      acc.T = __fsub_rn(acc.T, wgt);
+      stop = acc.T < kTStop;
+    }
+  }
+  *samples += count;
+  return stop;
+}
+
+// Channel c of a ray's pixel, by lane c of its first four.
+__device__ __forceinline__ void write_channel(const ViewBatch& vb, const DevScratch& s, uint32_t id, int c, float v) {
+  const RayMeta m = s.ray_meta[id];
+  const DevView& V = vb.v[m.view];
+  if (c < 3) {
+    if (V.rgb) V.rgb[(size_t)m.pixel * 3 + c] = v;
+  } else if (V.depth) {
+    V.depth[m.pixel] = v;
+  }
 }
 
 // The encoder warps' loop; true when a wait ran out.
@@ -459,9 +523,9 @@ march_tc_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScr
     constexpr uint32_t id64 = tc::idesc_f16_f32(128, 64), id16 = tc::idesc_f16_f32(128, 16);
     uint32_t pm = 0;
     uint32_t cur = kNoRay;  // ray being composited in this row
-    float T = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f, cz = 0.0f;
+    RayAcc acc;
     float dx = 0.0f, dy = 0.0f, dz = 1.0f;  // direction of the row's current ray
-    const int lanes = 1 << shift, ray_lane = lane & ~(lanes - 1);  // the row's ray: its lanes of the warp
+    const int ray_lane = lane & ~((1 << shift) - 1);  // first of the row's ray's lanes
 
     // Issues one layer (one thread) and waits for it (every thread); the
     // free barrier of the tile's buffer, if given, is released by the same
@@ -499,7 +563,7 @@ march_tc_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScr
       const uint32_t rid = hd.x & kIdMask, flags = hd.x >> 28;
       const float t = __uint_as_float(hd.y);
       if ((flags & kTagFirst) || !(flags & kTagRay)) {  // the row's ray, if it has not terminated, is complete
-        if (cur != kNoRay && lane == ray_lane) write_ray(vb, s, cur, cr, cg, cb, cz);
+        if (cur != kNoRay && lane - ray_lane < 4) write_channel(vb, s, cur, lane - ray_lane, acc.v);
         cur = kNoRay;
       }
       if (wfin[b * 4 + 0] & wfin[b * 4 + 1] & wfin[b * 4 + 2] & wfin[b * 4 + 3]) {
@@ -517,8 +581,7 @@ march_tc_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScr
         dy = rd.y;
         dz = rd.z;
         cur = rid;
-        T = 1.0f;
-        cr = cg = cb = cz = 0.0f;
+        acc = RayAcc();
       }
       const uint32_t a_col = enc_cols + 16 * b;  // encoded features of this tile
       // density 32 -> 64 -> 16 (the first layer is the features' last reader)
@@ -559,33 +622,16 @@ march_tc_kernel(const __grid_constant__ Src src, const DevScene sc, const DevScr
       layer(h_col, kWoffCW3, 64, id16, nullptr);
       float v5[16];
       tc::tmem_ld16(d_row, v5);
-      // Compositing (FP32, every operation rounded explicitly).  A ray's rows
-      // of the tile, its next steps in order, are composited one after another
-      // by each of its lanes alike.
       const float alpha = -expm1f(__fmul_rn(-sigma, kDt));
-      const float s0 = sigmoidf(v5[0]), s1 = sigmoidf(v5[1]), s2 = sigmoidf(v5[2]);
-      const uint32_t have = __ballot_sync(0xffffffffu, (flags & kTagSample) != 0u);
-      const bool open = cur != kNoRay;  // samples of a ray that already terminated are dropped
-      bool stop_early = false;
-      for (int i = 0; i < lanes; ++i) {
-        const float ai = __shfl_sync(0xffffffffu, alpha, ray_lane + i);
-        const float ri = __shfl_sync(0xffffffffu, s0, ray_lane + i);
-        const float gi = __shfl_sync(0xffffffffu, s1, ray_lane + i);
-        const float bi = __shfl_sync(0xffffffffu, s2, ray_lane + i);
-        const float ti = __shfl_sync(0xffffffffu, t, ray_lane + i);
-        if (open && !stop_early && ((have >> (ray_lane + i)) & 1u)) {
-          ++my_samples;
-          const float wgt = __fmul_rn(T, ai);
-          cr = __fmaf_rn(wgt, ri, cr);
-          cg = __fmaf_rn(wgt, gi, cg);
-          cb = __fmaf_rn(wgt, bi, cb);
-          cz = __fmaf_rn(wgt, ti, cz);
-          T = __fsub_rn(T, wgt);
-          stop_early = T < kTStop;
-        }
-      }
+      const float c3[3] = {sigmoidf(v5[0]), sigmoidf(v5[1]), sigmoidf(v5[2])};
+      const bool sample = (flags & kTagSample) != 0u;
+      // (samples of a ray that already terminated are dropped)
+      bool stop_early;
+      if (shift == 5) stop_early = composite_tile<5>(acc, cur != kNoRay, sample, alpha, c3, t, &my_samples);
+      else if (shift == 3) stop_early = composite_tile<3>(acc, cur != kNoRay, sample, alpha, c3, t, &my_samples);
+      else stop_early = composite_tile<2>(acc, cur != kNoRay, sample, alpha, c3, t, &my_samples);
       if (stop_early) {
-        if (lane == ray_lane) write_ray(vb, s, cur, cr, cg, cb, cz);
+        if (lane - ray_lane < 4) write_channel(vb, s, cur, lane - ray_lane, acc.v);
         term[row] = cur + 1u;  // tells the encoder to move on
         cur = kNoRay;
       }
