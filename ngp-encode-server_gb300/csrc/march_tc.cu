@@ -344,17 +344,7 @@ __device__ __forceinline__ bool composite_tile(RayAcc& acc, bool open, bool samp
   const int lane = threadIdx.x & 31, ray_lane = lane & ~(kLanes - 1);
   const uint32_t have = __ballot_sync(0xffffffffu, sample) >> ray_lane;
   float m[4] = {c[0], c[1], c[2], t};  // own sample's channels -> own channel of the four lanes' samples
-  {
-    const bool o1 = lane & 1, o2 = lane & 2;
-    float u = __shfl_xor_sync(0xffffffffu, o1 ? m[0] : m[1], 1);
-    if (o1) m[0] = u; else m[1] = u;
-    u = __shfl_xor_sync(0xffffffffu, o1 ? m[2] : m[3], 1);
-    if (o1) m[2] = u; else m[3] = u;
-    u = __shfl_xor_sync(0xffffffffu, o2 ? m[0] : m[2], 2);
-    if (o2) m[0] = u; else m[2] = u;
-    u = __shfl_xor_sync(0xffffffffu, o2 ? m[1] : m[3], 2);
-    if (o2) m[1] = u; else m[3] = u;
-  }
+  transpose4(m, lane);
   bool stop = false;
   uint32_t count = 0;
 #pragma unroll
@@ -372,17 +362,6 @@ __device__ __forceinline__ bool composite_tile(RayAcc& acc, bool open, bool samp
   }
   *samples += count;
   return stop;
-}
-
-// Channel c of a ray's pixel, by lane c of its first four.
-__device__ __forceinline__ void write_channel(const ViewBatch& vb, const DevScratch& s, uint32_t id, int c, float v) {
-  const RayMeta m = s.ray_meta[id];
-  const DevView& V = vb.v[m.view];
-  if (c < 3) {
-    if (V.rgb) V.rgb[(size_t)m.pixel * 3 + c] = v;
-  } else if (V.depth) {
-    V.depth[m.pixel] = v;
-  }
 }
 
 // The encoder warps' loop; true when a wait ran out.

@@ -102,6 +102,32 @@ __device__ __forceinline__ bool take_step(Slot& q, int j, int ray_lane, float* t
   return has;
 }
 
+// Four lanes' four values each -> lane c of the four has value c of all four
+// (m[i]: lane i's).
+__device__ __forceinline__ void transpose4(float (&m)[4], int lane) {
+  const bool o1 = lane & 1, o2 = lane & 2;
+  float u = __shfl_xor_sync(0xffffffffu, o1 ? m[0] : m[1], 1);
+  if (o1) m[0] = u; else m[1] = u;
+  u = __shfl_xor_sync(0xffffffffu, o1 ? m[2] : m[3], 1);
+  if (o1) m[2] = u; else m[3] = u;
+  u = __shfl_xor_sync(0xffffffffu, o2 ? m[0] : m[2], 2);
+  if (o2) m[0] = u; else m[2] = u;
+  u = __shfl_xor_sync(0xffffffffu, o2 ? m[1] : m[3], 2);
+  if (o2) m[1] = u; else m[3] = u;
+}
+
+// Channel c (red, green, blue, expected depth) of a ray's pixel, by lane c of
+// the ray's first four.
+__device__ __forceinline__ void write_channel(const ViewBatch& vb, const DevScratch& s, uint32_t id, int c, float v) {
+  const RayMeta m = s.ray_meta[id];
+  const DevView& V = vb.v[m.view];
+  if (c < 3) {
+    if (V.rgb) V.rgb[(size_t)m.pixel * 3 + c] = v;
+  } else if (V.depth) {
+    V.depth[m.pixel] = v;
+  }
+}
+
 // A ray's pixel.
 __device__ __forceinline__ void write_ray(const ViewBatch& vb, const DevScratch& s, uint32_t id, float cr, float cg,
                                           float cb, float dep) {

@@ -138,6 +138,11 @@ __device__ __forceinline__ bool occupied(const uint32_t* __restrict__ occ, const
   return (__ldg(occ + (i >> 5)) >> (i & 31)) & 1u;
 }
 
+// level_res for a level that is known at run time only.
+static __constant__ int level_res_table[kLevels] = {
+    level_res(0), level_res(1), level_res(2),  level_res(3),  level_res(4),  level_res(5),  level_res(6),  level_res(7),
+    level_res(8), level_res(9), level_res(10), level_res(11), level_res(12), level_res(13), level_res(14), level_res(15)};
+
 // Per-level cell and trilinear fractions: i0 = clamp(floor(x*N), 0, N-1).
 struct LevelCell {
   uint32_t ix, iy, iz;
@@ -213,6 +218,34 @@ __device__ __forceinline__ void encode_level_fp32(const float2* __restrict__ tab
   f0 = a0;
   f1 = a1;
 }
+
+// The same in two halves, for work between a level's table reads and their
+// use: begin() reads, finish() interpolates.
+struct LevelGather {
+  float2 e[8];
+  LevelCell c;
+  __device__ __forceinline__ void begin(const float2* __restrict__ table, uint32_t T, uint32_t dense_mask,
+                                        const float3& x, int l, bool has) {
+    const int N = level_res_table[l];
+    c = level_cell(x, N);
+    uint32_t idx[8];
+    corner_indices(c, N, (dense_mask >> l) & 1u, T, idx);
+    const float2* tab = table + (size_t)l * T;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) e[k] = has ? __ldg(tab + idx[k]) : make_float2(0.0f, 0.0f);
+  }
+  __device__ __forceinline__ float2 finish() const {
+    float w[8];
+    corner_weights(c, w);
+    float a0 = 0.0f, a1 = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      a0 = fmaf(w[k], e[k].x, a0);
+      a1 = fmaf(w[k], e[k].y, a1);
+    }
+    return make_float2(a0, a1);
+  }
+};
 
 // All levels of the FP32 table at x.
 __device__ __forceinline__ void encode_fp32(const float2* __restrict__ table, uint32_t T,

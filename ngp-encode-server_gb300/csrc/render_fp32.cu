@@ -18,10 +18,11 @@ namespace nes {
 namespace {
 
 constexpr int kRaygenThreads = 256;
-// Twelve warps of the march per SM: 150 KB of shared memory (weights and the
-// warps' tiles) leave L1 to the gathers, and 159 registers a thread hold the
-// tile product's operands ahead.  1080p: 8 warps 156 ms, 10 151, 12 145, 14
-// (126 registers) 145, 16 168 (before packed FMAs, against 150 with 12).
+// Twelve warps of the march per SM: 182 KB of shared memory (weights, the
+// warps' encodings and activations) and 168 registers a thread.  1080p: 8 warps
+// 132 ms, 10 131, 11 129, 12 128; it is bound by the products' operand reads
+// (a lane's 8 x 8 tile takes 64 bytes per 64 multiply-adds, 16 cycles of the
+// SM's 128 bytes a cycle against 16 of its FMA lanes).
 constexpr int kMarchWarps = 12;
 constexpr int kMarchThreads = 32 * kMarchWarps;
 
@@ -30,12 +31,14 @@ constexpr int kMarchThreads = 32 * kMarchWarps;
 // steps behind an opaque surface or leave lanes without an occupied step.  ms,
 // one ray per thread (as it was) -> 8 and 32 steps:
 //               rays   seeded scene          opaque, sparse scene
-//   64x48       1.6k   20   -> 2.2,  0.64    10.0 -> 0.61, 0.41
-//   256x256     34k    24   -> 3.6,  2.9     13.1 -> 0.86, 0.97
-//   400x300     61k    26.7 -> 7.2,  6.7     13.7 -> 1.5,  1.9
-//   640x360     118k   37.7 -> 16.5, 16.4    18.2 -> 2.9,  4.3
-//   853x481     210k   54.6 -> 28.5, 28.9    24.2 -> 4.9,  7.4
-//   1920x1080   1.06M  232  -> 138,  145     (1, 2, 4, 16 steps: 163, 144, 139, 141)
+//   64x48       1.6k   20   -> 2.2,  0.59    10.0 -> 0.61, 0.38
+//   256x256     34k    24   -> 3.6,  2.6     13.1 -> 0.86, 1.07
+//   400x300     61k    26.7 -> 6.0,  6.7     13.7 -> 1.5,  1.9
+//   640x360     118k   37.7 -> 15.3, 16.4    18.2 -> 3.0,  4.3
+//   853x481     210k   54.6 -> 26.3, 28.9    24.2 -> 5.1,  7.4
+//   1920x1080   1.06M  232  -> 128,  145     (1, 2, 4, 16 steps: 163, 144, 139, 141)
+// (the column not taken, before the next tile's encoding ran under the
+// products.)
 __device__ __forceinline__ int march32_shift(uint32_t nrays, uint32_t rows) { return nrays <= rows / 3 * 2 ? 5 : 3; }
 
 // Grid-stride over the batch's ray-generation threads (the loop bound is
@@ -99,30 +102,52 @@ raygen_kernel(const __grid_constant__ Src src, float4* __restrict__ ray_dt, RayM
 // time: (32 >> kShift) rays with their next 1 << kShift occupied steps each.
 // The warp encodes its lanes' samples into its shared-memory tile, evaluates
 // the MLPs as matrix products over it (tile32.cuh) and composites each ray's
-// samples in step order, every lane of the ray alike, by shuffle.
+// samples in step order, by shuffle.
+// While a tile is in the MLPs the next one is encoded, a level per eight
+// inputs of the products, so the gathers run under the multiply-adds (1080p 138
+// -> 128 ms, 256x256 2.9 -> 2.6 ms; before, the products alone took 94 ms, the
+// encoding alone 41).
 struct MarchSmem32 {
   TileWeights32 w;
-  float tile[kMarchWarps][kTileFloats];
+  float enc[kMarchWarps][kEnc * 32];
+  float act[kMarchWarps][kTileFloats];
+};
+
+// The encoding of the warp's next samples into its rows of E, level by level.
+struct EncodeNext {
+  const DevScene& sc;
+  float* E;
+  int lane;
+  float3 x;
+  bool has;
+  LevelGather g;
+  __device__ __forceinline__ void begin(int l) { g.begin(sc.table32, sc.T, sc.dense_mask, x, l, has); }
+  __device__ __forceinline__ void finish(int l) {
+    const float2 f = g.finish();
+    const int at = (2 * l) * 32 + (lane ^ tile_swap(2 * l));  // rows 2 l and 2 l + 1 swap alike
+    E[at] = has ? f.x : 0.0f;
+    E[at + 32] = has ? f.y : 0.0f;
+  }
 };
 
 template <int kShift>
 __device__ __forceinline__ unsigned long long march_fp32_loop(const ViewBatch& vb, const DevScene& sc,
                                                               const DevScratch& s, uint32_t nrays,
-                                                              const TileWeights32& W, float* X) {
+                                                              const TileWeights32& W, float* E, float* X) {
   constexpr int kLanes = 1 << kShift;
   const int lane = threadIdx.x & 31, j = lane & (kLanes - 1), ray_lane = lane - j;
   Slot q;
-  bool exhausted = false, open = false;  // open: the slot's ray is being composited
-  float T = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f, dep = 0.0f;
-  unsigned long long my_samples = 0;
-  for (;;) {
+  EncodeNext next{sc, E, lane, make_float3(0.0f, 0.0f, 0.0f), false, {}};
+  float t_next = 0.0f;
+  bool exhausted = false, first = false;
+  // Rays and steps of the next tile; false when the warp is out of rays.
+  auto take = [&]() -> bool {
+    first = false;
     for (;;) {
       next_window<kShift>(sc, q, j);
-      if (open && !q.live) {
-        if (j == 0) write_ray(vb, s, q.id, cr, cg, cb, dep);
-        open = false;
-      }
+      if (first && !q.live && j == 0) write_ray(vb, s, q.id, 0.0f, 0.0f, 0.0f, 0.0f);  // no occupied sample
       if (exhausted || __ballot_sync(0xffffffffu, q.live) != 0u) break;
+      first = false;
       const uint32_t base = warp_claim(s.counters + kCtrCursor, 32u >> kShift);
       if (base >= nrays) {
         exhausted = true;
@@ -131,48 +156,66 @@ __device__ __forceinline__ unsigned long long march_fp32_loop(const ViewBatch& v
       const uint32_t id = base + ((uint32_t)lane >> kShift);
       if (id < nrays) {
         q.start(vb, s, id);
-        open = true;
-        T = 1.0f;
-        cr = cg = cb = dep = 0.0f;
+        first = true;
       }
     }
-    if (__ballot_sync(0xffffffffu, q.live) == 0u) return my_samples;  // out of rays
-    float t;
-    const bool has = take_step<kShift>(q, j, ray_lane, &t);
-    const float3 x = sample_pos(q.o, q.d, t);
-#pragma unroll
+    next.has = take_step<kShift>(q, j, ray_lane, &t_next);
+    next.x = sample_pos(q.o, q.d, t_next);
+    return __ballot_sync(0xffffffffu, q.live) != 0u;
+  };
+
+  constexpr uint32_t kNone = 0xFFFFFFFFu;
+  uint32_t cur = kNone;  // ray being composited in this lane (none, or it has terminated)
+  // Its transmittance, and by lane c of each four its channel c (red, green,
+  // blue, expected depth).
+  float T = 1.0f, acc = 0.0f;
+  unsigned long long my_samples = 0;
+  bool more = take();
+  if (more)
+#pragma unroll 1
     for (int l = 0; l < kLevels; ++l) {
-      float f0 = 0.0f, f1 = 0.0f;
-      if (has) encode_level_fp32(sc.table32, sc.T, sc.dense_mask, x, l, f0, f1);
-      X[(2 * l) * 32 + (lane ^ tile_swap(2 * l))] = f0;
-      X[(2 * l + 1) * 32 + (lane ^ tile_swap(2 * l + 1))] = f1;
+      next.begin(l);
+      next.finish(l);
     }
+  while (more) {
     __syncwarp();
+    // The tile that is encoded becomes the current one.
+    const float t = t_next;
+    const float3 d = q.d;
+    const uint32_t have = __ballot_sync(0xffffffffu, next.has);
+    if (first) {
+      cur = q.id;
+      T = 1.0f;
+      acc = 0.0f;
+    }
+    more = take();
     float3 c;
-    const float sigma = tile_mlp32(W, X, lane, q.d, &c);
+    const float sigma = tile_mlp32(W, E, X, lane, d, &c, next);
     const float alpha_own = -expm1f(-sigma * kDt);
-    const uint32_t have = __ballot_sync(0xffffffffu, has);
+    float m[4] = {c.x, c.y, c.z, t};  // own sample's channels -> own channel of the four lanes' samples
+    transpose4(m, lane);
     bool stop = false;
-#pragma unroll 4
+#pragma unroll
     for (int i = 0; i < kLanes; ++i) {
       const float alpha = __shfl_sync(0xffffffffu, alpha_own, ray_lane + i);
-      const float ci0 = __shfl_sync(0xffffffffu, c.x, ray_lane + i);
-      const float ci1 = __shfl_sync(0xffffffffu, c.y, ray_lane + i);
-      const float ci2 = __shfl_sync(0xffffffffu, c.z, ray_lane + i);
-      const float ti = __shfl_sync(0xffffffffu, t, ray_lane + i);
-      if (q.live && !stop && ((have >> (ray_lane + i)) & 1u)) {
+      const float vi = __shfl_sync(0xffffffffu, m[i & 3], ray_lane + (i & ~3) + (lane & 3));
+      if (cur != kNone && !stop && ((have >> (ray_lane + i)) & 1u)) {
         ++my_samples;
         const float w = T * alpha;
-        cr = fmaf(w, ci0, cr);
-        cg = fmaf(w, ci1, cg);
-        cb = fmaf(w, ci2, cb);
-        dep = fmaf(w, ti, dep);
+        acc = fmaf(w, vi, acc);
         T -= w;
         stop = T < kTStop;
       }
     }
-    if (stop) q.live = false;  // written at the top of the loop
+    // A ray is complete when it has terminated (the steps of it that are
+    // already encoded are dropped) or its lanes turn to another or to none.
+    if (cur != kNone && (stop || first || !q.live)) {
+      if (stop && !first && q.live) q.live = next.has = false;
+      if (j < 4) write_channel(vb, s, cur, j, acc);
+      cur = kNone;
+    }
   }
+  return my_samples;
 }
 
 template <class Src>
@@ -185,11 +228,12 @@ march_fp32_kernel(const __grid_constant__ Src src, const DevScene sc, const DevS
   __syncthreads();
   const uint32_t nrays = min(s.counters[kCtrRays], s.max_rays);
   const uint32_t rows = gridDim.x * kMarchThreads;
-  float* X = S.tile[threadIdx.x >> 5];
+  float* E = S.enc[threadIdx.x >> 5];
+  float* X = S.act[threadIdx.x >> 5];
   unsigned long long my_samples;
   const int shift = march32_shift(nrays, rows);
-  if (shift == 5) my_samples = march_fp32_loop<5>(vb, sc, s, nrays, S.w, X);
-  else my_samples = march_fp32_loop<3>(vb, sc, s, nrays, S.w, X);
+  if (shift == 5) my_samples = march_fp32_loop<5>(vb, sc, s, nrays, S.w, E, X);
+  else my_samples = march_fp32_loop<3>(vb, sc, s, nrays, S.w, E, X);
   // One 64-bit atomic per warp for the sample count, which each of a ray's
   // lanes has.
 #pragma unroll

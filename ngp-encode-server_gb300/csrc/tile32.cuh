@@ -55,7 +55,9 @@ __device__ __forceinline__ float4 relu4(unsigned long long a, unsigned long long
   return make_float4(fmaxf(v.x, 0.0f), fmaxf(v.y, 0.0f), fmaxf(v.z, 0.0f), fmaxf(v.w, 0.0f));
 }
 
-// X[0..64) = relu(W^T X[0..K)) for the warp's samples, W [K][64].  A lane
+// X[0..64) = relu(W^T in[0..K)) for the warp's samples, W [K][64] (in may be
+// X).  Around each eight inputs' products, bg.begin(i) and bg.finish(i), i =
+// kBg + (input / 8): other work whose memory reads they hide.  A lane
 // has samples 4 sg + {0..3, 16..19} and outputs 4 og + {0..3, 32..35}, the
 // samples two by two in packed FMAs.  A 16-byte shared-memory read costs two
 // passes instead of four when lanes i and i ^ 1 (or i ^ 2) want the same
@@ -63,8 +65,8 @@ __device__ __forceinline__ float4 relu4(unsigned long long a, unsigned long long
 // do.  Seeded 1080p view: 232 ms one sample per thread; 155 ms as a product
 // with sg in bits 0-1 (four passes for the activations), 150 ms so, 145 ms
 // with packed FMAs (12 warps, 32 steps per ray).
-template <int K>
-__device__ __forceinline__ void tile_layer64(const float* __restrict__ W, float* X, int lane) {
+template <int K, int kBg, class Bg>
+__device__ __forceinline__ void tile_layer64(const float* __restrict__ W, const float* in, float* X, int lane, Bg& bg) {
   const int sg = 4 * ((lane >> 1) & 3), og = 4 * ((lane & 1) | ((lane >> 2) & 6));
   unsigned long long acc[8][4];  // [output][pair of samples]
 #pragma unroll
@@ -73,9 +75,10 @@ __device__ __forceinline__ void tile_layer64(const float* __restrict__ W, float*
     for (int s = 0; s < 4; ++s) acc[o][s] = 0ull;
 #pragma unroll 1
   for (int k0 = 0; k0 < K; k0 += 8) {
+    bg.begin(kBg + k0 / 8);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const float* xr = X + (k0 + k) * 32;
+      const float* xr = in + (k0 + k) * 32;
       const float* wr = W + (k0 + k) * kHid + og;
       const ulonglong2 x0 = *reinterpret_cast<const ulonglong2*>(xr + (sg ^ tile_swap(k)));
       const ulonglong2 x1 = *reinterpret_cast<const ulonglong2*>(xr + ((sg + 16) ^ tile_swap(k)));
@@ -90,6 +93,8 @@ __device__ __forceinline__ void tile_layer64(const float* __restrict__ W, float*
         for (int s = 0; s < 4; ++s) fma2(acc[o][s], ww, x[s]);
       }
     }
+    __syncwarp();  // in[k0 .. k0 + 8) has been read: finish may write there
+    bg.finish(kBg + k0 / 8);
   }
   __syncwarp();
   const int swap = tile_swap(og);
@@ -102,10 +107,14 @@ __device__ __forceinline__ void tile_layer64(const float* __restrict__ W, float*
   __syncwarp();
 }
 
-// The 32 encoded features of the warp's samples are in X[0..32): both MLPs.
-// Every lane gets its own sample's density and colour; d is its direction.
-__device__ __forceinline__ float tile_mlp32(const TileWeights32& W, float* X, int lane, const float3& d, float3* rgb) {
-  tile_layer64<kEnc>(W.dw1, X, lane);
+// Both MLPs of the warp's samples, whose 32 encoded features are in E; X is
+// scratch.  Every lane gets its own sample's density and colour; d is its
+// direction.  bg.begin(i) and bg.finish(i) are called for i = 0..15 on the
+// way; after finish(i), rows 2 i and 2 i + 1 of E are free.
+template <class Bg>
+__device__ __forceinline__ float tile_mlp32(const TileWeights32& W, const float* E, float* X, int lane,
+                                            const float3& d, float3* rgb, Bg& bg) {
+  tile_layer64<kEnc, 0>(W.dw1, E, X, lane, bg);
   {  // density 64 -> 16: samples 4 sg + {0..3}, outputs 4 og + {0..3}
     const int sg = 4 * ((lane >> 1) & 7), og = 4 * ((lane & 1) | ((lane >> 3) & 2));
     float acc[4][4];
@@ -145,8 +154,8 @@ __device__ __forceinline__ float tile_mlp32(const TileWeights32& W, float* X, in
   const float logit = *row31;
   *row31 = 0.0f;
   __syncwarp();
-  tile_layer64<kCIn>(W.cw1, X, lane);
-  tile_layer64<kHid>(W.cw2, X, lane);
+  tile_layer64<kCIn, 4>(W.cw1, X, X, lane, bg);
+  tile_layer64<kHid, 8>(W.cw2, X, X, lane, bg);
   float r = 0.0f, g = 0.0f, b = 0.0f;
 #pragma unroll 8
   for (int k = 0; k < kHid; ++k) {

@@ -908,10 +908,6 @@ constexpr uint32_t kBtColsPerGroup = 128;  // A: 64 columns, D: 64 columns
 // with shuffles and add them with one atomic per run.  Corners k and k + 1 are
 // one aligned entry pair {i, i ^ 1} half the time (a dense level's even index;
 // a hashed level's even x, the x prime being 1): one 16-byte atomic then.
-__constant__ int level_res_table[kLevels] = {level_res(0),  level_res(1),  level_res(2),  level_res(3),
-                                            level_res(4),  level_res(5),  level_res(6),  level_res(7),
-                                            level_res(8),  level_res(9),  level_res(10), level_res(11),
-                                            level_res(12), level_res(13), level_res(14), level_res(15)};
 constexpr int kAggLevels = 13;  // levels whose scatter-add is warp-aggregated (N <= 776)
 static_assert(level_res(kAggLevels - 1) < 1024, "cell key packs 10 bits per coordinate");
 
