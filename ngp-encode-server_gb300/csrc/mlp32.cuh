@@ -1,6 +1,6 @@
-// mlp32.cuh -- FP32 density and colour MLPs evaluated per thread with the
-// weights broadcast from shared memory (the occupancy build and the training
-// kernels; the march's form is tile32.cuh).
+// mlp32.cuh -- the FP32 density MLP evaluated per thread with the weights
+// broadcast from shared memory (the occupancy build; the form of the march
+// and the trainer is tile32.cuh).
 #pragma once
 #include "render_common.cuh"
 
@@ -60,40 +60,6 @@ __device__ __forceinline__ void density_mlp32(const SmemWeights32& W, const floa
       out[4 * k + 3] = fmaf(q.w, a, out[4 * k + 3]);
     }
   }
-}
-
-// Colour MLP [SH16 | out[1..15] | 0] 32->64->64->3, FP32.
-__device__ __forceinline__ float3 colour_mlp32(const SmemWeights32& W, const float sh[16],
-                                               const float dout[16]) {
-  float cin[32];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) cin[k] = sh[k];
-#pragma unroll
-  for (int k = 0; k < 15; ++k) cin[16 + k] = dout[1 + k];
-  cin[31] = 0.0f;
-  float g1[kHid];
-#pragma unroll
-  for (int j = 0; j < kHid; ++j) g1[j] = fmaxf(dot32(W.cw1 + j * kCIn, cin), 0.0f);
-  float r = 0.0f, g = 0.0f, b = 0.0f;
-#pragma unroll 2
-  for (int j = 0; j < kHid; ++j) {
-    const float4* w4 = reinterpret_cast<const float4*>(W.cw2 + j * kHid);
-    float a = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const float4 q = w4[k];
-      a = fmaf(q.x, g1[4 * k + 0], a);
-      a = fmaf(q.y, g1[4 * k + 1], a);
-      a = fmaf(q.z, g1[4 * k + 2], a);
-      a = fmaf(q.w, g1[4 * k + 3], a);
-    }
-    a = fmaxf(a, 0.0f);
-    const float4 c3 = *reinterpret_cast<const float4*>(W.cw3t + j * 4);
-    r = fmaf(c3.x, a, r);
-    g = fmaf(c3.y, a, g);
-    b = fmaf(c3.z, a, b);
-  }
-  return make_float3(sigmoidf(r), sigmoidf(g), sigmoidf(b));
 }
 
 }  // namespace nes

@@ -1,5 +1,5 @@
 // tile32.cuh -- the FP32 density and colour MLPs of 32 samples by one warp,
-// on the CUDA cores (the plain FP32 march).
+// on the CUDA cores (the plain FP32 march, the trainer's strict mode).
 //
 // Evaluated one sample per thread, every weight costs a shared-memory read
 // per four multiply-adds and the L1 / shared-memory pipe, not the FMA pipe,
@@ -48,15 +48,19 @@ __device__ __forceinline__ unsigned long long twice(float w) {
   asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(w));
   return r;
 }
-__device__ __forceinline__ float4 relu4(unsigned long long a, unsigned long long b) {
+__device__ __forceinline__ float4 four(unsigned long long a, unsigned long long b) {
   float4 v;
   asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(a));
   asm("mov.b64 {%0, %1}, %2;" : "=f"(v.z), "=f"(v.w) : "l"(b));
+  return v;
+}
+__device__ __forceinline__ float4 relu4(const float4& v) {
   return make_float4(fmaxf(v.x, 0.0f), fmaxf(v.y, 0.0f), fmaxf(v.z, 0.0f), fmaxf(v.w, 0.0f));
 }
 
-// X[0..64) = relu(W^T in[0..K)) for the warp's samples, W [K][64] (in may be
-// X).  Around each eight inputs' products, bg.begin(i) and bg.finish(i), i =
+// X[0..64) = ep(W^T in[0..K)) for the warp's samples, W [K][64] (in may be X);
+// ep(i, row, sample, v) gets this lane's i-th four outputs (i < 16): output
+// `row` of samples sample .. sample + 3.  Around each eight inputs' products, bg.begin(i) and bg.finish(i), i =
 // kBg + (input / 8): other work whose memory reads they hide.  A lane
 // has samples 4 sg + {0..3, 16..19} and outputs 4 og + {0..3, 32..35}, the
 // samples two by two in packed FMAs.  A 16-byte shared-memory read costs two
@@ -65,8 +69,9 @@ __device__ __forceinline__ float4 relu4(unsigned long long a, unsigned long long
 // do.  Seeded 1080p view: 232 ms one sample per thread; 155 ms as a product
 // with sg in bits 0-1 (four passes for the activations), 150 ms so, 145 ms
 // with packed FMAs (12 warps, 32 steps per ray).
-template <int K, int kBg, class Bg>
-__device__ __forceinline__ void tile_layer64(const float* __restrict__ W, const float* in, float* X, int lane, Bg& bg) {
+template <int K, int kBg, class Bg, class Ep>
+__device__ __forceinline__ void tile_layer64(const float* __restrict__ W, const float* in, float* X, int lane, Bg& bg,
+                                             Ep&& ep) {
   const int sg = 4 * ((lane >> 1) & 3), og = 4 * ((lane & 1) | ((lane >> 2) & 6));
   unsigned long long acc[8][4];  // [output][pair of samples]
 #pragma unroll
@@ -100,52 +105,69 @@ __device__ __forceinline__ void tile_layer64(const float* __restrict__ W, const 
   const int swap = tile_swap(og);
 #pragma unroll
   for (int o = 0; o < 8; ++o) {
-    float* xr = X + (og + (o & 3) + (o >> 2) * 32) * 32;
-    *reinterpret_cast<float4*>(xr + (sg ^ swap)) = relu4(acc[o][0], acc[o][1]);
-    *reinterpret_cast<float4*>(xr + ((sg + 16) ^ swap)) = relu4(acc[o][2], acc[o][3]);
+    const int row = og + (o & 3) + (o >> 2) * 32;
+    float* xr = X + row * 32;
+    *reinterpret_cast<float4*>(xr + (sg ^ swap)) = ep(2 * o, row, sg, four(acc[o][0], acc[o][1]));
+    *reinterpret_cast<float4*>(xr + ((sg + 16) ^ swap)) = ep(2 * o + 1, row, sg + 16, four(acc[o][2], acc[o][3]));
   }
   __syncwarp();
 }
 
-// Both MLPs of the warp's samples, whose 32 encoded features are in E; X is
-// scratch.  Every lane gets its own sample's density and colour; d is its
-// direction.  bg.begin(i) and bg.finish(i) are called for i = 0..15 on the
-// way; after finish(i), rows 2 i and 2 i + 1 of E are free.
-template <class Bg>
-__device__ __forceinline__ float tile_mlp32(const TileWeights32& W, const float* E, float* X, int lane,
-                                            const float3& d, float3* rgb, Bg& bg) {
-  tile_layer64<kEnc, 0>(W.dw1, E, X, lane, bg);
-  {  // density 64 -> 16: samples 4 sg + {0..3}, outputs 4 og + {0..3}
-    const int sg = 4 * ((lane >> 1) & 7), og = 4 * ((lane & 1) | ((lane >> 3) & 2));
-    float acc[4][4];
+// W^T X[0..K) for the warp's samples, 16 outputs, W [K][kLd]: ep(row, sample,
+// v) gets output `row` of samples sample .. sample + 3 after every lane has
+// read X.
+template <int K, int kLd, class Ep>
+__device__ __forceinline__ void tile_layer16(const float* __restrict__ W, const float* X, int lane, Ep&& ep) {
+  const int sg = 4 * ((lane >> 1) & 7), og = 4 * ((lane & 1) | ((lane >> 3) & 2));
+  float acc[4][4];
 #pragma unroll
-    for (int o = 0; o < 4; ++o)
+  for (int o = 0; o < 4; ++o)
 #pragma unroll
-      for (int s = 0; s < 4; ++s) acc[o][s] = 0.0f;
+    for (int s = 0; s < 4; ++s) acc[o][s] = 0.0f;
 #pragma unroll 1
-    for (int k0 = 0; k0 < kHid; k0 += 8) {
+  for (int k0 = 0; k0 < K; k0 += 8) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float4 xv = *reinterpret_cast<const float4*>(X + (k0 + k) * 32 + (sg ^ tile_swap(k)));
-        const float4 wv = *reinterpret_cast<const float4*>(W.dw2 + (k0 + k) * kDOut + og);
-        const float x[4] = {xv.x, xv.y, xv.z, xv.w}, w[4] = {wv.x, wv.y, wv.z, wv.w};
+    for (int k = 0; k < 8; ++k) {
+      const float4 xv = *reinterpret_cast<const float4*>(X + (k0 + k) * 32 + (sg ^ tile_swap(k)));
+      const float4 wv = *reinterpret_cast<const float4*>(W + (k0 + k) * kLd + og);
+      const float x[4] = {xv.x, xv.y, xv.z, xv.w}, w[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
-        for (int o = 0; o < 4; ++o)
+      for (int o = 0; o < 4; ++o)
 #pragma unroll
-          for (int s = 0; s < 4; ++s) acc[o][s] = fmaf(w[o], x[s], acc[o][s]);
-      }
-    }
-    __syncwarp();
-    // Colour input: SH in rows 0..15, density outputs 1..15 in rows 16..30;
-    // output 0 passes through row 31, which is then the input's zero.
-#pragma unroll
-    for (int o = 0; o < 4; ++o) {
-      const int m = og + o, row = m == 0 ? 31 : 15 + m;
-      *reinterpret_cast<float4*>(X + row * 32 + (sg ^ tile_swap(row))) =
-          make_float4(acc[o][0], acc[o][1], acc[o][2], acc[o][3]);
+        for (int s = 0; s < 4; ++s) acc[o][s] = fmaf(w[o], x[s], acc[o][s]);
     }
   }
-  float sh[16];
+  __syncwarp();
+#pragma unroll
+  for (int o = 0; o < 4; ++o) ep(og + o, sg, make_float4(acc[o][0], acc[o][1], acc[o][2], acc[o][3]));
+}
+
+// The colour logits of the lane's own sample, X[0..64) = the last hidden
+// layer.
+__device__ __forceinline__ float3 tile_logits(const float* __restrict__ cw3, const float* X, int lane) {
+  float r = 0.0f, g = 0.0f, b = 0.0f;
+#pragma unroll 8
+  for (int k = 0; k < kHid; ++k) {
+    const float a = X[k * 32 + (lane ^ tile_swap(k))];
+    const float4 c3 = *reinterpret_cast<const float4*>(cw3 + k * 4);
+    r = fmaf(c3.x, a, r);
+    g = fmaf(c3.y, a, g);
+    b = fmaf(c3.z, a, b);
+  }
+  __syncwarp();  // X may be written again
+  return make_float3(r, g, b);
+}
+
+// The density MLP's second layer and the colour input: X[0..64) = the hidden
+// layer -> X[0..32) = [SH16(d) | outputs 1..15 | 0]; every lane gets its own
+// sample's output 0 and SH basis.
+__device__ __forceinline__ float tile_colour_input(const float* __restrict__ dw2, float* X, int lane, const float3& d,
+                                                   float (&sh)[16]) {
+  // Output 0 passes through row 31, which is then the input's zero.
+  tile_layer16<kHid, kDOut>(dw2, X, lane, [&](int m, int sample, const float4& v) {
+    const int row = m == 0 ? 31 : 15 + m;
+    *reinterpret_cast<float4*>(X + row * 32 + (sample ^ tile_swap(row))) = v;
+  });
   sh16(d, sh);
 #pragma unroll
   for (int k = 0; k < 16; ++k) X[k * 32 + (lane ^ tile_swap(k))] = sh[k];
@@ -154,19 +176,30 @@ __device__ __forceinline__ float tile_mlp32(const TileWeights32& W, const float*
   const float logit = *row31;
   *row31 = 0.0f;
   __syncwarp();
-  tile_layer64<kCIn, 4>(W.cw1, X, X, lane, bg);
-  tile_layer64<kHid, 8>(W.cw2, X, X, lane, bg);
-  float r = 0.0f, g = 0.0f, b = 0.0f;
-#pragma unroll 8
-  for (int k = 0; k < kHid; ++k) {
-    const float a = X[k * 32 + (lane ^ tile_swap(k))];
-    const float4 c3 = *reinterpret_cast<const float4*>(W.cw3 + k * 4);
-    r = fmaf(c3.x, a, r);
-    g = fmaf(c3.y, a, g);
-    b = fmaf(c3.z, a, b);
-  }
-  __syncwarp();  // X may be written again
-  *rgb = make_float3(sigmoidf(r), sigmoidf(g), sigmoidf(b));
+  return logit;
+}
+
+// No other work under the products.
+struct NoOtherWork {
+  __device__ __forceinline__ void begin(int) {}
+  __device__ __forceinline__ void finish(int) {}
+};
+
+// Both MLPs of the warp's samples, whose 32 encoded features are in E; X is
+// scratch.  Every lane gets its own sample's density and colour; d is its
+// direction.  bg.begin(i) and bg.finish(i) are called for i = 0..15 on the
+// way; after finish(i), rows 2 i and 2 i + 1 of E are free.
+template <class Bg>
+__device__ __forceinline__ float tile_mlp32(const TileWeights32& W, const float* E, float* X, int lane,
+                                            const float3& d, float3* rgb, Bg& bg) {
+  const auto relu = [](int, int, int, const float4& v) { return relu4(v); };
+  tile_layer64<kEnc, 0>(W.dw1, E, X, lane, bg, relu);
+  float sh[16];
+  const float logit = tile_colour_input(W.dw2, X, lane, d, sh);
+  tile_layer64<kCIn, 4>(W.cw1, X, X, lane, bg, relu);
+  tile_layer64<kHid, 8>(W.cw2, X, X, lane, bg, relu);
+  const float3 lg = tile_logits(W.cw3, X, lane);
+  *rgb = make_float3(sigmoidf(lg.x), sigmoidf(lg.y), sigmoidf(lg.z));
   return expf(logit - 1.0f);
 }
 

@@ -52,6 +52,7 @@
 #include "mlp32.cuh"
 #include "nes_gb300.h"
 #include "tc_ptx.cuh"
+#include "tile32.cuh"
 
 using namespace nes;
 
@@ -107,11 +108,9 @@ __device__ __forceinline__ float* stage_row(float* a, int F, uint32_t s) {
 }
 __host__ __device__ constexpr int soff(int f) { return (f >> 3) * 256 + (f & 7) * 4; }
 
-// FP32 forward evaluation: 128-thread blocks, three resident per SM at its 167 registers.
 // Backward: 256-thread blocks capped at 128 registers, two resident per SM
 // (16 warps) with one shared copy of the weights per block, which leaves
 // L1 for the table gathers.
-constexpr int kFwdThreads = 128;
 constexpr int kBwdThreads = 256;
 constexpr uint32_t kErrBadRay = 2u, kErrOverflow = 3u;
 
@@ -178,7 +177,7 @@ struct RayOut {  // composited result of one training ray
 //  3. encode_kernel, thread per listed sample: the hash-grid encoding, kept
 //     for the backward (a warp's samples are consecutive samples of one or two
 //     rays: coherent gathers);
-//  4. eval_kernel (FP32, thread per listed sample) or eval_tc_kernel (the
+//  4. eval_kernel (FP32, warp per 32 listed samples) or eval_tc_kernel (the
 //     MLP products on tcgen05 as 3xTF32, thread = TMEM lane per sample): the
 //     MLPs at that sample, its t, alpha and colour written to the sample's
 //     place;
@@ -188,16 +187,19 @@ struct RayOut {  // composited result of one training ray
 // With eval_kernel the per-sample arithmetic is the one-pass FP32 march's;
 // only the samples after an early termination are evaluated and then left
 // unused.
-constexpr int kRayBlock = 256;  // rays per block of the per-ray kernels
+// Rays per block of the per-ray kernels: one warp, so that a small batch still
+// reaches most SMs (4,001 rays in blocks of 256 ran on 16 of the 152: counting,
+// listing, compositing and the adjoint took 1.21 of a strict gradient's 8.4
+// ms, 0.52 in single warps; of 2^18 rays the same).
+constexpr int kRayBlock = 32;
 constexpr uint32_t kListSamples = 1u << 26;  // samples listed at a time
 static_assert((uint32_t)kRayBlock * kMaxSteps <= kListSamples, "a block of rays fits the list");
 
 __global__ void __launch_bounds__(kRayBlock)
 count_kernel(const TrainRay* __restrict__ rays, int n, const DevScene sc, RayOut* __restrict__ rout,
              uint32_t* __restrict__ block_count) {
-  __shared__ uint32_t warp_sum[kRayBlock / 32];
-  const int i = blockIdx.x * kRayBlock + threadIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  static_assert(kRayBlock == 32, "a block is one warp");
+  const int lane = threadIdx.x, i = blockIdx.x * kRayBlock + lane;
   TrainRay r{};
   if (i < n) r = rays[i];
   const float3 o = make_float3(r.ox, r.oy, r.oz), d = make_float3(r.dx, r.dy, r.dz);
@@ -210,18 +212,10 @@ count_kernel(const TrainRay* __restrict__ rays, int n, const DevScene sc, RayOut
     const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
     if (lane >= off) incl += v;
   }
-  if (lane == 31) warp_sum[warp] = incl;
-  __syncthreads();
-  uint32_t before = 0, total = 0;
-#pragma unroll
-  for (int w = 0; w < kRayBlock / 32; ++w) {
-    before += w < warp ? warp_sum[w] : 0u;
-    total += warp_sum[w];
-  }
-  if (threadIdx.x == 0) block_count[blockIdx.x] = total;
+  if (lane == 31) block_count[blockIdx.x] = incl;
   if (i < n) {
     RayOut ro{};
-    ro.first = before + incl - cnt;
+    ro.first = incl - cnt;
     ro.count = cnt;
     rout[i] = ro;
   }
@@ -229,16 +223,18 @@ count_kernel(const TrainRay* __restrict__ rays, int n, const DevScene sc, RayOut
 
 // block_first[b] = samples of the blocks before b (one block of 1,024 threads;
 // block_first[blocks] = all samples).
-constexpr int kScanThreads = 1024, kScanItems = 4;
-static_assert((1 << 20) / kRayBlock <= kScanThreads * kScanItems, "one scan block covers the largest batch");
+constexpr int kScanThreads = 1024, kScanItems = 33;
+static_assert(((1 << 20) / kRayBlock + kScanThreads) / kScanThreads <= kScanItems, "one scan block covers the largest batch");
 __global__ void __launch_bounds__(kScanThreads)
 scan_kernel(const uint32_t* __restrict__ block_count, int blocks, uint32_t* __restrict__ block_first) {
   __shared__ uint32_t warp_sum[kScanThreads / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i0 = threadIdx.x * kScanItems;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (blocks + kScanThreads) / kScanThreads;  // covers entry `blocks` too
+  const int i0 = threadIdx.x * per;
   uint32_t v[kScanItems], sum = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    v[k] = i0 + k < blocks ? block_count[i0 + k] : 0u;
+    v[k] = k < per && i0 + k < blocks ? block_count[i0 + k] : 0u;
     sum += v[k];
   }
   uint32_t incl = sum;
@@ -253,7 +249,7 @@ scan_kernel(const uint32_t* __restrict__ block_count, int blocks, uint32_t* __re
   for (int w = 0; w < warp; ++w) first += warp_sum[w];
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    if (i0 + k <= blocks) block_first[i0 + k] = first;
+    if (k < per && i0 + k <= blocks) block_first[i0 + k] = first;
     first += v[k];
   }
 }
@@ -305,6 +301,21 @@ encode_kernel(const uint2* __restrict__ list, uint32_t m, const TrainRay* __rest
   }
 }
 
+// A warp's samples' features -> the rows of its shared-memory tile.
+__device__ __forceinline__ void load_enc_tile(const float* __restrict__ enc, uint32_t sample, bool valid, float* E,
+                                              int lane) {
+#pragma unroll
+  for (int c = 0; c < kEnc / 4; ++c) {
+    const float4 v = valid ? enc_chunk(enc, sample, c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float* row = E + 4 * c * 32 + (lane ^ tile_swap(4 * c));  // the chunk's four rows swap alike
+    row[0] = v.x;
+    row[32] = v.y;
+    row[64] = v.z;
+    row[96] = v.w;
+  }
+  __syncwarp();
+}
+
 // All 32 features of a listed sample.
 __device__ __forceinline__ void load_enc(const float* __restrict__ enc, uint32_t sample, float (&f)[kEnc]) {
 #pragma unroll
@@ -317,29 +328,43 @@ __device__ __forceinline__ void load_enc(const float* __restrict__ enc, uint32_t
   }
 }
 
-// Persistent grid-stride over the list.
-__global__ void __launch_bounds__(kFwdThreads)
+// The FP32 MLPs of the listed samples, a warp 32 at a time as matrix products
+// (tile32.cuh), over the list in strides of the grid (1.88 M samples: 0.61 ms;
+// one sample per thread with the weights broadcast, 1.01).
+constexpr int kEvalWarps = 12;
+struct EvalSmem {
+  TileWeights32 w;
+  float enc[kEvalWarps][kEnc * 32];
+  float act[kEvalWarps][kTileFloats];
+};
+
+__global__ void __launch_bounds__(32 * kEvalWarps, 1)
 eval_kernel(const uint2* __restrict__ list, uint32_t m, const TrainRay* __restrict__ rays, const DevScene sc,
             const float* __restrict__ encs, ScratchSample* __restrict__ scratch) {
   extern __shared__ float4 smem_raw[];
-  SmemWeights32& W = *reinterpret_cast<SmemWeights32*>(smem_raw);
-  load_weights32(W, sc.weights);
+  EvalSmem& S = *reinterpret_cast<EvalSmem*>(smem_raw);
+  load_tile_weights32(S.w, sc.weights);
   __syncthreads();
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < m; j += gridDim.x * blockDim.x) {
-    const uint2 e = list[j];
-    const TrainRay& r = rays[e.x];
-    const float3 d = make_float3(r.dx, r.dy, r.dz);
-    const float t = fmaf((float)e.y + 0.5f, kDt, r.ts);
-    float enc[kEnc];
-    load_enc(encs, j, enc);
-    float dout[kDOut];
-    density_mlp32(W, enc, dout);
-    const float sigma = expf(dout[0] - 1.0f);
-    float sh[16];
-    sh16(d, sh);
-    const float3 c = colour_mlp32(W, sh, dout);
-    const float alpha = -expm1f(-sigma * kDt);
-    scratch[j] = ScratchSample{t, alpha, 0.0f, c.x, c.y, c.z, 0.0f, 0.0f};
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* const E = S.enc[warp];
+  NoOtherWork none;
+  const uint32_t tiles = (m + 31u) / 32u;
+  for (uint32_t tile = blockIdx.x * kEvalWarps + warp; tile < tiles; tile += gridDim.x * kEvalWarps) {
+    const uint32_t j = tile * 32u + (uint32_t)lane;
+    const bool valid = j < m;
+    float t = 0.0f;
+    float3 d = make_float3(0.0f, 0.0f, 1.0f);
+    if (valid) {
+      const uint2 e = list[j];
+      const TrainRay& r = rays[e.x];
+      d = make_float3(r.dx, r.dy, r.dz);
+      t = fmaf((float)e.y + 0.5f, kDt, r.ts);
+    }
+    load_enc_tile(encs, j, valid, E, lane);
+    float3 c;
+    const float sigma = tile_mlp32(S.w, E, S.act[warp], lane, d, &c, none);
+    if (valid) scratch[j] = ScratchSample{t, -expm1f(-sigma * kDt), 0.0f, c.x, c.y, c.z, 0.0f, 0.0f};
+    __syncwarp();  // E is written again
   }
 }
 
@@ -1728,7 +1753,6 @@ struct nes_trainer {
   uint8_t* d_bimg = nullptr;  // TF32 weight images of backward_tc_kernel
   uint8_t* d_eimg = nullptr;  // high/low TF32 forward images of eval_tc_kernel
   uint32_t chunk = 0;
-  int fwd_blocks = 0;  // persistent eval_kernel grid: SMs x resident blocks
   uint64_t steps = 0;
   uint64_t last_samples = 0;
   // Phase events on the trainer's stream: 0 start of a part's forward, 1 its
@@ -1746,7 +1770,6 @@ namespace {
     if (e_ != cudaSuccess) return NES_EIO; \
   } while (0)
 
-constexpr int kSmemW = (int)sizeof(SmemWeights32);
 constexpr int kSmemB = (int)sizeof(SmemBackward);
 
 Staging staging(const nes_trainer* t) {
@@ -1860,7 +1883,7 @@ int loss_and_grad(nes_trainer* t, int n, double* loss) {
                                                                                   t->d_enc);
       TR_CUDA(cudaGetLastError());
       if (t->cfg.exact_weight_grads)
-        eval_kernel<<<t->fwd_blocks, kFwdThreads, kSmemW, t->st>>>(t->d_list, m, rays, c->scene, t->d_enc,
+        eval_kernel<<<c->num_sms, 32 * kEvalWarps, (int)sizeof(EvalSmem), t->st>>>(t->d_list, m, rays, c->scene, t->d_enc,
                                                                   t->d_scratch);
       else
         eval_tc_kernel<<<c->num_sms, kEtThreads, kEtSmem, t->st>>>(t->d_list, m, rays, t->d_enc, t->d_eimg,
@@ -2033,7 +2056,7 @@ int nes_trainer_create(nes_ctx* ctx, const nes_train_config* cfg, nes_trainer** 
       cudaMemset(t->d_vw, 0, kWeightFloats * sizeof(float)) != cudaSuccess ||
       cudaMemset(t->d_ctr, 0, 4 * sizeof(uint32_t)) != cudaSuccess)
     return fail(NES_EIO);
-  if (cudaFuncSetAttribute(eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemW) != cudaSuccess ||
+  if (cudaFuncSetAttribute(eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EvalSmem)) != cudaSuccess ||
       cudaFuncSetAttribute(backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemB) != cudaSuccess ||
       cudaFuncSetAttribute(dw_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DwTcSmem)) !=
           cudaSuccess ||
@@ -2050,10 +2073,6 @@ int nes_trainer_create(nes_ctx* ctx, const nes_train_config* cfg, nes_trainer** 
     if (cudaFuncGetAttributes(&fa, eval_tc_kernel) != cudaSuccess || fa.numRegs * kEtThreads * 2 <= 65536)
       return fail(NES_EIO);
   }
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, eval_kernel, kFwdThreads, kSmemW) != cudaSuccess)
-    return fail(NES_EIO);
-  t->fwd_blocks = ctx->num_sms * (per_sm < 1 ? 1 : per_sm);
   *out = t;
   return NES_OK;
 }
