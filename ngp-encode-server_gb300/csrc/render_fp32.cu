@@ -9,7 +9,6 @@
 #include <cuda_fp16.h>
 
 #include "kernels.h"
-#include "mlp32.cuh"
 #include "ray_slot.cuh"
 #include "tile32.cuh"
 
@@ -242,13 +241,61 @@ march_fp32_kernel(const __grid_constant__ Src src, const DevScene sc, const DevS
     atomicAdd(reinterpret_cast<unsigned long long*>(s.counters + kCtrSamples), my_samples >> shift);
 }
 
+// The density MLP per thread, its weights in shared memory laid out for
+// broadcast float4 reads (the occupancy build).
+struct DensityWeights32 {
+  float dw1[kHid * kEnc];    // [j][k]
+  float dw2t[kHid * kDOut];  // [j][m] (transposed)
+};
+
+__device__ inline void load_density_weights32(DensityWeights32& W, const float* __restrict__ g) {
+  for (int i = threadIdx.x; i < kHid * kEnc; i += blockDim.x) W.dw1[i] = g[kOffDW1 + i];
+  for (int i = threadIdx.x; i < kHid * kDOut; i += blockDim.x) {
+    const int j = i / kDOut, m = i % kDOut;
+    W.dw2t[i] = g[kOffDW2 + m * kHid + j];
+  }
+}
+
+__device__ __forceinline__ float dot32(const float* __restrict__ w, const float in[32]) {
+  const float4* w4 = reinterpret_cast<const float4*>(w);
+  float a = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float4 q = w4[k];
+    a = fmaf(q.x, in[4 * k + 0], a);
+    a = fmaf(q.y, in[4 * k + 1], a);
+    a = fmaf(q.z, in[4 * k + 2], a);
+    a = fmaf(q.w, in[4 * k + 3], a);
+  }
+  return a;
+}
+
+// Density MLP 32->64->16 (ReLU hidden), FP32.
+__device__ __forceinline__ void density_mlp32(const DensityWeights32& W, const float enc[32], float out[16]) {
+#pragma unroll
+  for (int m = 0; m < kDOut; ++m) out[m] = 0.0f;
+#pragma unroll 4
+  for (int j = 0; j < kHid; ++j) {
+    const float a = fmaxf(dot32(W.dw1 + j * kEnc, enc), 0.0f);
+    const float4* w2 = reinterpret_cast<const float4*>(W.dw2t + j * kDOut);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float4 q = w2[k];
+      out[4 * k + 0] = fmaf(q.x, a, out[4 * k + 0]);
+      out[4 * k + 1] = fmaf(q.y, a, out[4 * k + 1]);
+      out[4 * k + 2] = fmaf(q.z, a, out[4 * k + 2]);
+      out[4 * k + 3] = fmaf(q.w, a, out[4 * k + 3]);
+    }
+  }
+}
+
 constexpr int kOccThreads = 128;
 
 __global__ void __launch_bounds__(kOccThreads)
 occupancy_kernel(const DevScene sc, float threshold, uint32_t* __restrict__ occ) {
   extern __shared__ float4 smem_raw[];
-  SmemWeights32& W = *reinterpret_cast<SmemWeights32*>(smem_raw);
-  load_weights32(W, sc.weights);
+  DensityWeights32& W = *reinterpret_cast<DensityWeights32*>(smem_raw);
+  load_density_weights32(W, sc.weights);
   __syncthreads();
   const uint32_t cell = blockIdx.x * blockDim.x + threadIdx.x;  // grid covers 128^3 exactly
   const uint32_t cx = cell % kOccRes, cy = (cell / kOccRes) % kOccRes, cz = cell / (kOccRes * kOccRes);
@@ -318,7 +365,7 @@ cudaError_t launch_march_fp32(const ViewBatch* views_dev, const DevScene& scene,
 }
 
 cudaError_t launch_occupancy(const DevScene& scene, float threshold, uint32_t* occ_out, cudaStream_t stream) {
-  const int smem = (int)sizeof(SmemWeights32);
+  const int smem = (int)sizeof(DensityWeights32);
   cudaError_t e = cudaFuncSetAttribute(occupancy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const unsigned cells = kOccRes * kOccRes * kOccRes;

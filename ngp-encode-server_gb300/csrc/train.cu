@@ -24,14 +24,14 @@
 //     backward sweep keeps every term proportional to T_{k+1}; the equivalent
 //     forward form with suffix sums (C - prefix) cancels in FP32 late in
 //     the ray;
-//  3. backward (thread per record, in chunks): recompute both MLPs from the
+//  3. backward (in chunks of the records): recompute both MLPs from the
 //     kept encoding, backpropagate, and stage every layer's input activations
 //     and output deltas.  By default the ten layer products of the recompute
 //     and the backpropagation run on the tensor cores (backward_tc_kernel,
-//     tcgen05 kind::tf32), the staging is BF16 and scatter_kernel adds the
-//     encoding gradients into the FP32 gradient table; exact_weight_grads = 1
-//     keeps the products in FP32 on the CUDA cores with FP32 staging and
-//     scatter-adds in the same kernel (backward_kernel);
+//     tcgen05 kind::tf32) and the staging is BF16; exact_weight_grads = 1
+//     keeps the products and the staging in FP32, on the CUDA cores
+//     (backward_kernel); scatter_kernel adds the encoding gradients into the
+//     FP32 gradient table;
 //  4. weight gradients: per layer dW[out][in] += sum_s delta[s][out] act[s][in]
 //     over the chunk (by default dw_tc_kernel, tcgen05 kind::f16 with BF16
 //     operands; exact: dw_kernel, register-tiled split-K reduction);
@@ -49,7 +49,6 @@
 
 #include "ctx_internal.h"
 #include "kernels.h"
-#include "mlp32.cuh"
 #include "nes_gb300.h"
 #include "tc_ptx.cuh"
 #include "tile32.cuh"
@@ -83,17 +82,9 @@ struct SampleRec {  // compacted sample with its compositing adjoint
   float dsigma, dcr, dcg, dcb;
 };
 
-// Per-sample staging of the weight-gradient reductions, in 32-sample
-// tiles (FP32 layout of the strict mode; the tensor-core mode stages BF16,
-// see stage8).  Each tile of an F-wide array (F a multiple of 8) is one
-// contiguous block of F x 32 floats in the canonical K-major layout of the
-// tensor core's shared-memory operands, no swizzle, K = sample: 8-feature x
-// 4-sample core matrices of 128 bytes, the 8 core matrices of a feature
-// group along K at 128-byte steps, feature groups at 1,024-byte steps.
-// Feature f of sample k of a tile sits at float
-//   (f / 8) * 256 + (k / 4) * 32 + (f % 8) * 4 + k % 4,
-// so one bulk copy per array and tile lands a ready MMA operand, and a
-// thread's features sit at immediate offsets from one base.
+// Per-sample staging of the weight-gradient reductions, in 32-sample tiles.
+// Strict mode: FP32, each tile of an F-wide array F rows (features) of 32
+// samples.  The tensor-core mode stages BF16 operands, see stage8.
 constexpr int kStageFloats = kEnc + kHid + kCIn + kHid + kHid  // activations: enc, h1, cin, g1, g2
                              + kHid + kDOut + kHid + kHid + 8;  // deltas: dh1, dout, dg1, dg2, dlogit(3)+zeros
 struct Staging {
@@ -102,16 +93,8 @@ struct Staging {
 };
 constexpr int kFDlog = 8;
 
-__device__ __forceinline__ float* stage_row(float* a, int F, uint32_t s) {
-  const uint32_t k = s & 31u;
-  return a + (size_t)(s >> 5) * F * 32 + (k >> 2) * 32 + (k & 3);
-}
-__host__ __device__ constexpr int soff(int f) { return (f >> 3) * 256 + (f & 7) * 4; }
+__device__ __forceinline__ float* stage_tile(float* a, int F, uint32_t tile) { return a + (size_t)tile * F * 32; }
 
-// Backward: 256-thread blocks capped at 128 registers, two resident per SM
-// (16 warps) with one shared copy of the weights per block, which leaves
-// L1 for the table gathers.
-constexpr int kBwdThreads = 256;
 constexpr uint32_t kErrBadRay = 2u, kErrOverflow = 3u;
 
 __device__ __forceinline__ uint64_t mix64(uint64_t z) {
@@ -477,273 +460,268 @@ adjoint_kernel(const TrainRay* __restrict__ rays, const RayOut* __restrict__ rou
   if (lane == 0 && my_loss != 0.0f) atomicAdd(loss_sum, (double)my_loss);
 }
 
-// Backward, thread per record of the chunk [first, first + count).
-// Activations stay in registers (ReLU masks as 64-bit words); every staged
-// value is written once, feature f of the sample at row[soff(f)].
-__device__ __forceinline__ float dot64(const float* __restrict__ w, const float in[64]) {
-  const float4* w4 = reinterpret_cast<const float4*>(w);
-  float a = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 16; ++k) {
-    const float4 q = w4[k];
-    a = fmaf(q.x, in[4 * k + 0], a);
-    a = fmaf(q.y, in[4 * k + 1], a);
-    a = fmaf(q.z, in[4 * k + 2], a);
-    a = fmaf(q.w, in[4 * k + 3], a);
-  }
-  return a;
-}
-
-// Shared memory of the backward: the FP32 weights plus colour W1's
-// geometry-feature columns (16..30) transposed, for the dout pass.
-struct SmemBackward {
-  SmemWeights32 w;
-  float cw1g[16 * kHid];  // [m][j] = cw1[j][16 + m], m < 15; row 15 zero
+// Strict backward of the chunk [first, first + count), a warp 32 records at a
+// time: both MLPs recomputed and backpropagated as matrix products over the
+// warp's shared-memory tile (tile32.cuh), FP32 throughout, activations and
+// deltas staged from the lanes' registers.  ReLU masks are 64 bits of a lane's
+// own outputs: a layer's output and its delta lie in the same lanes.  Records
+// past the chunk's end have zero adjoints, hence zero deltas.  One sample per
+// thread with the weights broadcast from shared memory (L1 / shared-memory
+// pipe 87 % busy) took 3.94 ms per 1.88 M records, scatter-add included; this
+// 1.46 and scatter_kernel 0.43.
+constexpr int kBwdWarps = 12;
+struct BackwardSmem {
+  TileWeights32 w;                 // [input][output]
+  float dw1[kHid * kEnc];          // and as the products back want them: [output][input]
+  float dw2[kDOut * kHid];
+  float cw1[kHid * kCIn];
+  float cw2[kHid * kHid];
+  float act[kBwdWarps][kTileFloats];
+  float dlog[kBwdWarps][3 * 32];
 };
 
-__global__ void __launch_bounds__(kBwdThreads, 2)
+// v where the lane's i-th four mask bits are set, else 0.
+__device__ __forceinline__ float4 masked4(const float4& v, uint64_t mask, int i) {
+  const uint32_t m = (uint32_t)(mask >> (4 * i));
+  return make_float4((m & 1u) ? v.x : 0.0f, (m & 2u) ? v.y : 0.0f, (m & 4u) ? v.z : 0.0f, (m & 8u) ? v.w : 0.0f);
+}
+__device__ __forceinline__ uint64_t positive4(const float4& v, int i) {
+  return (uint64_t)((v.x > 0.0f ? 1u : 0u) | (v.y > 0.0f ? 2u : 0u) | (v.z > 0.0f ? 4u : 0u) | (v.w > 0.0f ? 8u : 0u))
+         << (4 * i);
+}
+
+__global__ void __launch_bounds__(32 * kBwdWarps, 1)
 backward_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t count, const uint2* __restrict__ list,
                 const TrainRay* __restrict__ rays, const float* __restrict__ encs, const DevScene sc, Staging st,
-                float2* __restrict__ gtable) {
+                float* __restrict__ denc) {
   extern __shared__ float4 smem_raw[];
-  SmemBackward& S = *reinterpret_cast<SmemBackward*>(smem_raw);
-  SmemWeights32& W = S.w;
-  load_weights32(W, sc.weights);
-  for (int i = threadIdx.x; i < 16 * kHid; i += blockDim.x) {
-    const int m = i / kHid, j = i % kHid;
-    S.cw1g[i] = m < 15 ? sc.weights[kOffCW1 + j * kCIn + 16 + m] : 0.0f;
-  }
+  BackwardSmem& S = *reinterpret_cast<BackwardSmem*>(smem_raw);
+  load_tile_weights32(S.w, sc.weights);
+  for (int i = threadIdx.x; i < kHid * kEnc; i += blockDim.x) S.dw1[i] = sc.weights[kOffDW1 + i];
+  for (int i = threadIdx.x; i < kDOut * kHid; i += blockDim.x) S.dw2[i] = sc.weights[kOffDW2 + i];
+  for (int i = threadIdx.x; i < kHid * kCIn; i += blockDim.x) S.cw1[i] = sc.weights[kOffCW1 + i];
+  for (int i = threadIdx.x; i < kHid * kHid; i += blockDim.x) S.cw2[i] = sc.weights[kOffCW2 + i];
   __syncthreads();
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ((count + 31u) & ~31u)) return;
-  if (s >= count) {  // rows of the last tile past the chunk's samples: zeros for the reductions
-    float* const arr[10] = {st.enc, st.h1, st.cin, st.g1, st.g2, st.dh1, st.dout, st.dg1, st.dg2, st.dlog};
-    const int F[10] = {kEnc, kHid, kCIn, kHid, kHid, kHid, kDOut, kHid, kHid, 8};
-    for (int a = 0; a < 10; ++a) {
-      float* r = stage_row(arr[a], F[a], s);
-      for (int f = 0; f < F[a]; ++f) r[soff(f)] = 0.0f;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* const X = S.act[warp];
+  float* const D = S.dlog[warp];
+  NoOtherWork none;
+  const uint32_t tiles = (count + 31u) / 32u;
+  for (uint32_t tile = blockIdx.x * kBwdWarps + warp; tile < tiles; tile += gridDim.x * kBwdWarps) {
+    const uint32_t s = tile * 32u + (uint32_t)lane;
+    const bool valid = s < count;
+    SampleRec q{};
+    float3 dir = make_float3(0.0f, 0.0f, 1.0f);
+    if (valid) {
+      q = recs[first + s];
+      const TrainRay& r = rays[list[q.place].x];
+      dir = make_float3(r.dx, r.dy, r.dz);
     }
-    return;
-  }
-  const SampleRec q = recs[first + s];
-  const float3 x = make_float3(q.x, q.y, q.z);
-  float* const r_enc = stage_row(st.enc, kEnc, s);
-  float* const r_h1 = stage_row(st.h1, kHid, s);
-  float* const r_cin = stage_row(st.cin, kCIn, s);
-  float* const r_g1 = stage_row(st.g1, kHid, s);
-  float* const r_g2 = stage_row(st.g2, kHid, s);
-  float* const r_dh1 = stage_row(st.dh1, kHid, s);
-  float* const r_dout = stage_row(st.dout, kDOut, s);
-  float* const r_dg1 = stage_row(st.dg1, kHid, s);
-  float* const r_dg2 = stage_row(st.dg2, kHid, s);
-  float* const r_dlog = stage_row(st.dlog, 8, s);
-  // ---- forward recompute ----
-  float enc[kEnc];
-  load_enc(encs, q.place, enc);
+    // Stages and passes on a lane's four outputs of row `row`.
+    auto put = [&](float* tile_rows, int row, int sample, const float4& v) {
+      *reinterpret_cast<float4*>(tile_rows + row * 32 + sample) = v;
+      return v;
+    };
+    // ---- forward recompute ----
+    load_enc_tile(encs, q.place, valid, X, lane);
+    {
+      float* const rows = stage_tile(st.enc, kEnc, tile);
 #pragma unroll
-  for (int k = 0; k < kEnc; ++k) r_enc[soff(k)] = enc[k];
-  float out[kDOut];
-#pragma unroll
-  for (int m = 0; m < kDOut; ++m) out[m] = 0.0f;
-  uint64_t m_h1 = 0;
-#pragma unroll 1
-  for (int j = 0; j < kHid; ++j) {
-    const float a = fmaxf(dot32(W.dw1 + j * kEnc, enc), 0.0f);
-    r_h1[soff(j)] = a;
-    m_h1 |= (uint64_t)(a > 0.0f) << j;
-    const float4* w2 = reinterpret_cast<const float4*>(W.dw2t + j * kDOut);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float4 w = w2[k];
-      out[4 * k + 0] = fmaf(w.x, a, out[4 * k + 0]);
-      out[4 * k + 1] = fmaf(w.y, a, out[4 * k + 1]);
-      out[4 * k + 2] = fmaf(w.z, a, out[4 * k + 2]);
-      out[4 * k + 3] = fmaf(w.w, a, out[4 * k + 3]);
+      for (int k = 0; k < kEnc; ++k) rows[k * 32 + lane] = X[k * 32 + (lane ^ tile_swap(k))];
     }
-  }
-  const float sigma = expf(out[0] - 1.0f);
-  float cin[kCIn];
-  {
-    const TrainRay& r = rays[list[q.place].x];
-    sh16(make_float3(r.dx, r.dy, r.dz), cin);
-  }
+    uint64_t m_h1 = 0, m_g1 = 0, m_g2 = 0;
+    float* rows = stage_tile(st.h1, kHid, tile);
+    tile_layer64<kEnc, 0>(S.w.dw1, X, X, lane, none, [&](int i, int row, int sample, const float4& v) {
+      m_h1 |= positive4(v, i);
+      return put(rows, row, sample, relu4(v));
+    });
+    float sh[16];
+    const float sigma = expf(tile_colour_input(S.w.dw2, X, lane, dir, sh) - 1.0f);
+    rows = stage_tile(st.cin, kCIn, tile);
 #pragma unroll
-  for (int k = 0; k < 15; ++k) cin[16 + k] = out[1 + k];
-  cin[31] = 0.0f;
+    for (int k = 0; k < kCIn; ++k) rows[k * 32 + lane] = k < 16 ? sh[k] : X[k * 32 + (lane ^ tile_swap(k))];
+    rows = stage_tile(st.g1, kHid, tile);
+    tile_layer64<kCIn, 0>(S.w.cw1, X, X, lane, none, [&](int i, int row, int sample, const float4& v) {
+      m_g1 |= positive4(v, i);
+      return put(rows, row, sample, relu4(v));
+    });
+    rows = stage_tile(st.g2, kHid, tile);
+    tile_layer64<kHid, 0>(S.w.cw2, X, X, lane, none, [&](int i, int row, int sample, const float4& v) {
+      m_g2 |= positive4(v, i);
+      return put(rows, row, sample, relu4(v));
+    });
+    const float3 lg = tile_logits(S.w.cw3, X, lane);
+    // ---- backward ----
+    {
+      const float c0 = sigmoidf(lg.x), c1 = sigmoidf(lg.y), c2 = sigmoidf(lg.z);
+      const float dl[3] = {q.dcr * c0 * (1.0f - c0), q.dcg * c1 * (1.0f - c1), q.dcb * c2 * (1.0f - c2)};
+      rows = stage_tile(st.dlog, kFDlog, tile);
 #pragma unroll
-  for (int k = 0; k < kCIn; ++k) r_cin[soff(k)] = cin[k];
-  float g[kHid];  // g1, then its gradient
+      for (int c = 0; c < kFDlog; ++c) rows[c * 32 + lane] = c < 3 ? dl[c] : 0.0f;
 #pragma unroll
-  for (int j = 0; j < kHid; ++j) {
-    g[j] = fmaxf(dot32(W.cw1 + j * kCIn, cin), 0.0f);
-    r_g1[soff(j)] = g[j];
-  }
-  uint64_t m_g1 = 0;
-#pragma unroll
-  for (int j = 0; j < kHid; ++j) m_g1 |= (uint64_t)(g[j] > 0.0f) << j;
-  float lg0 = 0.0f, lg1 = 0.0f, lg2 = 0.0f;
-  uint64_t m_g2 = 0;
-#pragma unroll 1
-  for (int j = 0; j < kHid; ++j) {
-    const float a = fmaxf(dot64(W.cw2 + j * kHid, g), 0.0f);
-    r_g2[soff(j)] = a;
-    m_g2 |= (uint64_t)(a > 0.0f) << j;
-    const float4 c3 = *reinterpret_cast<const float4*>(W.cw3t + j * 4);
-    lg0 = fmaf(c3.x, a, lg0);
-    lg1 = fmaf(c3.y, a, lg1);
-    lg2 = fmaf(c3.z, a, lg2);
-  }
-  // ---- backward ----
-  const float c0 = sigmoidf(lg0), c1 = sigmoidf(lg1), c2 = sigmoidf(lg2);
-  const float dl0 = q.dcr * c0 * (1.0f - c0), dl1 = q.dcg * c1 * (1.0f - c1), dl2 = q.dcb * c2 * (1.0f - c2);
-  r_dlog[soff(0)] = dl0;
-  r_dlog[soff(1)] = dl1;
-  r_dlog[soff(2)] = dl2;
-#pragma unroll
-  for (int f = 3; f < 8; ++f) r_dlog[soff(f)] = 0.0f;
-#pragma unroll
-  for (int k = 0; k < kHid; ++k) g[k] = 0.0f;
-#pragma unroll 1
-  for (int j = 0; j < kHid; ++j) {  // dg2_j, and dg1 += cw2[j][:] dg2_j
-    const float4 c3 = *reinterpret_cast<const float4*>(W.cw3t + j * 4);
-    const float d2 = ((m_g2 >> j) & 1) ? fmaf(c3.x, dl0, fmaf(c3.y, dl1, c3.z * dl2)) : 0.0f;
-    r_dg2[soff(j)] = d2;
-    const float4* w4 = reinterpret_cast<const float4*>(W.cw2 + j * kHid);
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const float4 w = w4[k];
-      g[4 * k + 0] = fmaf(w.x, d2, g[4 * k + 0]);
-      g[4 * k + 1] = fmaf(w.y, d2, g[4 * k + 1]);
-      g[4 * k + 2] = fmaf(w.z, d2, g[4 * k + 2]);
-      g[4 * k + 3] = fmaf(w.w, d2, g[4 * k + 3]);
+      for (int c = 0; c < 3; ++c) D[c * 32 + lane] = dl[c];
     }
-  }
+    __syncwarp();
+    rows = stage_tile(st.dg2, kHid, tile);
+    {  // dg2 = (cW3^T dlogit) of the lane's outputs and samples, as tile_layer64 gives them
+      const int sg = 4 * ((lane >> 1) & 3), og = 4 * ((lane & 1) | ((lane >> 2) & 6));
 #pragma unroll
-  for (int k = 0; k < kHid; ++k) {
-    g[k] = ((m_g1 >> k) & 1) ? g[k] : 0.0f;
-    r_dg1[soff(k)] = g[k];
-  }
-  float dout[kDOut];
-  dout[0] = q.dsigma * sigma;
+      for (int h = 0; h < 2; ++h) {
+        float4 d[3];
 #pragma unroll
-  for (int m = 0; m < 15; ++m) dout[1 + m] = dot64(S.cw1g + m * kHid, g);
+        for (int c = 0; c < 3; ++c) d[c] = *reinterpret_cast<const float4*>(D + c * 32 + sg + 16 * h);
 #pragma unroll
-  for (int m = 0; m < kDOut; ++m) r_dout[soff(m)] = dout[m];
-  float denc[kEnc];
-#pragma unroll
-  for (int k = 0; k < kEnc; ++k) denc[k] = 0.0f;
-#pragma unroll 1
-  for (int j = 0; j < kHid; ++j) {  // dh1_j, and denc += dw1[j][:] dh1_j
-    const float4* w2 = reinterpret_cast<const float4*>(W.dw2t + j * kDOut);
-    float a = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float4 w = w2[k];
-      a = fmaf(w.x, dout[4 * k + 0], a);
-      a = fmaf(w.y, dout[4 * k + 1], a);
-      a = fmaf(w.z, dout[4 * k + 2], a);
-      a = fmaf(w.w, dout[4 * k + 3], a);
+        for (int o = 0; o < 8; ++o) {
+          const int row = og + (o & 3) + (o >> 2) * 32;
+          const float4 w = *reinterpret_cast<const float4*>(S.w.cw3 + row * 4);
+          float4 v;
+          v.x = fmaf(w.x, d[0].x, fmaf(w.y, d[1].x, w.z * d[2].x));
+          v.y = fmaf(w.x, d[0].y, fmaf(w.y, d[1].y, w.z * d[2].y));
+          v.z = fmaf(w.x, d[0].z, fmaf(w.y, d[1].z, w.z * d[2].z));
+          v.w = fmaf(w.x, d[0].w, fmaf(w.y, d[1].w, w.z * d[2].w));
+          *reinterpret_cast<float4*>(X + row * 32 + ((sg + 16 * h) ^ tile_swap(row))) =
+              put(rows, row, sg + 16 * h, masked4(v, m_g2, 2 * o + h));
+        }
+      }
     }
-    const float dh = ((m_h1 >> j) & 1) ? a : 0.0f;
-    r_dh1[soff(j)] = dh;
-    const float4* w1 = reinterpret_cast<const float4*>(W.dw1 + j * kEnc);
+    __syncwarp();
+    rows = stage_tile(st.dg1, kHid, tile);
+    tile_layer64<kHid, 0>(S.cw2, X, X, lane, none, [&](int i, int row, int sample, const float4& v) {
+      return put(rows, row, sample, masked4(v, m_g1, i));
+    });
+    rows = stage_tile(st.dout, kDOut, tile);
+    tile_layer16<kHid, kCIn>(S.cw1 + 16, X, lane, [&](int m, int sample, const float4& v) {
+      if (m == 15) return;  // the input's padding column
+      *reinterpret_cast<float4*>(X + (1 + m) * 32 + (sample ^ tile_swap(1 + m))) = put(rows, 1 + m, sample, v);
+    });
+    X[lane] = rows[lane] = q.dsigma * sigma;  // row 0
+    __syncwarp();
+    rows = stage_tile(st.dh1, kHid, tile);
+    tile_layer64<kDOut, 0>(S.dw2, X, X, lane, none, [&](int i, int row, int sample, const float4& v) {
+      return put(rows, row, sample, masked4(v, m_h1, i));
+    });
+    {  // the encoding's gradient: samples 4 sg + {0..3, 16..19}, features 4 og + {0..3}, a chunk of denc
+      const int sg = 4 * ((lane >> 1) & 3), og = (lane & 1) | ((lane >> 2) & 6);
+      float acc[4][8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float4 w = w1[k];
-      denc[4 * k + 0] = fmaf(w.x, dh, denc[4 * k + 0]);
-      denc[4 * k + 1] = fmaf(w.y, dh, denc[4 * k + 1]);
-      denc[4 * k + 2] = fmaf(w.z, dh, denc[4 * k + 2]);
-      denc[4 * k + 3] = fmaf(w.w, dh, denc[4 * k + 3]);
-    }
-  }
-  // ---- hash-grid scatter-add: dtable[level][corner] += w_corner * denc[level] ----
+      for (int o = 0; o < 4; ++o)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[o][k] = 0.0f;
 #pragma unroll 1
-  for (int l = 0; l < kLevels; ++l) {
-    const int N = level_res(l);
-    const LevelCell c = level_cell(x, N);
-    uint32_t idx[8];
-    corner_indices(c, N, (sc.dense_mask >> l) & 1u, sc.T, idx);
-    float w[8];
-    corner_weights(c, w);
-    float2* gt = gtable + (size_t)l * sc.T;
-    float d0 = 0.0f, d1 = 0.0f;
+      for (int k0 = 0; k0 < kHid; k0 += 8) {
 #pragma unroll
-    for (int k = 0; k < kLevels; ++k)
-      if (k == l) {
-        d0 = denc[2 * k];
-        d1 = denc[2 * k + 1];
+        for (int k = 0; k < 8; ++k) {
+          const float* xr = X + (k0 + k) * 32;
+          const float4 x0 = *reinterpret_cast<const float4*>(xr + (sg ^ tile_swap(k)));
+          const float4 x1 = *reinterpret_cast<const float4*>(xr + ((sg + 16) ^ tile_swap(k)));
+          const float4 w0 = *reinterpret_cast<const float4*>(S.dw1 + (k0 + k) * kEnc + 4 * og);
+          const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+          const float w[4] = {w0.x, w0.y, w0.z, w0.w};
+#pragma unroll
+          for (int o = 0; o < 4; ++o)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[o][i] = fmaf(w[o], x[i], acc[o][i]);
+        }
       }
 #pragma unroll
-    for (int k = 0; k < 8; ++k) atomicAdd(gt + idx[k], make_float2(w[k] * d0, w[k] * d1));
+      for (int i = 0; i < 8; ++i)
+        *enc_chunk(denc, tile * 32u + (uint32_t)(sg + (i & 3) + (i >> 2) * 16), og) =
+            make_float4(acc[0][i], acc[1][i], acc[2][i], acc[3][i]);
+    }
+    __syncwarp();  // X is written again
   }
 }
 
-// dW[o][i] += sum_s delta[s][o] * act[s][i] over S samples of tiled staging
-// (IN activation features, LDD-wide delta tiles of which OUT are real).  Every thread owns a 4x4 tile of dW; when the
-// tiles number fewer than the block's threads, the thread groups split
-// each 32-sample smem tile between them.  Each block reduces a contiguous
-// range of samples and adds its partial dW with one atomic per element.
+// dW[o][i] += sum_s delta[s][o] * act[s][i] over `tiles` staged tiles of 32
+// samples (IN activation features, LDD-wide delta tiles of which OUT are
+// real).  A thread owns P x Q of dW, four samples at a time; when these are
+// fewer than the block's threads, thread groups split the samples of a
+// 64-sample smem tile.  Each block reduces a contiguous range of samples,
+// the next tile's reads in flight during the current one's products, and adds
+// its partial dW with one atomic per element and group.  All five per 1.88 M
+// samples: 1.01 ms (3.5 GB read), 2.03 with 4 x 4 per thread, one sample at a
+// time and a transposing copy.
 constexpr int kDwThreads = 256;
-constexpr int kDwTile = 32;
+constexpr int kDwSamples = 64;
 
-template <int IN, int OUT, int LDD>
+template <int IN, int OUT, int LDD, int P, int Q>
 __global__ void __launch_bounds__(kDwThreads)
-dw_kernel(const float* __restrict__ act, const float* __restrict__ delta, uint32_t S, float* __restrict__ dw) {
-  static_assert(IN % 4 == 0 && LDD % 4 == 0 && OUT <= LDD, "tile shape");
-  constexpr int TI = IN / 4, TO = LDD / 4, TILES = TI * TO;
-  static_assert(TILES <= kDwThreads && kDwThreads % TILES == 0, "tile count");
-  constexpr int G = kDwThreads / TILES;  // sample groups
-  // Rows padded by 4 floats: the transposing stores (sample-fastest) hit 8
-  // banks instead of 1, the float4 reads stay aligned.
-  __shared__ __align__(16) float sa[kDwTile][IN + 4];
-  __shared__ __align__(16) float sd[kDwTile][LDD + 4];
+dw_kernel(const float* __restrict__ act, const float* __restrict__ delta, uint32_t tiles, float* __restrict__ dw) {
+  constexpr int TI = IN / P, TO = LDD / Q, THREADS = TI * TO;
+  static_assert(TI == 8 && IN % P == 0 && LDD % Q == 0 && TO % 2 == 0 && OUT <= LDD && kDwThreads % THREADS == 0,
+                "thread tiles");
+  constexpr int G = kDwThreads / THREADS;  // sample groups
+  static_assert(G <= kDwSamples / 4, "at least four samples per group");
+  // Rows of 64 samples padded by 4 floats: eight neighbouring rows' 16-byte
+  // reads fall into different banks.
+  constexpr int kRow = kDwSamples + 4;
+  __shared__ __align__(16) float sa[IN][kRow];
+  __shared__ __align__(16) float sd[LDD][kRow];
   const int tid = threadIdx.x;
-  const int ti = tid % TI, to = (tid / TI) % TO, grp = tid / TILES;
-  float acc[4][4] = {};
-  const uint32_t per = ((S + gridDim.x - 1) / gridDim.x + kDwTile - 1) / kDwTile * kDwTile;
-  const uint32_t lo = blockIdx.x * per, hi = min(S, lo + per);
-  for (uint32_t base = lo; base < hi; base += kDwTile) {
-    const uint32_t rows = min((uint32_t)kDwTile, hi - base);
-    // The tile is one contiguous block: each float4 holds 4 samples of one
-    // feature (core-matrix layout), stored transposed.
-    const float4* ta = reinterpret_cast<const float4*>(act + (size_t)(base / kDwTile) * IN * kDwTile);
-    const float4* td = reinterpret_cast<const float4*>(delta + (size_t)(base / kDwTile) * LDD * kDwTile);
-    for (int e = tid; e < kDwTile * IN / 4; e += kDwThreads) {
-      const int f = (e >> 6) * 8 + (e & 7), r = ((e >> 3) & 7) * 4;
-      const float4 v = ta[e];
-      sa[r + 0][f] = (uint32_t)(r + 0) < rows ? v.x : 0.0f;
-      sa[r + 1][f] = (uint32_t)(r + 1) < rows ? v.y : 0.0f;
-      sa[r + 2][f] = (uint32_t)(r + 2) < rows ? v.z : 0.0f;
-      sa[r + 3][f] = (uint32_t)(r + 3) < rows ? v.w : 0.0f;
+  // As in tile_layer64: lanes i and i ^ 1 share an activation row, i and i ^ 2
+  // a delta row.
+  const int ti = (tid >> 1) & 7, to = ((tid & 1) | ((tid >> 4) << 1)) % TO, grp = tid / THREADS;
+  constexpr int NA = IN * kDwSamples / 4 / kDwThreads;                                // float4 per thread
+  constexpr int ND = (LDD * kDwSamples / 4 + kDwThreads - 1) / kDwThreads;
+  const uint32_t pairs = (tiles + 1u) / 2u;  // 64-sample tiles
+  const uint32_t per = (pairs + gridDim.x - 1) / gridDim.x;
+  const uint32_t lo = blockIdx.x * per, hi = min(pairs, lo + per);
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  // float4 e of a 64-sample tile of an F-wide array: staged tile e / (8 F),
+  // feature e / 8 % F, samples 4 (e % 8) and on.
+  auto read = [&](const float* a, int F, uint32_t pair, int e) {
+    const uint32_t t = 2u * pair + (uint32_t)(e / (8 * F));
+    return t < tiles ? __ldg(reinterpret_cast<const float4*>(a + (size_t)t * F * 32) + e % (8 * F)) : zero;
+  };
+  float4 pa[NA], pd[ND];
+  auto fetch = [&](uint32_t pair) {
+#pragma unroll
+    for (int n = 0; n < NA; ++n) pa[n] = read(act, IN, pair, tid + n * kDwThreads);
+#pragma unroll
+    for (int n = 0; n < ND; ++n)
+      if (tid + n * kDwThreads < LDD * kDwSamples / 4) pd[n] = read(delta, LDD, pair, tid + n * kDwThreads);
+  };
+  float acc[P][Q];
+#pragma unroll
+  for (int p = 0; p < P; ++p)
+#pragma unroll
+    for (int c = 0; c < Q; ++c) acc[p][c] = 0.0f;
+  if (lo < hi) fetch(lo);
+  for (uint32_t pair = lo; pair < hi; ++pair) {
+#pragma unroll
+    for (int n = 0; n < NA; ++n) {
+      const int e = tid + n * kDwThreads;
+      *reinterpret_cast<float4*>(&sa[e / 8 % IN][e / (8 * IN) * 32 + (e & 7) * 4]) = pa[n];
     }
-    for (int e = tid; e < kDwTile * LDD / 4; e += kDwThreads) {
-      const int f = (e >> 6) * 8 + (e & 7), r = ((e >> 3) & 7) * 4;
-      const float4 v = f < OUT ? td[e] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      sd[r + 0][f] = (uint32_t)(r + 0) < rows ? v.x : 0.0f;
-      sd[r + 1][f] = (uint32_t)(r + 1) < rows ? v.y : 0.0f;
-      sd[r + 2][f] = (uint32_t)(r + 2) < rows ? v.z : 0.0f;
-      sd[r + 3][f] = (uint32_t)(r + 3) < rows ? v.w : 0.0f;
+#pragma unroll
+    for (int n = 0; n < ND; ++n) {
+      const int e = tid + n * kDwThreads;
+      if (e < LDD * kDwSamples / 4) *reinterpret_cast<float4*>(&sd[e / 8 % LDD][e / (8 * LDD) * 32 + (e & 7) * 4]) = pd[n];
     }
     __syncthreads();
-#pragma unroll 4
-    for (int r = grp; r < kDwTile; r += G) {
-      const float4 a = *reinterpret_cast<const float4*>(&sa[r][ti * 4]);
-      const float4 d = *reinterpret_cast<const float4*>(&sd[r][to * 4]);
-      const float av[4] = {a.x, a.y, a.z, a.w}, dv[4] = {d.x, d.y, d.z, d.w};
+    if (pair + 1 < hi) fetch(pair + 1);
+#pragma unroll 1
+    for (int r = 4 * grp; r < kDwSamples; r += 4 * G) {
+      float4 a[P];
 #pragma unroll
-      for (int p = 0; p < 4; ++p)
+      for (int p = 0; p < P; ++p) a[p] = *reinterpret_cast<const float4*>(&sa[ti + p * TI][r]);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[p][c] = fmaf(dv[p], av[c], acc[p][c]);
+      for (int c = 0; c < Q; ++c) {
+        const float4 d = *reinterpret_cast<const float4*>(&sd[to + c * TO][r]);
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+          acc[p][c] = fmaf(d.w, a[p].w, fmaf(d.z, a[p].z, fmaf(d.y, a[p].y, fmaf(d.x, a[p].x, acc[p][c]))));
+      }
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int o = to * 4 + p;
+  for (int c = 0; c < Q; ++c) {
+    const int o = to + c * TO;
     if (o < OUT)
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (acc[p][c] != 0.0f) atomicAdd(dw + o * IN + ti * 4 + c, acc[p][c]);
+      for (int p = 0; p < P; ++p)
+        if (acc[p][c] != 0.0f) atomicAdd(dw + o * IN + ti + p * TI, acc[p][c]);
   }
 }
 
@@ -1749,7 +1727,7 @@ struct nes_trainer {
   float* d_gw = nullptr;
   float *d_mt = nullptr, *d_vt = nullptr, *d_mw = nullptr, *d_vw = nullptr;
   float* d_stage = nullptr;
-  float* d_denc = nullptr;  // encoding gradients of a tensor-core backward chunk, tiled as d_enc
+  float* d_denc = nullptr;  // encoding gradients of a backward chunk, tiled as d_enc
   uint8_t* d_bimg = nullptr;  // TF32 weight images of backward_tc_kernel
   uint8_t* d_eimg = nullptr;  // high/low TF32 forward images of eval_tc_kernel
   uint32_t chunk = 0;
@@ -1770,7 +1748,6 @@ namespace {
     if (e_ != cudaSuccess) return NES_EIO; \
   } while (0)
 
-constexpr int kSmemB = (int)sizeof(SmemBackward);
 
 Staging staging(const nes_trainer* t) {
   Staging s;
@@ -1789,11 +1766,10 @@ Staging staging(const nes_trainer* t) {
   return s;
 }
 
-template <int IN, int OUT, int LDD>
-cudaError_t launch_dw(const float* act, const float* delta, uint32_t S, float* dw, int num_sms, cudaStream_t st) {
-  const uint32_t tiles = (S + kDwTile - 1) / kDwTile;
-  const uint32_t want = 8u * (uint32_t)num_sms;  // 8 resident 256-thread blocks per SM
-  dw_kernel<IN, OUT, LDD><<<tiles < want ? tiles : want, kDwThreads, 0, st>>>(act, delta, S, dw);
+template <int IN, int OUT, int LDD, int P, int Q>
+cudaError_t launch_dw(const float* act, const float* delta, uint32_t tiles, float* dw, int num_sms, cudaStream_t st) {
+  const uint32_t pairs = (tiles + 1) / 2, want = 2u * (uint32_t)num_sms;  // two resident blocks per SM
+  dw_kernel<IN, OUT, LDD, P, Q><<<pairs < want ? pairs : want, kDwThreads, 0, st>>>(act, delta, tiles, dw);
   return cudaGetLastError();
 }
 
@@ -1808,28 +1784,29 @@ int backward_records(nes_trainer* t, const TrainRay* rays, uint32_t total) {
   for (uint32_t first = 0; first < total; first += chunk) {
     const uint32_t cnt = total - first < chunk ? total - first : chunk;
     if (t->cfg.exact_weight_grads) {
-      backward_kernel<<<(cnt + kBwdThreads - 1) / kBwdThreads, kBwdThreads, kSmemB, t->st>>>(
-          t->d_recs, first, cnt, t->d_list, rays, t->d_enc, c->scene, sg, t->d_gtable);
+      const uint32_t tiles = (cnt + 31) / 32, want = (tiles + kBwdWarps - 1) / kBwdWarps;
+      backward_kernel<<<want < (uint32_t)sms ? want : (uint32_t)sms, 32 * kBwdWarps, (int)sizeof(BackwardSmem),
+                        t->st>>>(t->d_recs, first, cnt, t->d_list, rays, t->d_enc, c->scene, sg, t->d_denc);
       TR_CUDA(cudaGetLastError());
-      TR_CUDA((launch_dw<kEnc, kHid, kHid>(sg.enc, sg.dh1, cnt, gw + kOffDW1, sms, t->st)));
-      TR_CUDA((launch_dw<kHid, kDOut, kDOut>(sg.h1, sg.dout, cnt, gw + kOffDW2, sms, t->st)));
-      TR_CUDA((launch_dw<kCIn, kHid, kHid>(sg.cin, sg.dg1, cnt, gw + kOffCW1, sms, t->st)));
-      TR_CUDA((launch_dw<kHid, kHid, kHid>(sg.g1, sg.dg2, cnt, gw + kOffCW2, sms, t->st)));
-      TR_CUDA((launch_dw<kHid, 3, kFDlog>(sg.g2, sg.dlog, cnt, gw + kOffCW3, sms, t->st)));
+      TR_CUDA((launch_dw<kEnc, kHid, kHid, 4, 8>(sg.enc, sg.dh1, tiles, gw + kOffDW1, sms, t->st)));
+      TR_CUDA((launch_dw<kHid, kDOut, kDOut, 8, 4>(sg.h1, sg.dout, tiles, gw + kOffDW2, sms, t->st)));
+      TR_CUDA((launch_dw<kCIn, kHid, kHid, 4, 8>(sg.cin, sg.dg1, tiles, gw + kOffCW1, sms, t->st)));
+      TR_CUDA((launch_dw<kHid, kHid, kHid, 8, 4>(sg.g1, sg.dg2, tiles, gw + kOffCW2, sms, t->st)));
+      TR_CUDA((launch_dw<kHid, 3, kFDlog, 8, 4>(sg.g2, sg.dlog, tiles, gw + kOffCW3, sms, t->st)));
     } else {
       const uint32_t groups = (cnt + 127u) / 128u;
       const uint32_t want = (groups + kBtGroups - 1) / kBtGroups;
       backward_tc_kernel<<<want < (uint32_t)sms ? want : (uint32_t)sms, kBtThreads, kBtSmem, t->st>>>(
           t->d_recs, first, cnt, t->d_list, rays, t->d_enc, t->d_bimg, sg, t->d_denc, t->d_ctr + 1);
       TR_CUDA(cudaGetLastError());
-      scatter_kernel<<<(cnt + kScatThreads - 1) / kScatThreads, kScatThreads, 0, t->st>>>(
-          t->d_recs, first, cnt, c->scene, t->d_denc, t->d_gtable);
-      TR_CUDA(cudaGetLastError());
       const uint32_t tiles = (cnt + 31) / 32;
       const uint32_t grid = tiles < (uint32_t)sms ? tiles : (uint32_t)sms;
       dw_tc_kernel<<<grid, kDwTcThreads, sizeof(DwTcSmem), t->st>>>(sg, tiles, gw, t->d_ctr + 1);
       TR_CUDA(cudaGetLastError());
     }
+    scatter_kernel<<<(cnt + kScatThreads - 1) / kScatThreads, kScatThreads, 0, t->st>>>(
+        t->d_recs, first, cnt, c->scene, t->d_denc, t->d_gtable);
+    TR_CUDA(cudaGetLastError());
   }
   return NES_OK;
 }
@@ -2043,8 +2020,8 @@ int nes_trainer_create(nes_ctx* ctx, const nes_train_config* cfg, nes_trainer** 
       cudaMalloc(&t->d_mw, kWeightFloats * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&t->d_vw, kWeightFloats * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&t->d_stage, (size_t)t->chunk * kStageFloats * sizeof(float)) != cudaSuccess ||
-      (!cfg->exact_weight_grads &&
-       cudaMalloc(&t->d_denc, (size_t)2 * t->chunk * kEnc * sizeof(float)) != cudaSuccess) ||
+      cudaMalloc(&t->d_denc, (size_t)(cfg->exact_weight_grads ? 1 : 2) * t->chunk * kEnc * sizeof(float)) !=
+          cudaSuccess ||
       cudaMalloc(&t->d_bimg, kBtImageBytes) != cudaSuccess ||
       cudaMalloc(&t->d_eimg, kEtImageBytes) != cudaSuccess)
     return fail(NES_ENOMEM);
@@ -2057,7 +2034,7 @@ int nes_trainer_create(nes_ctx* ctx, const nes_train_config* cfg, nes_trainer** 
       cudaMemset(t->d_ctr, 0, 4 * sizeof(uint32_t)) != cudaSuccess)
     return fail(NES_EIO);
   if (cudaFuncSetAttribute(eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EvalSmem)) != cudaSuccess ||
-      cudaFuncSetAttribute(backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemB) != cudaSuccess ||
+      cudaFuncSetAttribute(backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BackwardSmem)) != cudaSuccess ||
       cudaFuncSetAttribute(dw_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DwTcSmem)) !=
           cudaSuccess ||
       cudaFuncSetAttribute(backward_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBtSmem) != cudaSuccess ||
