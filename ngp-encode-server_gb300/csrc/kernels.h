@@ -98,16 +98,22 @@ void frame_batch_index(FrameBatch* fb);
 // Batched frame glue: up to kMaxBatchFrames frames of one geometry per
 // launch, per-frame device pointers passed by value.
 constexpr int kMaxBatchFrames = 64;
-struct FrameSet {
-  const uint8_t* src[kMaxBatchFrames];
-  uint8_t* y[kMaxBatchFrames];
-  uint8_t* u[kMaxBatchFrames];
-  uint8_t* v[kMaxBatchFrames];
+template <int N>
+struct Frames {
+  static constexpr int kFrames = N;
+  const uint8_t* src[N];
+  uint8_t* y[N];
+  uint8_t* u[N];
+  uint8_t* v[N];
 };
-struct DepthSet {
-  const float* src[kMaxBatchFrames];
-  uint16_t* dst[kMaxBatchFrames];
+template <int N>
+struct Depths {
+  static constexpr int kFrames = N;
+  const float* src[N];
+  uint16_t* dst[N];
 };
+using FrameSet = Frames<kMaxBatchFrames>;
+using DepthSet = Depths<kMaxBatchFrames>;
 cudaError_t launch_yuv420p_batch(bool gray, const FrameSet& fs, int nframes, int w, int h, int src_ls,
                                  const int ls[3], cudaStream_t stream);
 cudaError_t launch_depth_pack_u16mm_batch(const DepthSet& ds, int nframes, size_t n, cudaStream_t stream);
