@@ -1295,25 +1295,27 @@ constexpr int kBtSmem = (int)kBtImageBytes + 8 * (kBtGroups + 1) + 16;
 // below 2^-21 of each product, so the loss keeps the FP32 evaluation's value
 // (plain TF32 products would move it by ~1e-3 relative: a refit whose
 // rendered colour sits within 1e-2 of the target then sees a few per cent of
-// error in its loss and adjoints).  One CTA per SM, two independent groups of
+// error in its loss and adjoints).  One CTA per SM, four independent groups of
 // 4 warps; a group takes 128 listed samples at a time (thread = sample = TMEM
-// lane), writes each layer's input as A_hi and A_lo into TMEM, one thread
-// issues the three K-chains against the weight images' high and low parts in
-// shared memory, and every thread reads its row of D back for the
-// elementwise step (ReLU, exp, SH, sigmoid) and the next layer's input.  The
-// encodings of the group's next tile are read while the MMAs of layers 1-4 of
-// the current one run (four levels per layer), into TMEM columns of their own
-// that layer 0 of the next tile reads: only two tiles' worth of warps per SM
-// fit the TMEM, so the reads' latency is hidden behind the layer chain.
-constexpr int kEtGroups = 2;
+// lane), writes each layer's input as A_hi into TMEM and as A_lo into shared
+// memory, one thread issues the three K-chains against the weight images'
+// high and low parts in shared memory, and every thread reads its row of D
+// back for the elementwise step (ReLU, exp, SH, sigmoid) and the next layer's
+// input.  The encodings of a group's next tile are read under the last
+// layer's MMAs.  A group's layers are one serial chain, so the groups in
+// flight set the rate: with A_lo and the next encoding in TMEM two fit, which
+// took 28.0 of the forward phase's 52.2 ms at 122 M samples; four bring the
+// phase to 44.1.
+constexpr int kEtGroups = 4;
 constexpr int kEtThreads = 128 * kEtGroups;
-// A_hi: 0..63, A_lo: 64..127, D: 128..191, next tile's encoding E_hi:
-// 192..223, E_lo: 224..255.
-constexpr uint32_t kEtColsPerGroup = 256;
+constexpr uint32_t kEtColsPerGroup = 128;  // A_hi: 64 columns, D: 64 columns
 constexpr uint32_t kFwdImageBytes = 40960;  // bt_image 0..4: dW1, dW2, cW1, cW2, cW3
 static_assert(bt_image(5).off == kFwdImageBytes, "forward images first");
 constexpr uint32_t kEtImageBytes = 2 * kFwdImageBytes;  // high parts, then low parts
-constexpr int kEtSmem = (int)kEtImageBytes + 8 * (kEtGroups + 1) + 16;
+constexpr uint32_t kEtLoBytes = 128 * kHid * 4;         // a group's A_lo, laid out as a weight image
+constexpr uint32_t kEtBars = kEtImageBytes + kEtGroups * kEtLoBytes;
+constexpr int kEtSmem = (int)kEtBars + 8 * (kEtGroups + 1) + 16;
+static_assert(2 * kEtSmem > 228 * 1024, "one CTA per SM: its TMEM allocation takes all columns");
 
 __device__ __forceinline__ float tf32_hi(float v) {
   uint32_t r;
@@ -1358,36 +1360,12 @@ __device__ __forceinline__ EtSample et_sample(const uint2* __restrict__ list, ui
   return q;
 }
 
-// Levels L0..L0+3 of a sample's encoding -> E_hi / E_lo columns 2 L0 ..
-// 2 L0 + 7 of this thread's lane (no wait).  Every lane of the warp calls it.
-template <int L0>
-__device__ __forceinline__ void et_encode4(const float* __restrict__ encs, uint32_t j, bool valid, uint32_t ehi_row,
-                                           uint32_t elo_row) {
-  float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
-  if (valid) {
-    a = enc_chunk(encs, j, L0 / 2);
-    b = enc_chunk(encs, j, L0 / 2 + 1);
-  }
-  const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-  uint32_t h[8], l[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const float hi = tf32_hi(f[k]);
-    h[k] = __float_as_uint(hi);
-    l[k] = __float_as_uint(f[k] - hi);
-  }
-  tc::tmem_st4(ehi_row + 2 * L0, h[0], h[1], h[2], h[3]);
-  tc::tmem_st4(ehi_row + 2 * L0 + 4, h[4], h[5], h[6], h[7]);
-  tc::tmem_st4(elo_row + 2 * L0, l[0], l[1], l[2], l[3]);
-  tc::tmem_st4(elo_row + 2 * L0 + 4, l[4], l[5], l[6], l[7]);
-}
-
 __global__ void __launch_bounds__(kEtThreads, 1)
 eval_tc_kernel(const uint2* __restrict__ list, uint32_t m, const TrainRay* __restrict__ rays,
                const float* __restrict__ encs, const uint8_t* __restrict__ images, ScratchSample* __restrict__ scratch,
                uint32_t* __restrict__ err) {
   extern __shared__ __align__(128) uint8_t smem_et[];
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_et + kEtImageBytes);  // [group] mma, [kEtGroups] images
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_et + kEtBars);  // [group] mma, [kEtGroups] images
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + kEtGroups + 1);
   const int tid = threadIdx.x, warp = tid >> 5, g = tid >> 7, row = tid & 127;
   if (tid == 0) {
@@ -1410,36 +1388,37 @@ eval_tc_kernel(const uint2* __restrict__ list, uint32_t m, const TrainRay* __res
   }
   fail = __syncthreads_or(fail);
   const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-  const uint32_t hi_col = tmem + g * kEtColsPerGroup, lo_col = hi_col + 64, d_col = hi_col + 128;
-  const uint32_t ehi_col = hi_col + 192, elo_col = hi_col + 224;
-  const uint32_t hi_row = hi_col + lane_off, lo_row = lo_col + lane_off, d_row = d_col + lane_off;
-  const uint32_t ehi_row = ehi_col + lane_off, elo_row = elo_col + lane_off;
-  const uint32_t sB = tc::smem_addr(smem_et);
+  const uint32_t hi_col = tmem + g * kEtColsPerGroup, d_col = hi_col + 64;
+  const uint32_t hi_row = hi_col + lane_off, d_row = d_col + lane_off;
+  uint8_t* const lo = smem_et + kEtImageBytes + g * kEtLoBytes;
+  const uint32_t sB = tc::smem_addr(smem_et), s_lo = tc::smem_addr(lo);
   const uint32_t gbar = 1 + g;
   uint64_t* mbar = bars + g;
   uint32_t pm = 0;
   bool ok = true;
-  // The layer input x[0..K) -> A_hi, A_lo (no wait: the next issue waits).
-  auto put = [&](const float* x, int K) {
+  // Columns 32 c .. 32 c + 31 of a K-wide layer input -> A_hi, A_lo (no wait:
+  // the next issue waits).
+  auto put32 = [&](const float (&x)[32], int c, int K) {
+    uint32_t uh[32];
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      if (c * 32 >= K) break;
-      uint32_t uh[32], ul[32];
+    for (int j = 0; j < 32; j += 4) {
+      float l[4];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float h = tf32_hi(x[32 * c + j]);
-        uh[j] = __float_as_uint(h);
-        ul[j] = __float_as_uint(x[32 * c + j] - h);
+      for (int e = 0; e < 4; ++e) {
+        const float h = tf32_hi(x[j + e]);
+        uh[j + e] = __float_as_uint(h);
+        l[e] = x[j + e] - h;
       }
-      tc::tmem_st32_nowait(hi_row + 32 * c, uh);
-      tc::tmem_st32_nowait(lo_row + 32 * c, ul);
+      *reinterpret_cast<float4*>(lo + tf32_off(row, 32 * c + j, K)) = make_float4(l[0], l[1], l[2], l[3]);
     }
+    tc::tmem_st32_nowait(hi_row + 32 * c, uh);
   };
-  // D[:, :N] = A B_i^T at 3xTF32, A from columns (a_hi, a_lo): every thread
-  // publishes its TMEM writes, one thread issues; the group learns of any
-  // failed wait here and stops as a whole.
-  auto issue = [&](int i, uint32_t a_hi, uint32_t a_lo) -> bool {
+  // D[:, :N] = A B_i^T at 3xTF32: every thread publishes its writes of A, one
+  // thread issues; the group learns of any failed wait here and stops as a
+  // whole.
+  auto issue = [&](int i) -> bool {
     tc::tmem_wait_st();
+    tc::fence_async_smem();
     tc::fence_before();
     if (tc::named_sync_or(gbar, 128, !ok)) return false;
     const BtImage b = bt_image(i);
@@ -1448,11 +1427,12 @@ eval_tc_kernel(const uint2* __restrict__ list, uint32_t m, const TrainRay* __res
       const uint32_t idesc = tc::idesc_tf32_f32(128, (int)b.N);
       const uint32_t steps = b.K / 8;
       for (uint32_t j = 0; j < steps; ++j)
-        tc::mma_tf32_at(d_col, a_hi + 8 * j, tc::sdesc(sB + b.off + 256 * j, 128, b.K * 32), idesc, j > 0 ? 1u : 0u);
+        tc::mma_tf32_at(d_col, hi_col + 8 * j, tc::sdesc(sB + b.off + 256 * j, 128, b.K * 32), idesc, j > 0 ? 1u : 0u);
       for (uint32_t j = 0; j < steps; ++j)
-        tc::mma_tf32_at(d_col, a_lo + 8 * j, tc::sdesc(sB + b.off + 256 * j, 128, b.K * 32), idesc, 1u);
+        tc::mma_tf32(d_col, tc::sdesc(s_lo + 256 * j, 128, b.K * 32), tc::sdesc(sB + b.off + 256 * j, 128, b.K * 32),
+                     idesc, 1u);
       for (uint32_t j = 0; j < steps; ++j)
-        tc::mma_tf32_at(d_col, a_hi + 8 * j, tc::sdesc(sB + kFwdImageBytes + b.off + 256 * j, 128, b.K * 32),
+        tc::mma_tf32_at(d_col, hi_col + 8 * j, tc::sdesc(sB + kFwdImageBytes + b.off + 256 * j, 128, b.K * 32),
                         idesc, 1u);
       tc::mma_commit(mbar);
     }
@@ -1463,14 +1443,23 @@ eval_tc_kernel(const uint2* __restrict__ list, uint32_t m, const TrainRay* __res
     pm ^= 1u;
     tc::fence_after();
   };
-  // ReLU of D[:, :64] -> x.
-  auto relu64 = [&](float (&x)[64]) {
+  // ReLU of D[:, :64] -> the next layer's input.
+  auto relu64 = [&]() {
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       float v[32];
       tc::tmem_ld32(d_row + 32 * c, v);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) x[32 * c + j] = fmaxf(v[j], 0.0f);
+      for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
+      put32(v, c, kHid);
+    }
+  };
+  auto load = [&](uint32_t j, bool valid, float (&enc)[kEnc]) {
+    if (valid) {
+      load_enc(encs, j, enc);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kEnc; ++k) enc[k] = 0.0f;
     }
   };
 
@@ -1478,51 +1467,44 @@ eval_tc_kernel(const uint2* __restrict__ list, uint32_t m, const TrainRay* __res
   const uint32_t stride = gridDim.x * kEtGroups;
   uint32_t tile = blockIdx.x * kEtGroups + g;
   if (!fail && tile < ntiles) {
-    // The first tile's encoding; later tiles' are read during the previous
-    // tile's layers.
     uint32_t j = tile * 128u + (uint32_t)row;
     EtSample cur = et_sample(list, j, m, rays);
-    et_encode4<0>(encs, j, cur.valid, ehi_row, elo_row);
-    et_encode4<4>(encs, j, cur.valid, ehi_row, elo_row);
-    et_encode4<8>(encs, j, cur.valid, ehi_row, elo_row);
-    et_encode4<12>(encs, j, cur.valid, ehi_row, elo_row);
+    float enc[kEnc];
+    load(j, cur.valid, enc);
     for (; tile < ntiles; tile += stride, j += stride * 128u) {
       const uint32_t jn = j + stride * 128u;
+      put32(enc, 0, kEnc);
+      if (!issue(0)) break;  // h1 = relu(enc dW1^T)
       const EtSample nxt = et_sample(list, jn, tile + stride < ntiles ? m : 0u, rays);
-      float x[64];
-      if (!issue(0, ehi_col, elo_col)) break;  // h1 = relu(enc dW1^T)
       wait();
-      relu64(x);
-      put(x, kHid);
-      if (!issue(1, hi_col, lo_col)) break;  // out = h1 dW2^T
-      et_encode4<0>(encs, jn, nxt.valid, ehi_row, elo_row);
+      relu64();
+      if (!issue(1)) break;  // out = h1 dW2^T
+      float x[32];
+      {
+        float sh[16];
+        sh16(cur.d, sh);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) x[q] = sh[q];
+      }
       wait();
       float sigma;
       {
         float out[16];
         tc::tmem_ld16(d_row, out);
         sigma = expf(out[0] - 1.0f);
-        float sh[16];
-        sh16(cur.d, sh);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) x[q] = sh[q];
 #pragma unroll
         for (int q = 0; q < 15; ++q) x[16 + q] = out[1 + q];
         x[31] = 0.0f;
       }
-      put(x, kCIn);
-      if (!issue(2, hi_col, lo_col)) break;  // g1 = relu(cin cW1^T)
-      et_encode4<4>(encs, jn, nxt.valid, ehi_row, elo_row);
+      put32(x, 0, kCIn);
+      if (!issue(2)) break;  // g1 = relu(cin cW1^T)
       wait();
-      relu64(x);
-      put(x, kHid);
-      if (!issue(3, hi_col, lo_col)) break;  // g2 = relu(g1 cW2^T)
-      et_encode4<8>(encs, jn, nxt.valid, ehi_row, elo_row);
+      relu64();
+      if (!issue(3)) break;  // g2 = relu(g1 cW2^T)
       wait();
-      relu64(x);
-      put(x, kHid);
-      if (!issue(4, hi_col, lo_col)) break;  // logit = g2 cW3^T
-      et_encode4<12>(encs, jn, nxt.valid, ehi_row, elo_row);
+      relu64();
+      if (!issue(4)) break;  // logit = g2 cW3^T
+      load(jn, nxt.valid, enc);
       wait();
       float lg[16];
       tc::tmem_ld16(d_row, lg);
@@ -2045,10 +2027,6 @@ int nes_trainer_create(nes_ctx* ctx, const nes_train_config* cfg, nes_trainer** 
     // which its register footprint (512 threads x > 64) guarantees.
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, backward_tc_kernel) != cudaSuccess || fa.numRegs <= 64) return fail(NES_EIO);
-    // eval_tc_kernel too: two of its 256-thread CTAs must not fit an SM's
-    // 65,536 registers.
-    if (cudaFuncGetAttributes(&fa, eval_tc_kernel) != cudaSuccess || fa.numRegs * kEtThreads * 2 <= 65536)
-      return fail(NES_EIO);
   }
   *out = t;
   return NES_OK;
