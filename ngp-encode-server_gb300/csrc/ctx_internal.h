@@ -31,6 +31,7 @@ struct nes_ctx {
   float* d_depth = nullptr;       // max_pixels
   uint8_t* d_rgb8 = nullptr;      // max_pixels * 3
   uint8_t* d_gray = nullptr;      // max_pixels
+  uint32_t* h_status = nullptr;   // pinned: a render's status words, then kHostFrameBytes of a small frame
   uint8_t* d_yuv = nullptr;       // yuv_capacity
   size_t yuv_capacity = 0;
   uint16_t* d_depth16 = nullptr;  // max_pixels

@@ -290,6 +290,33 @@ __global__ void rgb_to_rgb24_kernel(const float* __restrict__ rgb, size_t n, uin
   for (size_t i = done + i0; i < n; i += stride) out[i] = unit_q(rgb[i]);
 }
 
+// A RenderedFrame's payload in one launch: RGB24 and GRAY8 of a view (both
+// outputs 4-byte aligned) and the render's three status words.  The outputs
+// may be pinned host memory: a small frame then needs no copies.
+__global__ void __launch_bounds__(kGlueThreads)
+frame_bytes_kernel(const float* __restrict__ rgb, const float* __restrict__ depth, size_t px, float dmax,
+                   uint8_t* __restrict__ rgb8, uint8_t* __restrict__ gray, const uint32_t* __restrict__ status,
+                   uint32_t* __restrict__ status_out) {
+  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (i < 3) status_out[i] = status[i];
+  const size_t n3 = 3 * px, g3 = (n3 + 3) / 4;
+  const bool colour = i < g3;
+  const size_t e = 4 * (colour ? i : i - g3), n = colour ? n3 : px;
+  if (e >= n) return;
+  const float* in = (colour ? rgb : depth) + e;
+  uint8_t* out = (colour ? rgb8 : gray) + e;
+  if (e + 4 <= n) {
+    const float4 v = __ldg(reinterpret_cast<const float4*>(in));
+    const float x[4] = {v.x, v.y, v.z, v.w};
+    uint32_t word = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) word |= (uint32_t)(colour ? unit_q(x[k]) : gray_q(x[k], dmax)) << (8 * k);
+    *reinterpret_cast<uint32_t*>(out) = word;
+  } else {
+    for (size_t k = 0; e + k < n; ++k) out[k] = colour ? unit_q(in[k]) : gray_q(in[k], dmax);
+  }
+}
+
 // Fused frame output: one thread per 2x2 pixel block of a view of the
 // batch.  Each pixel's FP32 colour is quantised to RGB24 (unit_q), its luma
 // written, the block's chroma computed from the quantised 2x2 sum (edge
@@ -420,6 +447,14 @@ cudaError_t launch_depth_to_gray8(const float* d, size_t n, float dmax, uint8_t*
 
 cudaError_t launch_rgb_to_rgb24(const float* rgb, size_t n, uint8_t* out, cudaStream_t stream) {
   rgb_to_rgb24_kernel<<<grid_for(n), kGlueThreads, 0, stream>>>(rgb, n, out, aligned(rgb, 16) && aligned(out, 4));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_frame_bytes(const float* rgb, const float* depth, size_t px, float dmax, uint8_t* rgb8,
+                               uint8_t* gray, const uint32_t* status, uint32_t* status_out, cudaStream_t stream) {
+  const size_t groups = (3 * px + 3) / 4 + (px + 3) / 4;
+  const unsigned blocks = (unsigned)((groups + kGlueThreads - 1) / kGlueThreads);
+  frame_bytes_kernel<<<blocks, kGlueThreads, 0, stream>>>(rgb, depth, px, dmax, rgb8, gray, status, status_out);
   return cudaGetLastError();
 }
 

@@ -95,6 +95,11 @@ cudaError_t launch_frame_out(const FrameBatch* fb_dev, int num_sms, cudaStream_t
 // Fills fb->f[i].first_block and fb->total_blocks from the views' sizes.
 void frame_batch_index(FrameBatch* fb);
 
+// RGB24 and GRAY8 of px pixels and three status words in one launch.  rgb and
+// depth 16-byte aligned, rgb8 and gray 4-byte aligned, device or pinned host.
+cudaError_t launch_frame_bytes(const float* rgb, const float* depth, size_t px, float dmax, uint8_t* rgb8,
+                               uint8_t* gray, const uint32_t* status, uint32_t* status_out, cudaStream_t stream);
+
 // Batched frame glue: up to kMaxBatchFrames frames of one geometry per
 // launch, per-frame device pointers passed by value.
 constexpr int kMaxBatchFrames = 64;

@@ -4,6 +4,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -53,15 +54,29 @@ int render_batch_locked(nes_ctx* c, const nes_view* views, int n, float* const* 
   return NES_OK;
 }
 
-// After the stream is idle: reads the last render's sample count and the
-// device error word (set when a bounded wait inside a kernel ran out).
-int collect_status(nes_ctx* c) {
-  if (!c->samples_pending) return NES_OK;
-  uint32_t w[3] = {0, 0, 0};  // samples lo, samples hi, error
-  NES_CUDA(cudaMemcpy(w, c->scratch.counters + kCtrSamples, sizeof(w), cudaMemcpyDeviceToHost));
+// Frames of up to this many bytes are written by frame_bytes_kernel straight
+// into pinned host memory and copied to the caller's buffer by the CPU: two
+// copies to pageable memory and a third for the status cost 30 us of a 64 x 48
+// frame's 160 (surface scene) and 18 of a 480 x 270 frame's 550; at 900 KiB the
+// two ways take the same time (789 and 795 us), above it the driver's copy is
+// as good and needs no buffer.
+constexpr size_t kHostFrameBytes = 512u << 10;
+constexpr size_t kStatusBytes = 64;  // the three status words and their padding
+
+// The last render's sample count and error word (set when a bounded wait
+// inside a kernel ran out): samples lo, samples hi, error.
+int take_status(nes_ctx* c, const uint32_t* w) {
   c->last_samples = (uint64_t)w[0] | ((uint64_t)w[1] << 32);
   c->samples_pending = false;
   return w[2] ? NES_ETIMEDOUT : NES_OK;
+}
+
+// After the stream is idle: reads a pending render's status.
+int collect_status(nes_ctx* c) {
+  if (!c->samples_pending) return NES_OK;
+  uint32_t w[3] = {0, 0, 0};
+  NES_CUDA(cudaMemcpy(w, c->scratch.counters + kCtrSamples, sizeof(w), cudaMemcpyDeviceToHost));
+  return take_status(c, w);
 }
 
 // Runs fn on ctx->stream ordered after everything already queued on `user`
@@ -96,6 +111,7 @@ void free_ctx(nes_ctx* c) {
   cudaFree(c->d_depth);
   cudaFree(c->d_rgb8);
   cudaFree(c->d_gray);
+  cudaFreeHost(c->h_status);
   cudaFree(c->d_yuv);
   cudaFree(c->d_depth16);
   for (cudaEvent_t e : c->ev_t)
@@ -220,6 +236,9 @@ int nes_create(const nes_config* cfg, nes_ctx** out) {
   if ((rc = dalloc(&c->d_depth, P)) != NES_OK) return fail(rc);
   if ((rc = dalloc(&c->d_rgb8, P * 3)) != NES_OK) return fail(rc);
   if ((rc = dalloc(&c->d_gray, P)) != NES_OK) return fail(rc);
+  if (cudaHostAlloc(reinterpret_cast<void**>(&c->h_status), kStatusBytes + std::min(4 * P + 16, kHostFrameBytes),
+                    cudaHostAllocDefault) != cudaSuccess)
+    return fail(NES_ENOMEM);
   c->yuv_capacity = 2 * P + 65536;
   if ((rc = dalloc(&c->d_yuv, c->yuv_capacity)) != NES_OK) return fail(rc);
   if ((rc = dalloc(&c->d_depth16, P)) != NES_OK) return fail(rc);
@@ -265,13 +284,23 @@ int nes_render(nes_ctx* c, const uint8_t* request, size_t request_len, uint8_t* 
   float* dep[1] = {c->d_depth};
   int rc = render_batch_locked(c, &v, 1, rgb, dep);
   if (rc != NES_OK) return rc;
-  NES_CUDA(launch_rgb_to_rgb24(c->d_rgb, px * 3, c->d_rgb8, c->stream));
-  NES_CUDA(launch_depth_to_gray8(c->d_depth, px, c->cfg.depth_gray_max, c->d_gray, c->stream));
+  const size_t gray_at = (px * 3 + 15) / 16 * 16;
+  const bool small = gray_at + px <= kHostFrameBytes;
+  uint8_t* const host = reinterpret_cast<uint8_t*>(c->h_status) + kStatusBytes;
+  NES_CUDA(launch_frame_bytes(c->d_rgb, c->d_depth, px, c->cfg.depth_gray_max, small ? host : c->d_rgb8,
+                              small ? host + gray_at : c->d_gray, c->scratch.counters + kCtrSamples, c->h_status,
+                              c->stream));
   write_rendered_frame_header(req.index, &req.camera, req.is_left, px * 3, px, frame_out);
-  NES_CUDA(cudaMemcpyAsync(frame_out + L.frame_offset, c->d_rgb8, px * 3, cudaMemcpyDeviceToHost, c->stream));
-  NES_CUDA(cudaMemcpyAsync(frame_out + L.depth_offset, c->d_gray, px, cudaMemcpyDeviceToHost, c->stream));
+  if (!small) {
+    NES_CUDA(cudaMemcpyAsync(frame_out + L.frame_offset, c->d_rgb8, px * 3, cudaMemcpyDeviceToHost, c->stream));
+    NES_CUDA(cudaMemcpyAsync(frame_out + L.depth_offset, c->d_gray, px, cudaMemcpyDeviceToHost, c->stream));
+  }
   NES_CUDA(cudaStreamSynchronize(c->stream));
-  return collect_status(c);
+  if (small) {
+    std::memcpy(frame_out + L.frame_offset, host, px * 3);
+    std::memcpy(frame_out + L.depth_offset, host + gray_at, px);
+  }
+  return take_status(c, c->h_status);
 }
 
 int nes_render_views(nes_ctx* c, const nes_view* views, int nviews, float* const* rgb_dev,
@@ -340,8 +369,10 @@ int nes_render_yuv_views(nes_ctx* c, const nes_view* views, int nviews, uint8_t*
       NES_CUDA(cudaMemcpyAsync(depth_mm_host[i], F.depth_mm, px * sizeof(uint16_t), cudaMemcpyDeviceToHost,
                                c->stream));
   }
+  NES_CUDA(cudaMemcpyAsync(c->h_status, c->scratch.counters + kCtrSamples, 3 * sizeof(uint32_t),
+                           cudaMemcpyDeviceToHost, c->stream));
   NES_CUDA(cudaStreamSynchronize(c->stream));
-  return collect_status(c);
+  return take_status(c, c->h_status);
 }
 
 int nes_render_yuv(nes_ctx* c, const nes_view* view, uint8_t* y_host, uint8_t* u_host, uint8_t* v_host,
