@@ -65,18 +65,22 @@ struct TrainView {
   uint64_t offset;  // first pixel of this view in the concatenated targets
 };
 
-struct TrainRay {
+// The alignments of the three structs let them be read and written in 16-byte
+// words; member by member (4 bytes, 32-byte stride per lane) compositing and
+// the adjoint were bound by the load / store unit, 5 L1 sectors per record:
+// 106.1 ms per 122 M sample step, 112.0 without.
+struct alignas(16) TrainRay {
   float ox, oy, oz, ts;
   float dx, dy, dz;
   int n;                 // march steps (0: the ray misses the cube)
   float tr, tg, tb, td;  // target colour and depth
 };
 
-struct ScratchSample {  // state of one evaluated sample, at its place in the sample list
+struct alignas(32) ScratchSample {  // state of one evaluated sample, at its place in the sample list
   float t, alpha, T, cr, cg, cb, pad0, pad1;  // T: transmittance before the sample
 };
 
-struct SampleRec {  // compacted sample with its compositing adjoint
+struct alignas(32) SampleRec {  // compacted sample with its compositing adjoint
   float x, y, z;
   uint32_t place;  // in the sample list
   float dsigma, dcr, dcg, dcb;
