@@ -160,7 +160,7 @@ struct RayOut {  // composited result of one training ray
 //     sample set before early termination -- counted, and their places in a
 //     list of all of them, ray after ray;
 // then for as many rays at a time as kListSamples samples hold:
-//  2. list_kernel, thread per ray: (ray, step) of each sample;
+//  2. list_kernel, warp per ray: (ray, step) of each sample;
 //  3. encode_kernel, thread per listed sample: the hash-grid encoding, kept
 //     for the backward (a warp's samples are consecutive samples of one or two
 //     rays: coherent gathers);
@@ -175,24 +175,50 @@ struct RayOut {  // composited result of one training ray
 // only the samples after an early termination are evaluated and then left
 // unused.
 // Rays per block of the per-ray kernels: one warp, so that a small batch still
-// reaches most SMs (4,001 rays in blocks of 256 ran on 16 of the 152: counting,
-// listing, compositing and the adjoint took 1.21 of a strict gradient's 8.4
-// ms, 0.52 in single warps; of 2^18 rays the same).
+// reaches most SMs (4,001 rays in blocks of 256 ran on 16 of the 152: the four
+// per-ray kernels took 1.21 of a strict gradient's 8.4 ms, 0.52 in single
+// warps; of 2^18 rays the same).  Counting and listing have a warp per ray.
 constexpr int kRayBlock = 32;
 constexpr uint32_t kListSamples = 1u << 26;  // samples listed at a time
 static_assert((uint32_t)kRayBlock * kMaxSteps <= kListSamples, "a block of rays fits the list");
 
-__global__ void __launch_bounds__(kRayBlock)
+// A ray per thread left a small batch's walk serial over ~800 steps and its
+// list entries scattered (counting and listing 4,001 rays: 65 + 71 us; 17 + 19
+// so); a 122 M sample step is 1.0 ms shorter.
+//
+// Walks rays [first, first + kRayBlock) of n, a warp per ray, 32 steps at a
+// time: visit(k, step, occ) for ray number k of the block, occ the
+// occupied steps among step .. step + 31, lane by lane.
+constexpr int kWalkThreads = 512;
+template <class Visit>
+__device__ __forceinline__ void walk_rays(const TrainRay* __restrict__ rays, int first, int n, const DevScene& sc,
+                                          Visit&& visit) {
+  const int lane = threadIdx.x & 31;
+  for (int k = threadIdx.x >> 5; k < kRayBlock && first + k < n; k += kWalkThreads / 32) {
+    const TrainRay r = rays[first + k];
+    const float3 o = make_float3(r.ox, r.oy, r.oz), d = make_float3(r.dx, r.dy, r.dz);
+    for (int step = 0; step < r.n; step += 32) {
+      const int st = step + lane;
+      const bool in = st < r.n && occupied(sc.occ, sample_pos(o, d, fmaf((float)st + 0.5f, kDt, r.ts)));
+      visit(k, step, __ballot_sync(0xffffffffu, in));
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kWalkThreads)
 count_kernel(const TrainRay* __restrict__ rays, int n, const DevScene sc, RayOut* __restrict__ rout,
              uint32_t* __restrict__ block_count) {
-  static_assert(kRayBlock == 32, "a block is one warp");
-  const int lane = threadIdx.x, i = blockIdx.x * kRayBlock + lane;
-  TrainRay r{};
-  if (i < n) r = rays[i];
-  const float3 o = make_float3(r.ox, r.oy, r.oz), d = make_float3(r.dx, r.dy, r.dz);
-  uint32_t cnt = 0;
-  for (int st = 0; st < r.n; ++st)
-    if (occupied(sc.occ, sample_pos(o, d, fmaf((float)st + 0.5f, kDt, r.ts)))) ++cnt;
+  static_assert(kRayBlock == 32, "a lane per ray");
+  __shared__ uint32_t count[kRayBlock];
+  const int lane = threadIdx.x & 31, first = blockIdx.x * kRayBlock;
+  if (threadIdx.x < kRayBlock) count[threadIdx.x] = 0;
+  __syncthreads();
+  walk_rays(rays, first, n, sc, [&](int k, int, uint32_t occ) {
+    if (lane == 0) count[k] += __popc(occ);
+  });
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const uint32_t cnt = count[lane];
   uint32_t incl = cnt;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
@@ -200,11 +226,11 @@ count_kernel(const TrainRay* __restrict__ rays, int n, const DevScene sc, RayOut
     if (lane >= off) incl += v;
   }
   if (lane == 31) block_count[blockIdx.x] = incl;
-  if (i < n) {
+  if (first + lane < n) {
     RayOut ro{};
     ro.first = incl - cnt;
     ro.count = cnt;
-    rout[i] = ro;
+    rout[first + lane] = ro;
   }
 }
 
@@ -243,16 +269,17 @@ scan_kernel(const uint32_t* __restrict__ block_count, int blocks, uint32_t* __re
 
 // The samples of rays [0, n) from list place 0 (the rays' blocks start at
 // sample `base` of the batch).
-__global__ void __launch_bounds__(kRayBlock)
+__global__ void __launch_bounds__(kWalkThreads)
 list_kernel(const TrainRay* __restrict__ rays, int n, const DevScene sc, const RayOut* __restrict__ rout,
             const uint32_t* __restrict__ block_first, uint32_t base, uint2* __restrict__ list) {
-  const int i = blockIdx.x * kRayBlock + threadIdx.x;
-  if (i >= n) return;
-  const TrainRay r = rays[i];
-  const float3 o = make_float3(r.ox, r.oy, r.oz), d = make_float3(r.dx, r.dy, r.dz);
-  uint2* out = list + (block_first[blockIdx.x] - base + rout[i].first);
-  for (int st = 0; st < r.n; ++st)
-    if (occupied(sc.occ, sample_pos(o, d, fmaf((float)st + 0.5f, kDt, r.ts)))) *out++ = make_uint2((uint32_t)i, (uint32_t)st);
+  const uint32_t lane = threadIdx.x & 31;
+  const int first = blockIdx.x * kRayBlock;
+  uint2* out = nullptr;
+  walk_rays(rays, first, n, sc, [&](int k, int step, uint32_t occ) {
+    if (step == 0) out = list + (block_first[blockIdx.x] - base + rout[first + k].first);
+    if ((occ >> lane) & 1u) out[__popc(occ & ((1u << lane) - 1u))] = make_uint2((uint32_t)(first + k), step + lane);
+    out += __popc(occ);
+  });
 }
 
 // Encodings of the listed samples, FP32: 32-sample tiles of 8 chunks, a
@@ -1822,7 +1849,7 @@ int loss_and_grad(nes_trainer* t, int n, double* loss) {
   t->phase_ms[0] = t->phase_ms[1] = 0.0f;
   TR_CUDA(cudaMemsetAsync(t->d_loss, 0, sizeof(double), t->st));
   TR_CUDA(cudaEventRecord(t->ev[0], t->st));
-  count_kernel<<<blocks, kRayBlock, 0, t->st>>>(t->d_rays, n, c->scene, t->d_rout, t->d_block_count);
+  count_kernel<<<blocks, kWalkThreads, 0, t->st>>>(t->d_rays, n, c->scene, t->d_rout, t->d_block_count);
   TR_CUDA(cudaGetLastError());
   scan_kernel<<<1, kScanThreads, 0, t->st>>>(t->d_block_count, blocks, t->d_block_first);
   TR_CUDA(cudaGetLastError());
@@ -1847,7 +1874,7 @@ int loss_and_grad(nes_trainer* t, int n, double* loss) {
     if (b0 > 0) TR_CUDA(cudaEventRecord(t->ev[0], t->st));
     TR_CUDA(cudaMemsetAsync(t->d_ctr, 0, sizeof(uint32_t), t->st));  // the error word is cleared by the caller
     if (m > 0) {
-      list_kernel<<<nb, kRayBlock, 0, t->st>>>(rays, nr, c->scene, rout, block_first, base, t->d_list);
+      list_kernel<<<nb, kWalkThreads, 0, t->st>>>(rays, nr, c->scene, rout, block_first, base, t->d_list);
       TR_CUDA(cudaGetLastError());
       encode_kernel<<<(m + kEncThreads - 1) / kEncThreads, kEncThreads, 0, t->st>>>(t->d_list, m, rays, c->scene,
                                                                                   t->d_enc);
