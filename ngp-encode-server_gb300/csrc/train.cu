@@ -770,25 +770,42 @@ dw_kernel(const float* __restrict__ act, const float* __restrict__ delta, uint32
 // CTA's tiles and is added to dW once at the end.  One CTA per SM: warp 0
 // lane 0 streams tiles into a 3-stage ring with bulk copies (one per array,
 // the staging is already in the operand layout), warp 1 lane 0 issues the
-// MMAs and releases stages by tcgen05.commit, all four warps read D back.
-// The kernel is bound by reading the staging (30,208 B per tile).
+// MMAs and releases stages by tcgen05.commit, warps 0 to 3 read D back.  dg2 is
+// not staged: warps 4 to 7 make it, (dlog cW3) where g2 > 0, from the FP32 dlog
+// and the BF16 g2 of the tile, with the operands of the backward chain's own
+// product so that it is the same dg2.  The kernel is bound by reading the staging
+// (26,112 B per tile, 7 TB/s; with dg2 staged 30,208, which also cost the
+// backward, bound by writing it: 67.7 ms for both and the scatter-add at 122 M
+// records, 65.3 so).
 constexpr int kTcStages = 3;
 // Operand tiles of 32 records, BF16 (64 bytes per feature row).
 constexpr uint32_t kA1Bytes = 128 * 64, kB1Bytes = 144 * 64, kA2Bytes = 128 * 64, kB2Bytes = 80 * 64;
 constexpr uint32_t kStageBytes = kA1Bytes + kB1Bytes + kA2Bytes + kB2Bytes;
-constexpr uint32_t kTileTx = (kEnc + kCIn + kHid + kHid + kHid + kDOut + kHid + kHid + kHid + kFDlog) * 64;
+constexpr uint32_t kTileTx = (kEnc + kCIn + kHid + kHid + kHid + kDOut + kHid + kHid) * 64 + 32 * 16;
 constexpr uint32_t kD1Col = 0, kD2Col = 144, kTmemCols = 256;
-constexpr int kDwTcThreads = 128;
+constexpr int kDwTcThreads = 256, kDwDeltaThreads = 128;  // warps 4..7 compute dg2 and dlog
 constexpr uint32_t kErrTimeout = 4u;
 
 struct DwTcSmem {
   uint8_t stage[kTcStages][kStageBytes];
-  uint64_t full[kTcStages], empty[kTcStages], done;
+  float4 dlog[kTcStages][32];
+  uint64_t full[kTcStages], ready[kTcStages], empty[kTcStages], done;
   uint32_t tmem_base;
 };
 
+// Two FP32 values -> packed BF16 (round to nearest even), lo in the low half.
+__device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+
+// The TF32 operand that the tensor core reads of an FP32 value.
+__device__ __forceinline__ float tf32_trunc(float v) { return __uint_as_float(__float_as_uint(v) & 0xffffe000u); }
+
 __global__ void __launch_bounds__(kDwTcThreads, 1)
-dw_tc_kernel(Staging st, uint32_t ntiles, float* __restrict__ dw, uint32_t* __restrict__ err) {
+dw_tc_kernel(Staging st, const float* __restrict__ cw3, uint32_t ntiles, float* __restrict__ dw,
+             uint32_t* __restrict__ err) {
   extern __shared__ __align__(128) uint8_t smem_dw[];
   DwTcSmem& S = *reinterpret_cast<DwTcSmem*>(smem_dw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -799,6 +816,7 @@ dw_tc_kernel(Staging st, uint32_t ntiles, float* __restrict__ dw, uint32_t* __re
   if (threadIdx.x == 0) {
     for (int i = 0; i < kTcStages; ++i) {
       tc::mbar_init(&S.full[i], 1);
+      tc::mbar_init(&S.ready[i], kDwDeltaThreads);
       tc::mbar_init(&S.empty[i], 1);
     }
     tc::mbar_init(&S.done, 1);
@@ -828,7 +846,6 @@ dw_tc_kernel(Staging st, uint32_t ntiles, float* __restrict__ dw, uint32_t* __re
       uint8_t* a1 = S.stage[sidx];
       uint8_t* b1 = a1 + kA1Bytes;
       uint8_t* a2 = b1 + kB1Bytes;
-      uint8_t* b2 = a2 + kA2Bytes;
       const size_t t = t0 + i;
       uint64_t* bar = &S.full[sidx];
       tc::mbar_arrive_expect_tx(bar, kTileTx);
@@ -842,8 +859,7 @@ dw_tc_kernel(Staging st, uint32_t ntiles, float* __restrict__ dw, uint32_t* __re
       tc::bulk_g2s(b1 + 2 * kHid * 64, tile(st.dout, kDOut), kDOut * 64, bar);
       tc::bulk_g2s(a2, tile(st.g1, kHid), kHid * 64, bar);
       tc::bulk_g2s(a2 + kHid * 64, tile(st.g2, kHid), kHid * 64, bar);
-      tc::bulk_g2s(b2, tile(st.dg2, kHid), kHid * 64, bar);
-      tc::bulk_g2s(b2 + kHid * 64, tile(st.dlog, kFDlog), kFDlog * 64, bar);
+      tc::bulk_g2s(S.dlog[sidx], tile(st.dlog, 8), 32 * 16, bar);
       ++issued;
     }
     if (!ok) atomicExch(err, kErrTimeout);
@@ -857,7 +873,8 @@ dw_tc_kernel(Staging st, uint32_t ntiles, float* __restrict__ dw, uint32_t* __re
     constexpr uint32_t id1 = tc::idesc_bf16_f32_mn(128, 144), id2 = tc::idesc_bf16_f32_mn(128, 80);
     for (uint32_t i = 0; i < my; ++i) {
       const int sidx = (int)(i % kTcStages);
-      if (!tc::mbar_wait_sleep(&S.full[sidx], (i / kTcStages) & 1u)) {
+      if (!tc::mbar_wait_sleep(&S.full[sidx], (i / kTcStages) & 1u) ||
+          !tc::mbar_wait_sleep(&S.ready[sidx], (i / kTcStages) & 1u)) {
         atomicExch(err, kErrTimeout);
         break;
       }
@@ -872,12 +889,51 @@ dw_tc_kernel(Staging st, uint32_t ntiles, float* __restrict__ dw, uint32_t* __re
       tc::mma_commit(&S.empty[sidx]);
     }
     tc::mma_commit(&S.done);
+  } else if (warp >= 4) {  // dg2 = (dlog cW3) where g2 > 0, and dlog, as BF16 operands
+    const int f0 = 2 * (warp - 4);  // this thread's record `lane`, features 8 f0 .. 8 f0 + 15
+    float w[3][16];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int e = 0; e < 16; ++e) w[c][e] = tf32_trunc(__ldg(cw3 + c * kHid + 8 * f0 + e));
+    for (uint32_t i = 0; i < my; ++i) {
+      const int sidx = (int)(i % kTcStages);
+      if (!tc::mbar_wait_sleep(&S.full[sidx], (i / kTcStages) & 1u)) {
+        atomicExch(err, kErrTimeout);
+        break;
+      }
+      const uint8_t* g2 = S.stage[sidx] + kA1Bytes + kB1Bytes + kHid * 64;
+      uint8_t* b2 = S.stage[sidx] + kA1Bytes + kB1Bytes + kA2Bytes;
+      const float4 dl = S.dlog[sidx][lane];
+      const float d0 = tf32_trunc(dl.x), d1 = tf32_trunc(dl.y), d2 = tf32_trunc(dl.z);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int at = (f0 + h) * 512 + lane * 16;
+        const uint4 g = *reinterpret_cast<const uint4*>(g2 + at);
+        const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
+        uint32_t out[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          // g2 is never negative: its BF16 halves are positive or zero.
+          const int k = 8 * h + 2 * e;
+          const float a = fmaf(w[0][k], d0, fmaf(w[1][k], d1, w[2][k] * d2));
+          const float b = fmaf(w[0][k + 1], d0, fmaf(w[1][k + 1], d1, w[2][k + 1] * d2));
+          out[e] = bf16x2((gw[e] & 0x7fffu) ? a : 0.0f, (gw[e] & 0x7fff0000u) ? b : 0.0f);
+        }
+        *reinterpret_cast<uint4*>(b2 + at) = make_uint4(out[0], out[1], out[2], out[3]);
+      }
+      if (warp == 4)
+        *reinterpret_cast<uint4*>(b2 + 8 * 512 + lane * 16) = make_uint4(bf16x2(dl.x, dl.y), bf16x2(dl.z, 0.0f), 0u, 0u);
+      tc::fence_async_smem();
+      tc::mbar_arrive(&S.ready[sidx]);
+    }
   }
   __syncwarp();
-  // Epilogue: warp w owns TMEM lanes 32w..32w+31 (rows of D1 and D2).
-  const bool done = tc::mbar_wait_sleep(&S.done, 0);
+  // Epilogue: warp w < 4 owns TMEM lanes 32w..32w+31 (rows of D1 and D2).
+  const bool done = warp >= 4 || tc::mbar_wait_sleep(&S.done, 0);
   tc::fence_after();
-  if (!done) {
+  if (warp >= 4) {
+  } else if (!done) {
     if (lane == 0) atomicExch(err, kErrTimeout);
   } else {
     const uint32_t lanes = tmem + ((uint32_t)(warp * 32) << 16);
@@ -1096,13 +1152,6 @@ __global__ void pack_bt_images_kernel(const float* __restrict__ w, uint8_t* __re
 
 __device__ __forceinline__ uint32_t f2u(float v) { return __float_as_uint(v); }
 
-// Two FP32 values -> packed BF16 (round to nearest even), lo in the low half.
-__device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
-  uint32_t r;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-  return r;
-}
-
 // Staging of features f..f+7 (f % 8 == 0) of this thread's record as BF16,
 // in the canonical MN-major layout of a 16-bit tensor-core operand with
 // K = record: a record's 8 features are one 16-byte row, 8 records a 128-byte
@@ -1269,9 +1318,10 @@ backward_tc_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t 
 #pragma unroll
         for (int k = 0; k < 16; ++k) w16[k] = k < 3 ? f2u(dl[k]) : 0u;
         tc::tmem_st16_nowait(a_row, w16);
-        stage8(st.dlog, kFDlog, s, 0, dl[0], dl[1], dl[2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, stage);
+        // FP32: the weight-gradient kernel makes its dlog and dg2 operands of it.
+        if (stage) reinterpret_cast<float4*>(st.dlog)[s] = make_float4(dl[0], dl[1], dl[2], 0.0f);
       }
-      // Masked D[:, :64] -> staging, next A.
+      // Masked D[:, :64] -> staging (if any), next A.
       auto mask64 = [&](float* delta, const uint32_t (&m)[2]) {
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -1283,11 +1333,11 @@ backward_tc_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t 
           }
           tc::tmem_st32_nowait(a_row + 32 * c, u);
 #pragma unroll
-          for (int j = 0; j < 32; j += 8) stage8(delta, kHid, s, 32 * c + j, v[j + 0], v[j + 1], v[j + 2], v[j + 3], v[j + 4], v[j + 5], v[j + 6], v[j + 7], stage);
+          for (int j = 0; j < 32; j += 8) stage8(delta, kHid, s, 32 * c + j, v[j + 0], v[j + 1], v[j + 2], v[j + 3], v[j + 4], v[j + 5], v[j + 6], v[j + 7], stage && delta);
         }
       };
       if (!mma(5)) break;
-      mask64(st.dg2, m_g2);
+      mask64(nullptr, m_g2);
       if (!mma(6)) break;
       mask64(st.dg1, m_g1);
       if (!mma(7)) break;
@@ -1821,7 +1871,7 @@ int backward_records(nes_trainer* t, const TrainRay* rays, uint32_t total) {
       TR_CUDA(cudaGetLastError());
       const uint32_t tiles = (cnt + 31) / 32;
       const uint32_t grid = tiles < (uint32_t)sms ? tiles : (uint32_t)sms;
-      dw_tc_kernel<<<grid, kDwTcThreads, sizeof(DwTcSmem), t->st>>>(sg, tiles, gw, t->d_ctr + 1);
+      dw_tc_kernel<<<grid, kDwTcThreads, sizeof(DwTcSmem), t->st>>>(sg, c->d_weights + kOffCW3, tiles, gw, t->d_ctr + 1);
       TR_CUDA(cudaGetLastError());
     }
     scatter_kernel<<<(cnt + kScatThreads - 1) / kScatThreads, kScatThreads, 0, t->st>>>(
