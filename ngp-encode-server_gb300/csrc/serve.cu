@@ -219,14 +219,15 @@ struct nes_server {
   uint64_t next_ticket = 1, next_batch = 1;
   // Admission by expected delay: the expected cost (estimate_work) of the
   // requests admitted but not yet batched and of the batches on the GPU, and
-  // the measured service rate (cost per ms, an exponential average over
-  // completed batches; 0 until the first).  The model leaves out batching
+  // the measured service rate (cost per ms: the ratio of exponentially
+  // weighted sums over completed batches, so that two batches that finish
+  // together share their time; 0 until the first).  The model leaves out batching
   // granularity and host work between batches, so its predictions are
   // scaled by the running ratio of measured to predicted latency of
   // completed requests.  Pixel counts still bound the first batch.
   uint64_t pending_pixels = 0, inflight_pixels = 0;
   double pending_work = 0.0, inflight_work = 0.0;
-  double rate_work_per_ms = 0.0, delay_scale = 1.0;
+  double rate_work = 0.0, rate_ms = 0.0, rate_work_per_ms = 0.0, delay_scale = 1.0;
   Clock::time_point last_done;
   bool stop = false;
   nes_server_stats stats{};
@@ -422,9 +423,10 @@ void completion_main(nes_server* s) {
        // completion if the GPU was still busy with that one
       const Clock::time_point from = sl.t_launch > s->last_done ? sl.t_launch : s->last_done;
       const double ms = std::chrono::duration<double, std::milli>(now - from).count();
-      if (status == NES_OK && ms > 0.0 && sl.work > 0.0) {
-        const double r = sl.work / ms;
-        s->rate_work_per_ms = s->rate_work_per_ms > 0.0 ? 0.8 * s->rate_work_per_ms + 0.2 * r : r;
+      if (status == NES_OK && sl.work > 0.0) {
+        s->rate_work = 0.8 * s->rate_work + sl.work;
+        s->rate_ms = 0.8 * s->rate_ms + ms;
+        if (s->rate_ms > 0.0) s->rate_work_per_ms = s->rate_work / s->rate_ms;
       }
       s->last_done = now;
     }
