@@ -20,6 +20,7 @@ namespace nes {
 namespace {
 
 constexpr int kGlueThreads = 256;
+constexpr int kSms = 152;
 
 __device__ __forceinline__ uint8_t clamp8(int32_t v) { return (uint8_t)min(max(v, 0), 255); }
 
@@ -219,22 +220,30 @@ __device__ __forceinline__ uint8_t unit_q(float x) {
   return (uint8_t)__float2uint_rz(__fadd_rn(__fmul_rn(c, 255.0f), 0.5f));
 }
 
-// Depth packing: frame f = blockIdx.y, n elements per frame.  A thread has four
-// groups of four elements, all read before the first is written, a block's
-// width apart: one group per step of a grid-sized stride leaves fewer bytes in
+// Depth packing: frame f = blockIdx.y, n elements per frame.  A thread has
+// kPackGroups (four; one for inputs that do not fill the chip) groups of four
+// elements, all read before the first is written, a block's width apart: one group per step of a grid-sized stride leaves fewer bytes in
 // flight than HBM needs (30 frames of 1280 x 720, 166 MB, launch included: 77
 // us so, 70 now).  Groups as one 16-byte load when the input is 16-byte aligned
 // and the output aligned to 8 (the host checks), else element by element.
-constexpr int kPackGroups = 4;
-template <class Set>
+template <class Set, int kPackGroups>
 __global__ void __launch_bounds__(kGlueThreads) depth_pack_u16mm_kernel(const Set ds, size_t n, int vec) {
   const int f = Set::kFrames == 1 ? 0 : blockIdx.y;
   const float* __restrict__ d = ds.src[f];
   uint16_t* __restrict__ out = ds.dst[f];
   const size_t base = (size_t)blockIdx.x * (4 * kPackGroups * kGlueThreads);
   if (!vec) {
-    for (size_t e = base + threadIdx.x; e < base + 4 * kPackGroups * kGlueThreads && e < n; e += kGlueThreads)
-      out[e] = pack_mm(d[e]);
+    float x[4 * kPackGroups];
+#pragma unroll
+    for (int k = 0; k < 4 * kPackGroups; ++k) {
+      const size_t e = base + k * kGlueThreads + threadIdx.x;
+      if (e < n) x[k] = __ldg(d + e);
+    }
+#pragma unroll
+    for (int k = 0; k < 4 * kPackGroups; ++k) {
+      const size_t e = base + k * kGlueThreads + threadIdx.x;
+      if (e < n) out[e] = pack_mm(x[k]);
+    }
     return;
   }
   const size_t first = base / 4 + threadIdx.x, n4 = n / 4;
@@ -406,7 +415,11 @@ cudaError_t launch_yuv(const Set& fs, int nframes, int w, int h, int src_ls, con
 template <bool kGray, class Set>
 cudaError_t launch_yuv(const Set& fs, int nframes, int w, int h, int src_ls, const int ls[3],
                        cudaStream_t stream) {
-  int px = 16;
+  // 16 pixels per thread once they give every SM two blocks; fewer blocks leave
+  // a frame to its threads' longer chains (90 launches over 30 frames of 1280 x
+  // 720, one frame each: 409 us so, 372 with 8).
+  const size_t threads16 = (size_t)((w + 15) / 16) * (size_t)((h + 1) / 2) * (size_t)nframes;
+  int px = threads16 >= (size_t)2 * kSms * kGlueThreads ? 16 : 8;
   for (int f = 0; f < nframes; ++f)
     px = std::min(px, yuv_word(fs.src[f], src_ls, fs.y[f], fs.u[f], fs.v[f], ls));
   if (px == 16) return launch_yuv<Set, 16, kGray>(fs, nframes, w, h, src_ls, ls, stream);
@@ -418,9 +431,13 @@ template <class Set>
 cudaError_t launch_pack(const Set& ds, int nframes, size_t n, cudaStream_t stream) {
   bool vec = true;
   for (int f = 0; f < nframes; ++f) vec = vec && aligned(ds.src[f], 16) && aligned(ds.dst[f], 8);
-  constexpr size_t kPerBlock = 4 * kPackGroups * kGlueThreads;
-  const dim3 grid((unsigned)((n + kPerBlock - 1) / kPerBlock), nframes);
-  depth_pack_u16mm_kernel<<<grid, kGlueThreads, 0, stream>>>(ds, n, vec);
+  const bool full = n * (size_t)nframes >= (size_t)2 * kSms * 16 * kGlueThreads;  // as launch_yuv
+  const size_t per_block = (full ? 16 : 4) * kGlueThreads;
+  const dim3 grid((unsigned)((n + per_block - 1) / per_block), nframes);
+  if (full)
+    depth_pack_u16mm_kernel<Set, 4><<<grid, kGlueThreads, 0, stream>>>(ds, n, vec);
+  else
+    depth_pack_u16mm_kernel<Set, 1><<<grid, kGlueThreads, 0, stream>>>(ds, n, vec);
   return cudaGetLastError();
 }
 
