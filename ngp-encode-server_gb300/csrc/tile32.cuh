@@ -58,20 +58,20 @@ __device__ __forceinline__ float4 relu4(const float4& v) {
   return make_float4(fmaxf(v.x, 0.0f), fmaxf(v.y, 0.0f), fmaxf(v.z, 0.0f), fmaxf(v.w, 0.0f));
 }
 
-// X[0..64) = ep(W^T in[0..K)) for the warp's samples, W [K][64] (in may be X);
-// ep(i, row, sample, v) gets this lane's i-th four outputs (i < 16): output
-// `row` of samples sample .. sample + 3.  Around each eight inputs' products, bg.begin(i) and bg.finish(i), i =
-// kBg + (input / 8): other work whose memory reads they hide.  A lane
-// has samples 4 sg + {0..3, 16..19} and outputs 4 og + {0..3, 32..35}, the
-// samples two by two in packed FMAs.  A 16-byte shared-memory read costs two
-// passes instead of four when lanes i and i ^ 1 (or i ^ 2) want the same
-// address: bit 0 of the lane is og's and bit 1 is sg's, so both operands' reads
-// do.  Seeded 1080p view: 232 ms one sample per thread; 155 ms as a product
-// with sg in bits 0-1 (four passes for the activations), 150 ms so, 145 ms
-// with packed FMAs (12 warps, 32 steps per ray).
-template <int K, int kBg, class Bg, class Ep>
-__device__ __forceinline__ void tile_layer64(const float* __restrict__ W, const float* in, float* X, int lane, Bg& bg,
-                                             Ep&& ep) {
+// X[0..64) = ep(W^T in[0..K)) for the warp's samples, W [K][64], K a multiple
+// of 8 (in may be X); ep(i, row, sample, v) gets this lane's i-th four outputs
+// (i < 16): output `row` of samples sample .. sample + 3.  Around each eight
+// inputs' products, bg.begin(i) and bg.finish(i), i = bg0 + (input / 8): other
+// work whose memory reads they hide.  A lane has samples 4 sg + {0..3, 16..19}
+// and outputs 4 og + {0..3, 32..35}, the samples two by two in packed FMAs.  A
+// 16-byte shared-memory read costs two passes instead of four when lanes i and
+// i ^ 1 (or i ^ 2) want the same address: bit 0 of the lane is og's and bit 1
+// is sg's, so both operands' reads do.  Seeded 1080p view: 232 ms one sample per
+// thread; 155 ms as a product with sg in bits 0-1 (four passes for the
+// activations), 150 ms so, 145 ms with packed FMAs (12 warps, 32 steps per ray).
+template <class Bg, class Ep>
+__device__ __forceinline__ void tile_layer64(const float* __restrict__ W, int K, const float* in, float* X, int lane,
+                                             Bg& bg, int bg0, Ep&& ep) {
   const int sg = 4 * ((lane >> 1) & 3), og = 4 * ((lane & 1) | ((lane >> 2) & 6));
   unsigned long long acc[8][4];  // [output][pair of samples]
 #pragma unroll
@@ -80,7 +80,7 @@ __device__ __forceinline__ void tile_layer64(const float* __restrict__ W, const 
     for (int s = 0; s < 4; ++s) acc[o][s] = 0ull;
 #pragma unroll 1
   for (int k0 = 0; k0 < K; k0 += 8) {
-    bg.begin(kBg + k0 / 8);
+    bg.begin(bg0 + k0 / 8);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const float* xr = in + (k0 + k) * 32;
@@ -99,7 +99,7 @@ __device__ __forceinline__ void tile_layer64(const float* __restrict__ W, const 
       }
     }
     __syncwarp();  // in[k0 .. k0 + 8) has been read: finish may write there
-    bg.finish(kBg + k0 / 8);
+    bg.finish(bg0 + k0 / 8);
   }
   __syncwarp();
   const int swap = tile_swap(og);
@@ -188,16 +188,23 @@ struct NoOtherWork {
 // Both MLPs of the warp's samples, whose 32 encoded features are in E; X is
 // scratch.  Every lane gets its own sample's density and colour; d is its
 // direction.  bg.begin(i) and bg.finish(i) are called for i = 0..15 on the
-// way; after finish(i), rows 2 i and 2 i + 1 of E are free.
+// way; after finish(i), rows 2 i and 2 i + 1 of E are free.  The three 64-wide
+// layers run through one copy of the product: with three, the march waited for
+// instructions (0.46 of its stalls per issue), 128.1 ms per 1080p view; 120.4
+// so.
 template <class Bg>
 __device__ __forceinline__ float tile_mlp32(const TileWeights32& W, const float* E, float* X, int lane,
                                             const float3& d, float3* rgb, Bg& bg) {
-  const auto relu = [](int, int, int, const float4& v) { return relu4(v); };
-  tile_layer64<kEnc, 0>(W.dw1, E, X, lane, bg, relu);
-  float sh[16];
-  const float logit = tile_colour_input(W.dw2, X, lane, d, sh);
-  tile_layer64<kCIn, 4>(W.cw1, X, X, lane, bg, relu);
-  tile_layer64<kHid, 8>(W.cw2, X, X, lane, bg, relu);
+  float logit = 0.0f;
+#pragma unroll 1
+  for (int layer = 0; layer < 3; ++layer) {
+    tile_layer64(layer == 0 ? W.dw1 : layer == 1 ? W.cw1 : W.cw2, layer < 2 ? 32 : 64, layer == 0 ? E : X, X, lane, bg,
+                 4 * layer, [](int, int, int, const float4& v) { return relu4(v); });
+    if (layer == 0) {
+      float sh[16];
+      logit = tile_colour_input(W.dw2, X, lane, d, sh);
+    }
+  }
   const float3 lg = tile_logits(W.cw3, X, lane);
   *rgb = make_float3(sigmoidf(lg.x), sigmoidf(lg.y), sigmoidf(lg.z));
   return expf(logit - 1.0f);

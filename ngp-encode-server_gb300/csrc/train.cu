@@ -8,7 +8,7 @@
 //  1. rays: (view, pixel) pairs (drawn from the step seed or given) -> the
 //     FP32 ray set-up of rendering, with the target colour and depth;
 //  2. forward, as many rays at a time as the sample list holds: the rays'
-//     occupied steps listed (thread per ray), each listed sample's hash-grid
+//     occupied steps listed (warp per ray), each listed sample's hash-grid
 //     encoding gathered (encode_kernel; kept for the backward), the MLPs
 //     evaluated (by default on the tensor cores as 3xTF32, FP32-level;
 //     exact_weight_grads = 1: FP32 on the CUDA cores), then each ray
@@ -562,7 +562,7 @@ backward_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t cou
     }
     uint64_t m_h1 = 0, m_g1 = 0, m_g2 = 0;
     float* rows = stage_tile(st.h1, kHid, tile);
-    tile_layer64<kEnc, 0>(S.w.dw1, X, X, lane, none, [&](int i, int row, int sample, const float4& v) {
+    tile_layer64(S.w.dw1, kEnc, X, X, lane, none, 0, [&](int i, int row, int sample, const float4& v) {
       m_h1 |= positive4(v, i);
       return put(rows, row, sample, relu4(v));
     });
@@ -572,12 +572,12 @@ backward_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t cou
 #pragma unroll
     for (int k = 0; k < kCIn; ++k) rows[k * 32 + lane] = k < 16 ? sh[k] : X[k * 32 + (lane ^ tile_swap(k))];
     rows = stage_tile(st.g1, kHid, tile);
-    tile_layer64<kCIn, 0>(S.w.cw1, X, X, lane, none, [&](int i, int row, int sample, const float4& v) {
+    tile_layer64(S.w.cw1, kCIn, X, X, lane, none, 0, [&](int i, int row, int sample, const float4& v) {
       m_g1 |= positive4(v, i);
       return put(rows, row, sample, relu4(v));
     });
     rows = stage_tile(st.g2, kHid, tile);
-    tile_layer64<kHid, 0>(S.w.cw2, X, X, lane, none, [&](int i, int row, int sample, const float4& v) {
+    tile_layer64(S.w.cw2, kHid, X, X, lane, none, 0, [&](int i, int row, int sample, const float4& v) {
       m_g2 |= positive4(v, i);
       return put(rows, row, sample, relu4(v));
     });
@@ -617,7 +617,7 @@ backward_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t cou
     }
     __syncwarp();
     rows = stage_tile(st.dg1, kHid, tile);
-    tile_layer64<kHid, 0>(S.cw2, X, X, lane, none, [&](int i, int row, int sample, const float4& v) {
+    tile_layer64(S.cw2, kHid, X, X, lane, none, 0, [&](int i, int row, int sample, const float4& v) {
       return put(rows, row, sample, masked4(v, m_g1, i));
     });
     rows = stage_tile(st.dout, kDOut, tile);
@@ -628,7 +628,7 @@ backward_kernel(const SampleRec* __restrict__ recs, uint32_t first, uint32_t cou
     X[lane] = rows[lane] = q.dsigma * sigma;  // row 0
     __syncwarp();
     rows = stage_tile(st.dh1, kHid, tile);
-    tile_layer64<kDOut, 0>(S.dw2, X, X, lane, none, [&](int i, int row, int sample, const float4& v) {
+    tile_layer64(S.dw2, kDOut, X, X, lane, none, 0, [&](int i, int row, int sample, const float4& v) {
       return put(rows, row, sample, masked4(v, m_h1, i));
     });
     {  // the encoding's gradient: samples 4 sg + {0..3, 16..19}, features 4 og + {0..3}, a chunk of denc
