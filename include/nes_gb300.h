@@ -312,8 +312,8 @@ void nes_train_config_default(nes_train_config *cfg);
  * 200 B per listed sample (list entry, encoding, state and adjoint record) for
  * up to 1024 steps of every ray or 2^26 samples (13.4 GB), whichever is less
  * -- a larger batch goes through in parts --, ~3.9 GB of per-sample staging
- * for the weight gradients, 0.5 GB of encoding gradients in the tensor-core
- * mode, 4x the table for gradient and Adam moments, and ~160 KB of weight
+ * for the weight gradients, 0.5 GB of encoding gradients (strict mode 0.25),
+ * 4x the table for gradient and Adam moments, and ~160 KB of weight
  * operand images. */
 int nes_trainer_create(nes_ctx *student, const nes_train_config *cfg, nes_trainer **out);
 void nes_trainer_destroy(nes_trainer *tr);
