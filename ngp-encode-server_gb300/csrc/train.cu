@@ -1890,9 +1890,14 @@ int train_error(uint32_t word) {
   }
 }
 
-// Loss and gradients (accumulated into d_gtable / d_gw) for the n rays in
-// d_rays, as many blocks of kRayBlock rays at a time as the sample list holds.
-int loss_and_grad(nes_trainer* t, int n, double* loss) {
+int clear_gradients(nes_trainer* t) {
+  TR_CUDA(cudaMemsetAsync(t->d_gtable, 0, (size_t)kLevels * t->ctx->scene.T * sizeof(float2), t->st));
+  TR_CUDA(cudaMemsetAsync(t->d_gw, 0, kWeightFloats * sizeof(float), t->st));
+  TR_CUDA(cudaStreamSynchronize(t->st));
+  return NES_OK;
+}
+
+int accumulate_parts(nes_trainer* t, int n, double* loss) {
   nes_ctx* c = t->ctx;
   const int blocks = (n + kRayBlock - 1) / kRayBlock;
   t->last_samples = 0;
@@ -1965,6 +1970,15 @@ int loss_and_grad(nes_trainer* t, int n, double* loss) {
     b0 = b1;
   }
   return NES_OK;
+}
+
+// Loss and gradients (accumulated into d_gtable / d_gw) for the n rays in
+// d_rays, as many blocks of kRayBlock rays at a time as the sample list holds.
+// A batch that fails in one part leaves no gradient of its earlier ones.
+int loss_and_grad(nes_trainer* t, int n, double* loss) {
+  const int rc = accumulate_parts(t, n, loss);
+  if (rc != NES_OK) clear_gradients(t);
+  return rc;
 }
 
 int upload_rays(nes_trainer* t, const int32_t* rays, int n) {
@@ -2193,14 +2207,15 @@ int nes_trainer_grad(nes_trainer* t, const int32_t* rays, int n, double* loss, f
   int rc = upload_rays(t, rays, n);
   if (rc == NES_OK) rc = loss_and_grad(t, n, loss);
   const size_t nt = (size_t)kLevels * t->ctx->scene.T * 2;
-  if (rc == NES_OK && grad_table)
-    TR_CUDA(cudaMemcpyAsync(grad_table, t->d_gtable, nt * sizeof(float), cudaMemcpyDeviceToHost, t->st));
-  if (rc == NES_OK && grad_weights)
-    TR_CUDA(cudaMemcpyAsync(grad_weights, t->d_gw, kWeightFloats * sizeof(float), cudaMemcpyDeviceToHost, t->st));
-  TR_CUDA(cudaMemsetAsync(t->d_gtable, 0, nt * sizeof(float), t->st));
-  TR_CUDA(cudaMemsetAsync(t->d_gw, 0, kWeightFloats * sizeof(float), t->st));
-  TR_CUDA(cudaStreamSynchronize(t->st));
-  return rc;
+  if (rc == NES_OK && grad_table &&
+      cudaMemcpyAsync(grad_table, t->d_gtable, nt * sizeof(float), cudaMemcpyDeviceToHost, t->st) != cudaSuccess)
+    rc = NES_EIO;
+  if (rc == NES_OK && grad_weights &&
+      cudaMemcpyAsync(grad_weights, t->d_gw, kWeightFloats * sizeof(float), cudaMemcpyDeviceToHost, t->st) !=
+          cudaSuccess)
+    rc = NES_EIO;
+  const int cleared = clear_gradients(t);
+  return rc != NES_OK ? rc : cleared;
 }
 
 int nes_trainer_loss_fp64(nes_trainer* t, const int32_t* rays, int n, int which, uint64_t index, double delta,
