@@ -49,6 +49,9 @@ cudaError_t launch_raygen(const ViewBatch* views_dev, uint32_t max_pixels, int n
 
 // Plain FP32 march: persistent CTAs pull compacted rays, evaluate the FP32
 // table + FP32 MLP on CUDA cores and composite.
+// prepare_march_fp32 comes first, once per device, with that device current: a
+// kernel's shared-memory opt-in belongs to the device it is made on.
+cudaError_t prepare_march_fp32();
 cudaError_t launch_march_fp32(const ViewBatch& views, const DevScene& scene, const DevScratch& s,
                               int num_sms, cudaStream_t stream);
 cudaError_t launch_march_fp32(const ViewBatch* views_dev, const DevScene& scene, const DevScratch& s, int num_sms,
@@ -56,6 +59,8 @@ cudaError_t launch_march_fp32(const ViewBatch* views_dev, const DevScene& scene,
 
 // FP16 tensor-core march (tcgen05 MLP).  Needs scene.table16 and
 // scene.tc_weights (the FP16 operand image from launch_pack_tc_weights).
+// prepare_march_tc (the scene's rec_levels) comes first, as prepare_march_fp32.
+cudaError_t prepare_march_tc(int rec_levels);
 cudaError_t launch_march_tc(const ViewBatch& views, const DevScene& scene, const DevScratch& s,
                             int num_sms, cudaStream_t stream);
 cudaError_t launch_march_tc(const ViewBatch* views_dev, const DevScene& scene, const DevScratch& s, int num_sms,

@@ -711,21 +711,26 @@ cudaError_t launch_pack_tc_weights(const float* w32, uint8_t* out, cudaStream_t 
 namespace {
 
 template <class Src, int kRec>
+cudaError_t prepare_march_tc_rec() {
+  const cudaError_t e =
+      cudaFuncSetAttribute(march_tc_kernel<Src, kRec>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemRequest);
+  if (e != cudaSuccess) return e;
+  // 14 % of 228 KiB selects the 32 KiB configuration, which holds the
+  // request: the rest of the SM's 256 KiB stays L1 for the table gathers.
+  return cudaFuncSetAttribute(march_tc_kernel<Src, kRec>, cudaFuncAttributePreferredSharedMemoryCarveout, 14);
+}
+
+template <int kRec>
+cudaError_t prepare_march_tc_rec() {
+  const cudaError_t e = prepare_march_tc_rec<InParam<ViewBatch>, kRec>();
+  return e != cudaSuccess ? e : prepare_march_tc_rec<InMemory<ViewBatch>, kRec>();
+}
+
+template <class Src, int kRec>
 cudaError_t launch_march_tc_rec(const Src& src, const DevScene& scene, const DevScratch& s, int num_sms,
                                 cudaStream_t stream) {
   if (!scene.table16 || !scene.rec16 || !scene.tc_weights) return cudaErrorInvalidValue;
   if (s.max_rays > kIdMask) return cudaErrorInvalidValue;  // ray ids share a word with the flags
-  static bool attr_set = false;  // idempotent; a race only repeats the calls
-  if (!attr_set) {
-    cudaError_t e =
-        cudaFuncSetAttribute(march_tc_kernel<Src, kRec>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemRequest);
-    if (e != cudaSuccess) return e;
-    // 14 % of 228 KiB selects the 32 KiB configuration, which holds the
-    // request: the rest of the SM's 256 KiB stays L1 for the table gathers.
-    e = cudaFuncSetAttribute(march_tc_kernel<Src, kRec>, cudaFuncAttributePreferredSharedMemoryCarveout, 14);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
   // One CTA per SM is what makes the 512-column TMEM allocation safe: two
   // 1024-thread CTAs fit on an SM only at <= 32 registers per thread.
   cudaFuncAttributes fa;
@@ -749,6 +754,12 @@ cudaError_t launch_march_tc_src(const Src& src, const DevScene& scene, const Dev
 }
 
 }  // namespace
+
+cudaError_t prepare_march_tc(int rec_levels) {
+  if (rec_levels == kRecLevelsDefault) return prepare_march_tc_rec<kRecLevelsDefault>();
+  if (rec_levels == kRecLevelsSmall) return prepare_march_tc_rec<kRecLevelsSmall>();
+  return cudaErrorInvalidValue;
+}
 
 cudaError_t launch_march_tc(const ViewBatch& views, const DevScene& scene, const DevScratch& s, int num_sms,
                             cudaStream_t stream) {

@@ -341,18 +341,18 @@ namespace {
 template <class Src>
 cudaError_t launch_march_fp32_src(const Src& src, const DevScene& scene, const DevScratch& s, int num_sms,
                                   cudaStream_t stream) {
-  const int smem = (int)sizeof(MarchSmem32);
-  static bool attr_set = false;  // idempotent; harmless if two threads race on it
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(march_fp32_kernel<Src>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
-  march_fp32_kernel<Src><<<num_sms, kMarchThreads, smem, stream>>>(src, scene, s);
+  march_fp32_kernel<Src><<<num_sms, kMarchThreads, sizeof(MarchSmem32), stream>>>(src, scene, s);
   return cudaGetLastError();
 }
 
 }  // namespace
+
+cudaError_t prepare_march_fp32() {
+  const cudaFuncAttribute dynamic = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  const int smem = (int)sizeof(MarchSmem32);
+  const cudaError_t e = cudaFuncSetAttribute(march_fp32_kernel<InParam<ViewBatch>>, dynamic, smem);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(march_fp32_kernel<InMemory<ViewBatch>>, dynamic, smem);
+}
 
 cudaError_t launch_march_fp32(const ViewBatch& views, const DevScene& scene, const DevScratch& s,
                               int num_sms, cudaStream_t stream) {

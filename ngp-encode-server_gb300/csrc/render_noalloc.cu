@@ -63,6 +63,7 @@ int scratch_for_current_device(unsigned char** base, int* sms) {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || p == nullptr) return NES_EIO;
     int n = 0;
+    if (prepare_march_fp32() != cudaSuccess) return NES_EIO;
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return NES_EIO;
     g_scratch_dev[dev] = p;
     g_num_sms[dev] = n;

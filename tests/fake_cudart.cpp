@@ -20,7 +20,14 @@ std::map<const void*, std::string>& kernels() {
 std::map<void*, size_t> allocs;  // live device allocations
 size_t allocated = 0;
 int device = 0;                  // current
-std::map<std::pair<int, const void*>, int> max_dynamic_smem;  // per device and kernel: the opt-in, if made
+int devices = 1;
+int num_regs = 128;
+// Per device and kernel, as set.
+std::map<std::pair<int, const void*>, int> max_dynamic_smem, carveout;
+int attribute(const std::map<std::pair<int, const void*>, int>& of, const void* kernel, int unset) {
+  const auto it = of.find({device, kernel});
+  return it == of.end() ? unset : it->second;
+}
 cudaError_t last = cudaSuccess;
 struct Config {
   dim3 grid, block;
@@ -57,26 +64,39 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3 block, void** arg
   const void* host = reinterpret_cast<const void*>(k);
   // More than 48 KiB of dynamic shared memory need the kernel's opt-in on the
   // current device.
-  const auto opt = fake::max_dynamic_smem.find({fake::device, host});
-  const size_t limit = opt == fake::max_dynamic_smem.end() ? 48u << 10 : (size_t)opt->second;
+  const size_t limit = (size_t)fake::attribute(fake::max_dynamic_smem, host, 48 << 10);
   const cudaError_t e = smem > limit ? cudaErrorInvalidValue
-                                     : on_launch(FakeLaunch{fake::kernels()[host], grid, block, smem, args});
+                                     : on_launch(FakeLaunch{fake::kernels()[host], grid, block, smem,
+                                                            fake::attribute(fake::carveout, host, -1), args});
   if (e != cudaSuccess) fake::last = e;
   return e;
 }
 
 cudaError_t cudaGetLastError() { return std::exchange(fake::last, cudaSuccess); }
+cudaError_t cudaGetDeviceCount(int* n) {
+  *n = fake::devices;
+  return cudaSuccess;
+}
+cudaError_t cudaGetDevice(int* d) {
+  *d = fake::device;
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) {  // asked for the SM count only
+  *v = 152;
+  return cudaSuccess;
+}
 cudaError_t cudaSetDevice(int d) {
   fake::device = d;
   return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute a, int v) {
   if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) fake::max_dynamic_smem[{fake::device, f}] = v;
+  if (a == cudaFuncAttributePreferredSharedMemoryCarveout) fake::carveout[{fake::device, f}] = v;
   return cudaSuccess;
 }
 cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) {
   std::memset(a, 0, sizeof(*a));
-  a->numRegs = 128;
+  a->numRegs = fake::num_regs;
   return cudaSuccess;
 }
 cudaError_t cudaMalloc(void** p, size_t n) {
@@ -115,12 +135,36 @@ cudaError_t cudaMemset(void* d, int v, size_t n) {
   return cudaSuccess;
 }
 cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return cudaMemset(d, v, n); }
+cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size_t w, size_t h, cudaMemcpyKind,
+                              cudaStream_t) {
+  for (size_t y = 0; y < h; ++y) std::memcpy(static_cast<char*>(d) + y * dp, static_cast<const char*>(s) + y * sp, w);
+  return cudaSuccess;
+}
+cudaError_t cudaGetSymbolAddress(void** p, const void* symbol) {  // a block larger than any of the library's arrays
+  static std::map<std::pair<int, const void*>, void*> at;
+  void*& m = at[{fake::device, symbol}];
+  if (!m) m = std::calloc(16u << 20, 1);
+  *p = m;
+  return m ? cudaSuccess : cudaErrorMemoryAllocation;
+}
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
   *s = nullptr;
   return cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaErrorNotSupported; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t*) { return cudaErrorNotSupported; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t*, cudaGraph_t, unsigned long long) { return cudaErrorNotSupported; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaErrorNotSupported; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+  *e = nullptr;
+  return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t* e) {
   *e = nullptr;
   return cudaSuccess;

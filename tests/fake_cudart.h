@@ -8,6 +8,7 @@ struct FakeLaunch {
   std::string name;  // mangled
   dim3 grid, block;
   size_t smem;
+  int carveout;  // the kernel's preferred shared-memory carveout on the current device, or -1
   void** args;
   bool is(const char* kernel) const { return name.find(kernel) != std::string::npos; }
   template <class T>
@@ -21,4 +22,6 @@ cudaError_t on_launch(const FakeLaunch& l);
 
 namespace fake {
 extern size_t allocated;  // bytes of the live device allocations
+extern int devices;       // their number
+extern int num_regs;      // registers per thread that every kernel reports
 }
