@@ -308,13 +308,13 @@ typedef struct nes_train_config {
 void nes_train_config_default(nes_train_config *cfg);
 
 /* The student must be an NES_PREC_FP32 context; its table and weights are
- * updated in place by the step calls.  batch_rays <= 2^20.  Device memory:
- * 200 B per listed sample (list entry, encoding, state and adjoint record) for
- * up to 1024 steps of every ray or 2^26 samples (13.4 GB), whichever is less
- * -- a larger batch goes through in parts --, ~3.9 GB of per-sample staging
- * for the weight gradients, 0.5 GB of encoding gradients (strict mode 0.25),
- * 4x the table for gradient and Adam moments, and ~160 KB of weight
- * operand images. */
+ * updated in place by the step calls.  batch_rays <= 2^20.  Device memory: at
+ * most 64 KiB per ray of the batch plus 3.96 GB -- 168 B per listed sample
+ * (list entry, encoding, adjoint record) for up to 512 samples of every ray,
+ * never more than 2^26 (11.3 GB), a batch that lists more going through in
+ * parts, and up to 4.2 GB for a backward chunk's staging and encoding gradients --,
+ * 3x the table for gradient and Adam moments, and ~160 KB of weight operand
+ * images. */
 int nes_trainer_create(nes_ctx *student, const nes_train_config *cfg, nes_trainer **out);
 void nes_trainer_destroy(nes_trainer *tr);
 

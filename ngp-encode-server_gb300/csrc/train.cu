@@ -159,7 +159,7 @@ struct RayOut {  // composited result of one training ray
 //  1. count_kernel and scan_kernel: the rays' occupied steps -- the march's
 //     sample set before early termination -- counted, and their places in a
 //     list of all of them, ray after ray;
-// then for as many rays at a time as kListSamples samples hold:
+// then for as many rays at a time as the list holds (trainer_sizes):
 //  2. list_kernel, warp per ray: (ray, step) of each sample;
 //  3. encode_kernel, thread per listed sample: the hash-grid encoding, kept
 //     for the backward (a warp's samples are consecutive samples of one or two
@@ -179,8 +179,6 @@ struct RayOut {  // composited result of one training ray
 // per-ray kernels took 1.21 of a strict gradient's 8.4 ms, 0.52 in single
 // warps; of 2^18 rays the same).  Counting and listing have a warp per ray.
 constexpr int kRayBlock = 32;
-constexpr uint32_t kListSamples = 1u << 26;  // samples listed at a time
-static_assert((uint32_t)kRayBlock * kMaxSteps <= kListSamples, "a block of rays fits the list");
 
 // A ray per thread left a small batch's walk serial over ~800 steps and its
 // list entries scattered (counting and listing 4,001 rays: 65 + 71 us; 17 + 19
@@ -1780,8 +1778,8 @@ struct nes_trainer {
   uint32_t max_rays = 0;
   int2* d_pairs = nullptr;
   TrainRay* d_rays = nullptr;
-  // Per listed sample (list_capacity of each): list entry, encoding, state
-  // and record of the backward.
+  // Per listed sample (list_capacity of each): list entry, encoding, state (in
+  // d_stage) and record of the backward.
   uint32_t list_capacity = 0;
   uint2* d_list = nullptr;
   float* d_enc = nullptr;
@@ -1796,11 +1794,11 @@ struct nes_trainer {
   float2* d_gtable = nullptr;
   float* d_gw = nullptr;
   float *d_mt = nullptr, *d_vt = nullptr, *d_mw = nullptr, *d_vw = nullptr;
-  float* d_stage = nullptr;
+  void* d_stage = nullptr;  // a backward chunk's staging; before it, the part's d_scratch
   float* d_denc = nullptr;  // encoding gradients of a backward chunk, tiled as d_enc
   uint8_t* d_bimg = nullptr;  // TF32 weight images of backward_tc_kernel
   uint8_t* d_eimg = nullptr;  // high/low TF32 forward images of eval_tc_kernel
-  uint32_t chunk = 0;
+  uint32_t chunk = 0;  // records of a backward chunk
   uint64_t steps = 0;
   uint64_t last_samples = 0;
   // Phase events on the trainer's stream: 0 start of a part's forward, 1 its
@@ -1819,20 +1817,57 @@ namespace {
   } while (0)
 
 
+// A staged record's bytes: FP32 in the strict mode; the tensor-core mode has
+// BF16 (dlog as four FP32), and dg2 is not staged there.
+constexpr size_t stage_bytes(bool exact) { return exact ? kStageFloats * sizeof(float) : (kStageFloats - kHid) * 2; }
+
+// Samples of the list and records of a backward chunk, by the trainer's device
+// memory: at most 64 KiB per ray of the batch and kTrainBytes (8 MB less than
+// the FP32 staging of 2^21 records, for the small arrays).  A record takes
+// stage_bytes and its encoding gradient, a listed sample kSampleBytes; its
+// state, read for the last time before the first record is staged, lies in the
+// staging.  The list gets 512 samples a ray (a view of the seeded field, occupied
+// throughout, lists 465) while the chunk keeps half its largest size, the chunk
+// the rest.  Batches of 180,000 rays and more have both at their largest.  With
+// the list at 1024 samples a ray and the largest chunk, 65,536 rays took 17.9
+// GB in place of 8.2.
+constexpr size_t kSampleBytes = sizeof(uint2) + kEnc * sizeof(float) + sizeof(SampleRec);
+constexpr size_t kTrainBytes = ((size_t)1 << 21) * kStageFloats * sizeof(float) - ((size_t)8 << 20);
+constexpr size_t kListSamples = (size_t)1 << 26;
+struct TrainerSizes {
+  size_t samples, records, stage_bytes;  // multiples of 32 and of 128
+};
+TrainerSizes trainer_sizes(size_t rays, bool exact) {
+  const size_t stage = stage_bytes(exact), record = stage + kEnc * sizeof(float), most = (size_t)1 << (exact ? 21 : 22);
+  const size_t bytes = rays * (64u << 10) + kTrainBytes, block = std::min<size_t>(rays, kRayBlock) * kMaxSteps;
+  TrainerSizes z;
+  z.samples = std::min({rays * 512, kListSamples, (bytes - most / 2 * record) / kSampleBytes});
+  z.samples = std::max(z.samples, block) & ~(size_t)31;  // a block of rays fits
+  z.records = std::min({most, rays * kMaxSteps, (bytes - z.samples * kSampleBytes) / record}) & ~(size_t)127;
+  z.samples = std::max(std::min(z.samples, z.records * stage / sizeof(ScratchSample)), block) & ~(size_t)31;
+  z.stage_bytes = std::max(z.records * stage, z.samples * sizeof(ScratchSample));
+  return z;
+}
+
 Staging staging(const nes_trainer* t) {
-  Staging s;
-  float* p = t->d_stage;
-  const size_t S = t->chunk;
-  s.enc = p; p += S * kEnc;
-  s.h1 = p; p += S * kHid;
-  s.cin = p; p += S * kCIn;
-  s.g1 = p; p += S * kHid;
-  s.g2 = p; p += S * kHid;
-  s.dh1 = p; p += S * kHid;
-  s.dout = p; p += S * kDOut;
-  s.dg1 = p; p += S * kHid;
-  s.dg2 = p; p += S * kHid;
-  s.dlog = p;
+  Staging s{};
+  const bool exact = t->cfg.exact_weight_grads != 0;
+  float* p = static_cast<float*>(t->d_stage);
+  auto take = [&](int F) {  // an F-wide array of the chunk's records, FP32 or BF16
+    float* const a = p;
+    p += (size_t)t->chunk * F / (exact ? 1 : 2);
+    return a;
+  };
+  s.enc = take(kEnc);
+  s.h1 = take(kHid);
+  s.cin = take(kCIn);
+  s.g1 = take(kHid);
+  s.g2 = take(kHid);
+  s.dh1 = take(kHid);
+  s.dout = take(kDOut);
+  s.dg1 = take(kHid);
+  if (exact) s.dg2 = take(kHid);
+  s.dlog = take(kFDlog);
   return s;
 }
 
@@ -1849,10 +1884,8 @@ int backward_records(nes_trainer* t, const TrainRay* rays, uint32_t total) {
   const Staging sg = staging(t);
   float* gw = t->d_gw;
   const int sms = c->num_sms;
-  // BF16 staging (tensor-core mode) holds twice the records in the same bytes.
-  const uint32_t chunk = t->cfg.exact_weight_grads ? t->chunk : 2u * t->chunk;
-  for (uint32_t first = 0; first < total; first += chunk) {
-    const uint32_t cnt = total - first < chunk ? total - first : chunk;
+  for (uint32_t first = 0; first < total; first += t->chunk) {
+    const uint32_t cnt = std::min(total - first, t->chunk);
     if (t->cfg.exact_weight_grads) {
       const uint32_t tiles = (cnt + 31) / 32, want = (tiles + kBwdWarps - 1) / kBwdWarps;
       backward_kernel<<<want < (uint32_t)sms ? want : (uint32_t)sms, 32 * kBwdWarps, (int)sizeof(BackwardSmem),
@@ -2019,7 +2052,6 @@ void free_trainer(nes_trainer* t) {
   cudaFree(t->d_rays);
   cudaFree(t->d_list);
   cudaFree(t->d_enc);
-  cudaFree(t->d_scratch);
   cudaFree(t->d_recs);
   cudaFree(t->d_block_count);
   cudaFree(t->d_block_first);
@@ -2080,19 +2112,19 @@ int nes_trainer_create(nes_ctx* ctx, const nes_train_config* cfg, nes_trainer** 
   for (cudaEvent_t& e : t->ev)
     if (cudaEventCreate(&e) != cudaSuccess) return fail(NES_EIO);
   const size_t nt = (size_t)kLevels * ctx->scene.T * 2;
-  // Every step of every ray, or as many samples as are listed at a time.
   const size_t blocks = (t->max_rays + kRayBlock - 1) / kRayBlock;
-  const size_t max_samples = std::min<size_t>((size_t)t->max_rays * kMaxSteps, kListSamples);
-  t->list_capacity = (uint32_t)max_samples;
-  t->chunk = 1u << 21;
+  const bool exact = cfg->exact_weight_grads != 0;
+  const TrainerSizes sizes = trainer_sizes(t->max_rays, exact);
+  const size_t max_samples = sizes.samples;
+  t->list_capacity = (uint32_t)sizes.samples;
+  t->chunk = (uint32_t)sizes.records;
   if (cudaMalloc(&t->d_pairs, (size_t)t->max_rays * sizeof(int2)) != cudaSuccess ||
       cudaMalloc(&t->d_rays, (size_t)t->max_rays * sizeof(TrainRay)) != cudaSuccess ||
       cudaMalloc(&t->d_list, max_samples * sizeof(uint2)) != cudaSuccess ||
-      cudaMalloc(&t->d_enc, (max_samples + 31) / 32 * kEncTileFloats * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&t->d_enc, max_samples * kEnc * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&t->d_block_count, blocks * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&t->d_block_first, (blocks + 1) * sizeof(uint32_t)) != cudaSuccess ||
       cudaMallocHost(&t->h_block_first, (blocks + 1) * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&t->d_scratch, max_samples * sizeof(ScratchSample)) != cudaSuccess ||
       cudaMalloc(&t->d_recs, max_samples * sizeof(SampleRec)) != cudaSuccess ||
       cudaMalloc(&t->d_rout, (size_t)t->max_rays * sizeof(RayOut)) != cudaSuccess ||
       cudaMalloc(&t->d_ctr, 4 * sizeof(uint32_t)) != cudaSuccess ||
@@ -2103,12 +2135,12 @@ int nes_trainer_create(nes_ctx* ctx, const nes_train_config* cfg, nes_trainer** 
       cudaMalloc(&t->d_vt, nt * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&t->d_mw, kWeightFloats * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&t->d_vw, kWeightFloats * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&t->d_stage, (size_t)t->chunk * kStageFloats * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&t->d_denc, (size_t)(cfg->exact_weight_grads ? 1 : 2) * t->chunk * kEnc * sizeof(float)) !=
-          cudaSuccess ||
+      cudaMalloc(&t->d_stage, sizes.stage_bytes) != cudaSuccess ||
+      cudaMalloc(&t->d_denc, (size_t)t->chunk * kEnc * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&t->d_bimg, kBtImageBytes) != cudaSuccess ||
       cudaMalloc(&t->d_eimg, kEtImageBytes) != cudaSuccess)
     return fail(NES_ENOMEM);
+  t->d_scratch = static_cast<ScratchSample*>(t->d_stage);
   if (cudaMemset(t->d_gtable, 0, nt * sizeof(float)) != cudaSuccess ||
       cudaMemset(t->d_gw, 0, kWeightFloats * sizeof(float)) != cudaSuccess ||
       cudaMemset(t->d_mt, 0, nt * sizeof(float)) != cudaSuccess ||

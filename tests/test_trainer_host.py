@@ -28,3 +28,12 @@ def test_a_failed_step_leaves_no_gradient_behind(trainer_host, nes_lib, exact, k
     assert int(step) == nes_lib.NES_ETIMEDOUT
     assert int(parts) >= 2
     assert float(table) == float(weights) == int(parts)
+
+
+@pytest.mark.parametrize("exact", [0, 1])
+@pytest.mark.parametrize("rays", [1, 31, 33, 63, 2048, 4001, 16384, 65536, 131072, 200000, 1 << 18, 1 << 20])
+def test_device_memory_of_a_trainer(trainer_host, exact, rays):
+    """At most 64 KiB per ray (64 B per ray and march step), the staging of 2^21
+    records in FP32 (472 values), the rays' own 88 bytes and 160 KB of weight
+    images: what a trainer took before its samples' encodings were kept."""
+    assert int(trainer_host("memory", exact, rays)[0]) <= (65536 + 88) * rays + (472 * 4 << 21) + 160000

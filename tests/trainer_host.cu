@@ -5,6 +5,9 @@
 //     Prints: the step's status, the parts of the gradient's batch, what its
 //     table and weight gradients hold (each part adds one to their first
 //     entries).
+//   trainer_host memory <exact> <rays>
+//     Prints the bytes of device memory that a trainer of so many rays takes
+//     beyond gradient and moments of the table and the weights.
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
@@ -85,6 +88,15 @@ int main(int argc, char** argv) {
     if (nes_trainer_grad(t, pairs.data(), (int)cfg.batch_rays, &loss, table.data(), weights.data()) != NES_OK)
       return 5;
     std::printf("%d %d %g %g\n", step, part, table[0], weights[0]);
+    nes_trainer_destroy(t);
+    return 0;
+  }
+  if (mode == "memory" && argc == 4) {
+    cfg.exact_weight_grads = std::atoi(argv[2]);
+    cfg.batch_rays = (uint32_t)std::atoi(argv[3]);
+    const size_t before = fake::allocated;
+    if (nes_trainer_create(&ctx, &cfg, &t) != NES_OK) return 3;
+    std::printf("%zu\n", fake::allocated - before - 3 * (table_floats + nes::kWeightFloats) * sizeof(float));
     nes_trainer_destroy(t);
     return 0;
   }
