@@ -364,7 +364,8 @@ int nes_trainer_last_timings(const nes_trainer *tr, float *forward_ms, float *ba
 
 /* RGB24 -> YUV420P, BT.601 studio range, 2x2 chroma average (edge pixels
  * replicated for odd sizes).  Replaces the scene SwsContextManager in
- * RenderedFrame::convert_frame (include/base/video/rendered_frame.h:28-29). */
+ * RenderedFrame::convert_frame (include/base/video/rendered_frame.h:28-29).
+ * All YUV420P conversions take up to 131,070 rows: NES_EIO above. */
 int nes_rgb24_to_yuv420p(const uint8_t *rgb_dev, int width, int height, int rgb_linesize,
                          uint8_t *y_dev, uint8_t *u_dev, uint8_t *v_dev, const int linesize[3],
                          void *stream);

@@ -402,7 +402,7 @@ template <class Set, int kPx, bool kGray>
 cudaError_t launch_yuv(const Set& fs, int nframes, int w, int h, int src_ls, const int ls[3],
                        cudaStream_t stream) {
   const int per_row = (w + kPx - 1) / kPx, ch = (h + 1) / 2;
-  if (ch > 65535) return cudaErrorInvalidConfiguration;
+  if (ch > 65535) return cudaErrorInvalidConfiguration;  // the limit of the public calls
   const int band = (int)std::min<size_t>(ch, ((size_t)1 << 31) / per_row);  // rows per launch: 32-bit block numbers
   for (int cy0 = 0; cy0 < ch; cy0 += band) {
     const size_t blocks = (size_t)per_row * std::min(band, ch - cy0);
