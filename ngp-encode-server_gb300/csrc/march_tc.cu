@@ -711,22 +711,6 @@ cudaError_t launch_pack_tc_weights(const float* w32, uint8_t* out, cudaStream_t 
 namespace {
 
 template <class Src, int kRec>
-cudaError_t prepare_march_tc_rec() {
-  const cudaError_t e =
-      cudaFuncSetAttribute(march_tc_kernel<Src, kRec>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemRequest);
-  if (e != cudaSuccess) return e;
-  // 14 % of 228 KiB selects the 32 KiB configuration, which holds the
-  // request: the rest of the SM's 256 KiB stays L1 for the table gathers.
-  return cudaFuncSetAttribute(march_tc_kernel<Src, kRec>, cudaFuncAttributePreferredSharedMemoryCarveout, 14);
-}
-
-template <int kRec>
-cudaError_t prepare_march_tc_rec() {
-  const cudaError_t e = prepare_march_tc_rec<InParam<ViewBatch>, kRec>();
-  return e != cudaSuccess ? e : prepare_march_tc_rec<InMemory<ViewBatch>, kRec>();
-}
-
-template <class Src, int kRec>
 cudaError_t launch_march_tc_rec(const Src& src, const DevScene& scene, const DevScratch& s, int num_sms,
                                 cudaStream_t stream) {
   if (!scene.table16 || !scene.rec16 || !scene.tc_weights) return cudaErrorInvalidValue;
@@ -755,12 +739,6 @@ cudaError_t launch_march_tc_src(const Src& src, const DevScene& scene, const Dev
 
 }  // namespace
 
-cudaError_t prepare_march_tc(int rec_levels) {
-  if (rec_levels == kRecLevelsDefault) return prepare_march_tc_rec<kRecLevelsDefault>();
-  if (rec_levels == kRecLevelsSmall) return prepare_march_tc_rec<kRecLevelsSmall>();
-  return cudaErrorInvalidValue;
-}
-
 cudaError_t launch_march_tc(const ViewBatch& views, const DevScene& scene, const DevScratch& s, int num_sms,
                             cudaStream_t stream) {
   return launch_march_tc_src(InParam<ViewBatch>{views}, scene, s, num_sms, stream);
@@ -769,6 +747,32 @@ cudaError_t launch_march_tc(const ViewBatch& views, const DevScene& scene, const
 cudaError_t launch_march_tc(const ViewBatch* views_dev, const DevScene& scene, const DevScratch& s, int num_sms,
                             cudaStream_t stream) {
   return launch_march_tc_src(InMemory<ViewBatch>{views_dev}, scene, s, num_sms, stream);
+}
+
+namespace {
+
+template <class Src, int kRec>
+cudaError_t prepare_march_tc_rec() {
+  const cudaError_t e =
+      cudaFuncSetAttribute(march_tc_kernel<Src, kRec>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemRequest);
+  if (e != cudaSuccess) return e;
+  // 14 % of 228 KiB selects the 32 KiB configuration, which holds the
+  // request: the rest of the SM's 256 KiB stays L1 for the table gathers.
+  return cudaFuncSetAttribute(march_tc_kernel<Src, kRec>, cudaFuncAttributePreferredSharedMemoryCarveout, 14);
+}
+
+template <int kRec>
+cudaError_t prepare_march_tc_rec() {
+  const cudaError_t e = prepare_march_tc_rec<InParam<ViewBatch>, kRec>();
+  return e != cudaSuccess ? e : prepare_march_tc_rec<InMemory<ViewBatch>, kRec>();
+}
+
+}  // namespace
+
+cudaError_t prepare_march_tc(int rec_levels) {
+  if (rec_levels == kRecLevelsDefault) return prepare_march_tc_rec<kRecLevelsDefault>();
+  if (rec_levels == kRecLevelsSmall) return prepare_march_tc_rec<kRecLevelsSmall>();
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace nes

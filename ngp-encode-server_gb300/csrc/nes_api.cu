@@ -190,9 +190,6 @@ int nes_create(const nes_config* cfg, nes_ctx** out) {
   };
   if (cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, cfg->device) != cudaSuccess)
     return fail(NES_EIO);
-  if ((cfg->precision == NES_PREC_FP16_TC ? prepare_march_tc((int)c->cfg.record_levels) : prepare_march_fp32()) !=
-      cudaSuccess)
-    return fail(NES_EIO);
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamDefault) != cudaSuccess) return fail(NES_EIO);
   if (cudaEventCreateWithFlags(&c->ev_in, cudaEventDisableTiming) != cudaSuccess) return fail(NES_EIO);
   if (cudaEventCreateWithFlags(&c->ev_out, cudaEventDisableTiming) != cudaSuccess) return fail(NES_EIO);
@@ -245,6 +242,9 @@ int nes_create(const nes_config* cfg, nes_ctx** out) {
   c->yuv_capacity = 2 * P + 65536;
   if ((rc = dalloc(&c->d_yuv, c->yuv_capacity)) != NES_OK) return fail(rc);
   if ((rc = dalloc(&c->d_depth16, P)) != NES_OK) return fail(rc);
+  if ((cfg->precision == NES_PREC_FP16_TC ? prepare_march_tc((int)c->cfg.record_levels) : prepare_march_fp32()) !=
+      cudaSuccess)
+    return fail(NES_EIO);
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return fail(NES_EIO);
   *out = c;
   return NES_OK;

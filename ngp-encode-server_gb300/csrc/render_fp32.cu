@@ -347,13 +347,6 @@ cudaError_t launch_march_fp32_src(const Src& src, const DevScene& scene, const D
 
 }  // namespace
 
-cudaError_t prepare_march_fp32() {
-  const cudaFuncAttribute dynamic = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  const int smem = (int)sizeof(MarchSmem32);
-  const cudaError_t e = cudaFuncSetAttribute(march_fp32_kernel<InParam<ViewBatch>>, dynamic, smem);
-  return e != cudaSuccess ? e : cudaFuncSetAttribute(march_fp32_kernel<InMemory<ViewBatch>>, dynamic, smem);
-}
-
 cudaError_t launch_march_fp32(const ViewBatch& views, const DevScene& scene, const DevScratch& s,
                               int num_sms, cudaStream_t stream) {
   return launch_march_fp32_src(InParam<ViewBatch>{views}, scene, s, num_sms, stream);
@@ -362,6 +355,13 @@ cudaError_t launch_march_fp32(const ViewBatch& views, const DevScene& scene, con
 cudaError_t launch_march_fp32(const ViewBatch* views_dev, const DevScene& scene, const DevScratch& s, int num_sms,
                               cudaStream_t stream) {
   return launch_march_fp32_src(InMemory<ViewBatch>{views_dev}, scene, s, num_sms, stream);
+}
+
+cudaError_t prepare_march_fp32() {
+  const cudaFuncAttribute dynamic = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  const int smem = (int)sizeof(MarchSmem32);
+  const cudaError_t e = cudaFuncSetAttribute(march_fp32_kernel<InParam<ViewBatch>>, dynamic, smem);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(march_fp32_kernel<InMemory<ViewBatch>>, dynamic, smem);
 }
 
 cudaError_t launch_occupancy(const DevScene& scene, float threshold, uint32_t* occ_out, cudaStream_t stream) {
