@@ -422,8 +422,8 @@ def roofline_terms(head, kind, tf_sust, src, hbm, sms, rec_levels):
             bound = "gather"
     g = head.get("gather")
     if g:
-        # Supporting measurements: the same load stream replayed alone, and
-        # the hardware's random-gather rate (no locality).
+        # Supporting measurements: the samples' loads alone, in the replay's
+        # order, and the hardware's random-gather rate (no locality).
         out["gather_probes"] = dict(g)
         out["gather_probes"]["replay_ms_scaled"] = round(g["replay_ms"] * n / head["samples_pose0"], 3)
     term = out["gather"] if bound == "gather" else out["tensor"]
@@ -450,8 +450,8 @@ def roofline_terms(head, kind, tf_sust, src, hbm, sms, rec_levels):
 
 
 def measure_gather_ceilings(r, views, flush, stream, dev, reps=5):
-    """Gather probes beside the march's roofline: the march's own load
-    stream replayed without arithmetic on the same views
+    """Gather probes beside the march's roofline: the loads of the march's
+    samples without arithmetic on the same views, one step of 32 rays per warp
     (nes_probe_gather_replay, 512 ray slots per SM, L2 flushed before each
     replay, median), and the random-gather rates of 4-, 16- and 32-byte loads
     over an L2-resident 32 MiB table (nes_probe_gather, CUDA events, median of
@@ -473,9 +473,9 @@ def measure_gather_ceilings(r, views, flush, stream, dev, reps=5):
         if i:
             rep.append(ms.value)
     out = {"replay_ms": round(statistics.median(rep), 3),
-           "replay_note": "the march's load stream alone (same rays, addresses and per-tile pacing, no "
-                          "interpolation, MLP or compositing): it runs no faster than the march, which "
-                          "overlaps its gathers with the MLP warps' work"}
+           "replay_note": "the loads of the march's samples alone (no interpolation, MLP or compositing), "
+                          "one step of 32 rays per warp at a time; the march takes several steps of fewer "
+                          "rays, whose gathers share more lines: a probe of another order, not a floor"}
     table = torch.randint(0, 1 << 30, ((32 << 20) // 4,), dtype=torch.int32, device=dev)
     threads, loads = sms * 2048, 256
     for nbytes in (4, 16, 32):

@@ -497,11 +497,11 @@ int nes_selftest_bounded_wait(nes_ctx *ctx, uint32_t poll_limit, int arrive);
  * load_bytes (4, 16, or 32 read as two 16-byte loads) over table_bytes of
  * device memory (table_bytes / load_bytes a power of two), XOR-folded into
  * sink_dev[thread]; the caller times it on `stream`.
- * nes_probe_gather_replay replays the march's own load stream for the views
- * on a tensor-core context -- the same rays, sample positions (one step of
- * 32 rays per warp at a time; the march takes 4, 8 or 32 steps of each),
- * record and table addresses, with no interpolation, MLP or compositing --
- * with `threads` (256 or 512) ray slots per SM, and returns its device time
+ * nes_probe_gather_replay makes the loads of the march's samples for the views
+ * on a tensor-core context -- the same rays, sample positions, records and
+ * table entries, with no interpolation, MLP or compositing, in an order of its
+ * own: one step of 32 rays per warp at a time, where the march takes 4, 8 or 32
+ * steps of fewer rays (the replay is no floor under the march) -- with `threads` (256 or 512) ray slots per SM, and returns its device time
  * (CUDA events) in *replay_ms; sink_dev holds at least (SM count) x threads
  * words.  Both write nothing but the sink. */
 int nes_probe_gather(const void *table_dev, uint64_t table_bytes, int load_bytes, uint32_t loads_per_thread,

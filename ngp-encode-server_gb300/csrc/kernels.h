@@ -138,9 +138,9 @@ cudaError_t launch_bounded_wait_probe(uint32_t poll_limit, int arrive, uint32_t*
 // `threads` threads (a multiple of 256) each make loads_per_thread uniformly
 // random loads of load_bytes (4, 16, or 32 as two 16-byte loads) over
 // table_bytes (table_bytes / load_bytes a power of two), XOR-folded into
-// sink[thread].  gather_replay: the march's own load stream over the rays
-// already generated in s (num_sms CTAs of `threads` = 256 or 512 threads;
-// sink holds num_sms * threads words).
+// sink[thread].  gather_replay: the loads of the march's samples, one step of
+// 32 rays per warp at a time, over the rays already generated in s (num_sms CTAs
+// of `threads` = 256 or 512 threads; sink holds num_sms * threads words).
 cudaError_t launch_gather_probe(const void* table, uint64_t table_bytes, int load_bytes, uint32_t loads_per_thread,
                                 uint32_t* sink, uint32_t threads, cudaStream_t stream);
 cudaError_t launch_gather_replay(const ViewBatch& views, const DevScene& scene, const DevScratch& s, int num_sms,

@@ -296,27 +296,28 @@ constexpr uint32_t kTagSample = 1u, kTagFirst = 2u, kTagRay = 8u;
 
 // log2 of the steps of one ray that a tile takes at once, in neighbouring rows
 // of a warp (32 >> shift rays per warp).  Two things set it.  A batch of few
-// rays must be split along them to fill the chip's 77,824 rows: at one row per
-// ray a 64x48 view keeps 2 % of them busy for as many tiles as its longest
-// ray has steps.  And a warp's 32 samples should lie close together, so that
-// its gathers share cells: a 4x2-pixel patch four steps deep is nearer a cube
-// than a 4x8 patch of single steps.  Measured, ms with L2 flushed, one row per
-// ray (as it was) against 4, 8 and 32 steps:
-//                 rays     seeded scene                 opaque, sparse scene
-//   64x48         1.6k     4.7  -> 1.16, 0.70, 0.21     1.06 -> 0.30, 0.20, 0.15
-//   256x256       34k      4.7  -> 1.22, 0.79, 0.70     1.25 -> 0.35, 0.25, 0.29
-//   320x240       39k              1.24, 1.17, 0.99             0.37, 0.32, 0.40
-//   400x300       61k              1.82, 1.62, 1.48
-//   480x360       88k              2.14, 2.01, 2.01             0.53, 0.49, 0.70
-//   640x360       118k     4.9  -> 3.18, 3.14, 3.54             0.75, 0.70, 1.18
-//   853x480       210k             5.10, 5.15, 6.24             1.14, 1.15, 2.04
-//   1280x720      470k     13.4 -> 10.3, 10.6, 13.8
-//   1920x1080     1.06M    25.2 -> 21.4, 22.4, 30.5
-//   2x1920x1832            32.2 -> 26.8, 27.7, 37.4
-//   3x853x481                                           3.19 -> 1.94, 1.99, 3.67
-// Sixteen steps were slower than both neighbours from 256x256 up.  Within the
-// warp a ray's steps are neighbours: with the rays next to each other and the
-// steps apart the 1080p march took 25.1 ms, with both interleaved 24.1, so 23.8.
+// rays must be split along them to fill the chip's 77,824 rows: one row per ray
+// keeps 1 % of them busy in a 64x48 view, for as many tiles as its longest ray
+// has steps.  And a warp's 32 samples should lie close together, so that its
+// gathers share cells: a 4x2-pixel patch four steps deep is nearer a cube than a
+// 4x8 patch of single steps.  32 steps up to half as many rays as rows, 8 up to
+// twice as many; ms with L2 flushed, 4, 8 and 32 steps:
+//                 rays     seeded scene       opaque, sparse scene
+//   64x48         0.9k     1.04, 0.53, 0.19   0.29, 0.19, 0.14
+//   256x256       14k      1.11, 0.76, 0.73   0.35, 0.26, 0.29
+//   320x240       21k      1.21, 1.06, 1.05   0.38, 0.32, 0.39
+//   400x300       33k      1.78, 1.47, 1.58   0.46, 0.39, 0.55
+//   480x360       48k      2.12, 1.89, 2.15   0.55, 0.46, 0.74
+//   640x360       84k      3.17, 3.05, 3.76   0.74, 0.68, 1.22
+//   853x480       149k     5.12, 5.02, 6.64   1.13, 1.09, 2.12
+//   3x853x481     269k     9.08, 9.15, 11.9   1.91, 1.89, 3.79
+//   1280x720      336k     10.5, 10.5, 14.7   2.13, 2.21, 4.70
+//   1920x1080     757k     21.9, 22.9, 32.6   4.35, 4.75, 10.5
+//   2x1920x1832   908k     27.3, 28.3, 40.2   5.49, 5.82, 12.8
+// From 21k rays on eight steps are as fast as 32 or faster, so the first line
+// lies high by up to a factor of two.  Within the warp a ray's steps are
+// neighbours: apart, or interleaved with other rays', the 1080p march took 5 and
+// 1 % longer.
 __device__ __forceinline__ uint32_t lane_shift(uint32_t nrays, uint32_t rows) {
   if (nrays <= rows / 2) return 5;
   if (nrays <= rows * 2) return 3;

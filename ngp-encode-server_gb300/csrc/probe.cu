@@ -2,18 +2,20 @@
 //
 // The march's MLP contraction has a tensor-core roofline (the measured bf16
 // peak); its other term is the hash-table gather stream: per sample one
-// per-cell corner record for each of the recorded levels (32 bytes,
-// read as two 16-byte loads) and 8 scattered 4-byte table entries for each
-// level above: the 512 bytes of algorithmic gathers.  No library figure exists for such a
+// per-cell corner record for each of the recorded levels (32 bytes) and 8
+// scattered 4-byte table entries for each level above: the 512 bytes of
+// algorithmic gathers.  No library figure exists for such a
 // stream, so these kernels measure it on the device itself:
 //
 //  - gather_probe_kernel: uniformly random loads of 4, 16 or 32 bytes over a
 //    table of a given size (e.g. the 32 MiB FP16 table, L2-resident): the
 //    hardware's random-gather rate with no locality to exploit;
-//  - replay_kernel: the march's own load stream -- the same compacted rays,
-//    the same warp-wide 32-ray refills, the same sample positions and the same
-//    record and table addresses -- with no interpolation, no MLP and no
-//    compositing: the floor the gathers alone put under the march.
+//  - replay_kernel: the loads of the march's samples -- the same compacted rays,
+//    sample positions and record and table entries -- with no interpolation, no
+//    MLP and no compositing, in an order of its own: one step of 32 rays per
+//    warp, records as two 16-byte loads.  The march takes 4, 8 or 32 steps of
+//    each ray, in 256-bit loads, and shares more lines; the replay is no floor
+//    under it.
 #include <cuda_fp16.h>
 
 #include "kernels.h"
@@ -46,7 +48,7 @@ gather_probe_kernel(const uint8_t* __restrict__ table, uint32_t mask, uint32_t l
     } else if (kBytes == 16) {
       const uint4 v = __ldg(reinterpret_cast<const uint4*>(table) + e);
       acc ^= v.x ^ v.y ^ v.z ^ v.w;
-    } else {  // a 32-byte record as two 16-byte loads, like the march
+    } else {  // a 32-byte record as two 16-byte loads
       const uint4 a = __ldg(reinterpret_cast<const uint4*>(table) + 2 * (size_t)e);
       const uint4 b = __ldg(reinterpret_cast<const uint4*>(table) + 2 * (size_t)e + 1);
       acc ^= a.x ^ a.y ^ a.z ^ a.w ^ b.x ^ b.y ^ b.z ^ b.w;
@@ -92,8 +94,8 @@ __device__ __forceinline__ uint32_t replay_level_tab(const uint32_t* __restrict_
   return acc;
 }
 
-// Level L as the march reads it: a per-cell record if the level is recorded, else
-// eight table entries.
+// Level L's entries: a per-cell record if the level is recorded, else eight table
+// entries.
 template <int L>
 __device__ __forceinline__ uint32_t replay_level(const DevScene& sc, const uint32_t* __restrict__ table,
                                                  const float3& x) {
@@ -103,12 +105,11 @@ __device__ __forceinline__ uint32_t replay_level(const DevScene& sc, const uint3
 
 // One thread per ray slot, warps refilled 32 rays at a time (one 4x8 pixel
 // tile) once all their lanes are done, every occupied sample's records and
-// table entries loaded in order, the occupancy bit of every sample read as
-// the march reads it; one CTA per SM of 512 threads (as many slots as the
-// march's encoder threads) or 256.  Like the march's encoder groups, each
-// group of 128 slots advances one sample per step together (a named-barrier
-// step per sample, the march's tile), so rays that are neighbours on screen
-// stay neighbours in t and share the lines they load.
+// table entries loaded in order, the occupancy bit of every sample read; one CTA
+// per SM of 512 threads (as many slots as the march's encoder threads) or 256.
+// Each group of 128 slots advances one sample per step together (a named-barrier
+// step per sample), so rays that are neighbours on screen stay neighbours in t
+// and share the lines they load.
 __global__ void __launch_bounds__(512, 1)
 replay_kernel(const __grid_constant__ InParam<ViewBatch> src, const DevScene sc, const DevScratch s,
               uint32_t* __restrict__ sink) {
@@ -124,7 +125,7 @@ replay_kernel(const __grid_constant__ InParam<ViewBatch> src, const DevScene sc,
   int n = 0, ei = 0;
   auto occ_at = [&](int i) { return occupied(sc.occ, sample_pos(o, d, fmaf((float)i + 0.5f, kDt, ts))); };
   for (;;) {
-    for (;;) {  // whole-warp refill, as the march's encoders
+    for (;;) {  // whole-warp refill
       if (__ballot_sync(0xffffffffu, live) != 0u || exhausted) break;
       const uint32_t base = warp_claim(s.counters + kCtrCursor, 32);
       if (base >= nrays) {

@@ -17,9 +17,9 @@ namespace nes {
 namespace {
 
 constexpr int kRaygenThreads = 256;
-// Twelve warps of the march per SM: 182 KB of shared memory (weights, the
+// Twelve warps of the march per SM: 185 KB of shared memory (weights, the
 // warps' encodings and activations) and 168 registers a thread.  1080p: 8 warps
-// 132 ms, 10 131, 11 129, 12 128; it is bound by the products' operand reads
+// 127 ms, 10 129, 11 125, 12 121; it is bound by the products' operand reads
 // (a lane's 8 x 8 tile takes 64 bytes per 64 multiply-adds, 16 cycles of the
 // SM's 128 bytes a cycle against 16 of its FMA lanes).
 constexpr int kMarchWarps = 12;
@@ -27,17 +27,16 @@ constexpr int kMarchThreads = 32 * kMarchWarps;
 
 // log2 of the steps of one ray that a warp takes at once: many where the rays
 // are too few for the chip's 58,368 rows, fewer where that would evaluate
-// steps behind an opaque surface or leave lanes without an occupied step.  ms,
-// one ray per thread (as it was) -> 8 and 32 steps:
-//               rays   seeded scene          opaque, sparse scene
-//   64x48       1.6k   20   -> 2.2,  0.59    10.0 -> 0.61, 0.38
-//   256x256     34k    24   -> 3.6,  2.6     13.1 -> 0.86, 1.07
-//   400x300     61k    26.7 -> 6.0,  6.7     13.7 -> 1.5,  1.9
-//   640x360     118k   37.7 -> 15.3, 16.4    18.2 -> 3.0,  4.3
-//   853x481     210k   54.6 -> 26.3, 28.9    24.2 -> 5.1,  7.4
-//   1920x1080   1.06M  232  -> 128,  145     (1, 2, 4, 16 steps: 163, 144, 139, 141)
-// (the column not taken, before the next tile's encoding ran under the
-// products.)
+// steps behind an opaque surface or leave lanes without an occupied step.  The
+// line lies at two rays for three rows, above which 32 steps gain nothing in a
+// dense field and lose two thirds in a sparse one.  ms, 8 and 32 steps:
+//               rays   seeded scene   opaque, sparse scene
+//   64x48       0.9k   1.72, 0.54     0.53, 0.36
+//   256x256     14k    3.35, 2.52     0.81, 1.01
+//   400x300     33k    6.55, 5.76     1.45, 2.17
+//   640x360     84k    14.2, 14.0     2.84, 4.73
+//   853x481     149k   24.7, 24.8     4.81, 8.33
+//   1920x1080   757k   121, 124       22.4, 41.5
 __device__ __forceinline__ int march32_shift(uint32_t nrays, uint32_t rows) { return nrays <= rows / 3 * 2 ? 5 : 3; }
 
 // Grid-stride over the batch's ray-generation threads (the loop bound is
@@ -104,8 +103,7 @@ raygen_kernel(const __grid_constant__ Src src, float4* __restrict__ ray_dt, RayM
 // samples in step order, by shuffle.
 // While a tile is in the MLPs the next one is encoded, a level per eight
 // inputs of the products, so the gathers run under the multiply-adds (1080p 138
-// -> 128 ms, 256x256 2.9 -> 2.6 ms; before, the products alone took 94 ms, the
-// encoding alone 41).
+// -> 128 ms, 256x256 2.9 -> 2.6 ms).
 struct MarchSmem32 {
   TileWeights32 w;
   float enc[kMarchWarps][kEnc * 32];
